@@ -188,32 +188,52 @@ void plan_release(holo_plan_s *p, cudaStream_t s) {
   delete p;
 }
 
-// Tile order of a point set into the plan's buffers (the order does not depend on
-// the tile size), or `known`, the order another plan computed for the same array.
-static int order_set(holo_plan_s *p, const double *pos, int n, int n_pad, double *pos_sorted,
-                     int32_t *order, cudaStream_t s, const int32_t *known, int tiling) {
-  if (n == 0) return launch_gather_pos(pos, nullptr, 0, n_pad, pos_sorted, s);
-  if (known) {
-    HOLO_CUDA(cudaMemcpyAsync(order, known, (size_t)n * sizeof(int32_t),
-                              cudaMemcpyDeviceToDevice, s));
-    return launch_gather_pos(pos, order, n, n_pad, pos_sorted, s);
+// Device scratch of the tiler for n points (the packed tiling's part only where asked for).
+static bool tiler_scratch(Scratch &tmp, int n, bool packed, TileScratch *t) {
+  t->bbox = tmp.get<double>(6);
+  t->bbox_scratch = tmp.get<double>(6 * 152);
+  t->keys = tmp.get<uint16_t>(n);
+  t->hist = tmp.get<uint32_t>(sort_hist_entries(n));
+  t->scan = tmp.get<uint32_t>(4096);
+  if (packed) {
+    t->keys2 = tmp.get<uint16_t>(n);
+    t->tmp_a = tmp.get<int32_t>(n);
+    t->tmp_b = tmp.get<int32_t>(n);
+    if (!t->keys2 || !t->tmp_a || !t->tmp_b) return false;
   }
+  return t->bbox && t->bbox_scratch && t->keys && t->hist && t->scan;
+}
+
+// Tile order of both point sets into the plan's buffers (the order does not depend on the
+// tile size), or the order another plan computed for the same array; their box pyramids,
+// and the statistics on the host (the one host round trip of a tiling).
+static int tile_both(holo_plan_s *p, const double *u, const double *v, int tiling,
+                     const int32_t *known_s, const int32_t *known_t, cudaStream_t s) {
+  if (p->N == 0 || p->M == 0) return HOLO_OK;
   Scratch tmp(p->h, s);
-  const size_t hist_n = sort_hist_entries(n);
-  TileScratch t{};
-  t.bbox = tmp.get<double>(6);
-  t.bbox_scratch = tmp.get<double>(6 * 1024);
-  t.keys = tmp.get<uint16_t>(n);
-  t.keys2 = tmp.get<uint16_t>(n);
-  t.hist = tmp.get<uint32_t>(hist_n);
-  t.scan = tmp.get<uint32_t>(hist_n + 4096 + 16);
-  t.tmp_a = tmp.get<int32_t>(n);
-  t.tmp_b = tmp.get<int32_t>(n);
-  if (!t.bbox || !t.bbox_scratch || !t.keys || !t.keys2 || !t.hist || !t.scan || !t.tmp_a ||
-      !t.tmp_b)
-    return fail(HOLO_ERR_ALLOC, "tiler scratch");
-  HOLO_TRY(tile_order(pos, n, order, t, s, tiling));
-  HOLO_TRY(launch_gather_pos(pos, order, n, n_pad, pos_sorted, s));
+  TileSet set[2] = {};
+  BoxStats *stats = tmp.get<BoxStats>(2);
+  bool ok = stats != nullptr;
+  for (int i = 0; i < 2; ++i) {
+    TileSet &t = set[i];
+    t.pos = i ? v : u;
+    t.n = i ? p->M : p->N;
+    t.n_pad = i ? p->M : p->n_pad;
+    t.known = i ? known_t : known_s;
+    t.order = i ? p->order_t : p->order_s;
+    t.pos_sorted = i ? p->pos_t : p->pos_s;
+    t.boxes = i ? p->boxes_t : p->boxes_s;
+    t.parts = tmp.get<BoxStats>((size_t)(t.n + kSuperTile - 1) / kSuperTile);
+    t.stats = stats + i;
+    ok = ok && t.parts && (t.known || tiler_scratch(tmp, t.n, tiling == kTilePacked, &t.scratch));
+  }
+  if (!ok) return fail(HOLO_ERR_ALLOC, "tiler scratch");
+  HOLO_TRY(tile_sets(set, 2, tiling, s));
+  BoxStats both[2];
+  HOLO_CUDA(cudaMemcpyAsync(both, stats, sizeof(both), cudaMemcpyDeviceToHost, s));
+  HOLO_CUDA(cudaStreamSynchronize(s));
+  p->stats_s = both[0];
+  p->stats_t = both[1];
   return HOLO_OK;
 }
 
@@ -261,44 +281,48 @@ void split_error_model(const TileStats &st, double *base, double *curv, double *
   *lin = rho * x2 + (x2 + y / 2.0 + ps * st.h_t / (qt * gap)) * (400e-9 / (2.0 * M_PI));
 }
 
-// Tile boxes for source tiles of `cs` and target tiles of `tt` points, and the
-// split-path error model of that tiling.
+// The split-path error model of source tiles of `cs` and target tiles of `tt` points, from the
+// plan's box pyramids; a tile size without a level (768) gets boxes of its own.  Leaves
+// the boxes in tiles_s / tiles_t.
 static int tile_error_bound(holo_plan_s *p, int cs, int tt, double *bound, double *curv,
                             double *lin, double *gemm, cudaStream_t s) {
-  const int ns = (p->N + cs - 1) / cs, nt = (p->M + tt - 1) / tt;
-  HOLO_TRY(launch_tile_bbox(p->pos_s, p->N, cs, p->tiles_s, s));
-  HOLO_TRY(launch_tile_bbox(p->pos_t, p->M, tt, p->tiles_t, s));
-  if (ns == 0 || nt == 0) {
+  const int ls = box_level(cs), lt = box_level(tt);
+  p->tiles_s = ls >= 0 ? p->boxes_s + 6 * box_offset(p->N, ls) : p->odd_tiles;
+  p->tiles_t = p->boxes_t + 6 * box_offset(p->M, lt);
+  if (p->N == 0 || p->M == 0) {
     *bound = *curv = *lin = *gemm = 0.0;
     return HOLO_OK;
   }
-  std::vector<double> ts((size_t)6 * ns), tg((size_t)6 * nt);
-  HOLO_CUDA(cudaMemcpyAsync(ts.data(), p->tiles_s, ts.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-  HOLO_CUDA(cudaMemcpyAsync(tg.data(), p->tiles_t, tg.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-  HOLO_CUDA(cudaStreamSynchronize(s));
-  auto boxes = [](const std::vector<double> &t, int n, double *lo, double *hi, double *hmax,
-                  double *hd) {
-    for (int d = 0; d < 3; ++d) { lo[d] = 1e300; hi[d] = -1e300; hd[d] = 0.0; }
-    *hmax = 0.0;
-    for (int i = 0; i < n; ++i) {
-      const double *c = &t[6 * (size_t)i];
+  TileStats st;
+  for (int d = 0; d < 3; ++d) {
+    st.lo_t[d] = p->stats_t.lo[d];
+    st.hi_t[d] = p->stats_t.hi[d];
+    st.hd_t[d] = p->stats_t.hd[lt][d];
+    st.lo_s[d] = p->stats_s.lo[d];
+    st.hi_s[d] = p->stats_s.hi[d];
+    st.hd_s[d] = ls >= 0 ? p->stats_s.hd[ls][d] : 0.0;
+  }
+  st.h_t = p->stats_t.h[lt];
+  st.h_s = ls >= 0 ? p->stats_s.h[ls] : 0.0;
+  if (ls < 0) {
+    const int ns = (p->N + cs - 1) / cs;
+    HOLO_TRY(launch_tile_bbox(p->pos_s, p->N, cs, p->tiles_s, s));
+    std::vector<double> ts((size_t)6 * ns);
+    HOLO_CUDA(cudaMemcpyAsync(ts.data(), p->tiles_s, ts.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+    HOLO_CUDA(cudaStreamSynchronize(s));
+    for (int i = 0; i < ns; ++i) {
       double h2 = 0.0;
       for (int d = 0; d < 3; ++d) {
-        lo[d] = std::min(lo[d], c[d] - c[3 + d]);
-        hi[d] = std::max(hi[d], c[d] + c[3 + d]);
-        hd[d] = std::max(hd[d], c[3 + d]);
-        h2 += c[3 + d] * c[3 + d];
+        const double h = ts[6 * (size_t)i + 3 + d];
+        st.hd_s[d] = std::max(st.hd_s[d], h);
+        h2 += h * h;
       }
-      *hmax = std::max(*hmax, sqrt(h2));
+      st.h_s = std::max(st.h_s, sqrt(h2));
     }
-  };
-  TileStats st;
-  boxes(ts, ns, st.lo_s, st.hi_s, &st.h_s, st.hd_s);
-  boxes(tg, nt, st.lo_t, st.hi_t, &st.h_t, st.hd_t);
+  }
   split_error_model(st, bound, curv, lin, gemm);
   return HOLO_OK;
 }
-
 
 int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, size_t M,
                      int precision, int forced_variant, cudaStream_t s, holo_plan_s **out,
@@ -333,14 +357,14 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
     HOLO_TRY(alloc_plan(pp, (void **)&p->order_s, std::max<size_t>(N, 1) * sizeof(int32_t), s));
     HOLO_TRY(alloc_plan(pp, (void **)&p->pos_t, (size_t)3 * std::max<size_t>(M, 1) * sizeof(double), s));
     HOLO_TRY(alloc_plan(pp, (void **)&p->order_t, std::max<size_t>(M, 1) * sizeof(int32_t), s));
-    HOLO_TRY(alloc_plan(pp, (void **)&p->tiles_s, (size_t)6 * (N / 256 + 1) * sizeof(double), s));
-    HOLO_TRY(alloc_plan(pp, (void **)&p->tiles_t, (size_t)6 * (M / 256 + 1) * sizeof(double), s));
+    HOLO_TRY(alloc_plan(pp, (void **)&p->boxes_s,
+                        (6 * box_offset((int)N, kBoxLevels) + 6) * sizeof(double), s));
+    HOLO_TRY(alloc_plan(pp, (void **)&p->boxes_t,
+                        (6 * box_offset((int)M, kBoxLevels) + 6) * sizeof(double), s));
     auto order_both = [&](int tiling, const int32_t *ks, const int32_t *kt) -> int {
-      HOLO_TRY(order_set(pp, u, (int)N, p->n_pad, p->pos_s, p->order_s, s, ks, tiling));
-      HOLO_TRY(order_set(pp, v, (int)M, (int)M, p->pos_t, p->order_t, s, kt, tiling));
       p->tiling_s = ks ? known_tiling_s : tiling;
       p->tiling_t = kt ? known_tiling_t : tiling;
-      return HOLO_OK;
+      return tile_both(pp, u, v, tiling, ks, kt, s);
     };
     // candidates: a forced variant alone; else the variant tuned for this size
     // bucket, then the preference list (fastest first, ever smaller tiles); the
@@ -353,6 +377,9 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
       if (h->variant_table[precision][bucket] >= 0) cands.push_back(h->variant_table[precision][bucket]);
       for (int c : split_preferences(N, M)) cands.push_back(c);
     }
+    for (int c : cands)
+      if (box_level(split_variant(c).cs) < 0 && !p->odd_tiles)
+        HOLO_TRY(alloc_plan(pp, (void **)&p->odd_tiles, (size_t)6 * (N / 256 + 1) * sizeof(double), s));
     // the first candidate whose bound holds on the current tiles (else the last);
     // leaves that candidate's tile boxes in tiles_s / tiles_t
     auto choose = [&](size_t *chosen) -> int {
@@ -449,11 +476,11 @@ int plan_execute_impl(holo_plan_s *p, int sign, double lambda, const double *amp
     return HOLO_OK;
   }
   Scratch tmp(p->h, s);
+  const double k = (2.0 * M_PI) / lambda;
+  const bool cst = (flags & HOLO_FLAG_CONST_PHASE) != 0;
   double2 *ap = tmp.get<double2>(p->n_pad);
   double2 *partial = p->splits > 1 ? tmp.get<double2>((size_t)p->splits * p->M) : nullptr;
   if (!ap || (p->splits > 1 && !partial)) return fail(HOLO_ERR_ALLOC, "execute scratch");
-  const double k = (2.0 * M_PI) / lambda;
-  const bool cst = (flags & HOLO_FLAG_CONST_PHASE) != 0;
   if (p->precision == HOLO_SPLIT32) {
     float2 *apf = reinterpret_cast<float2 *>(ap);  // n_pad float pairs fit in the buffer
     HOLO_TRY(launch_gather_apf(amp, phase, p->order_s, p->N, p->n_pad, apf, s));
@@ -744,19 +771,9 @@ int holo_tile_order(holo_handle h, const double *xyz, size_t n, int tiling, int3
   const double *dxyz = xyz;
   if (!dev) HOLO_TRY(st.up(xyz, 3 * n, &dxyz));
   Scratch tmp(h, s);
-  const size_t hist_n = sort_hist_entries((int)n);
   TileScratch t{};
-  t.bbox = tmp.get<double>(6);
-  t.bbox_scratch = tmp.get<double>(6 * 1024);
-  t.keys = tmp.get<uint16_t>(n);
-  t.keys2 = tmp.get<uint16_t>(n);
-  t.hist = tmp.get<uint32_t>(hist_n);
-  t.scan = tmp.get<uint32_t>(hist_n + 4096 + 16);
-  t.tmp_a = tmp.get<int32_t>(n);
-  t.tmp_b = tmp.get<int32_t>(n);
   int32_t *dorder = tmp.get<int32_t>(n);
-  if (!t.bbox || !t.bbox_scratch || !t.keys || !t.keys2 || !t.hist || !t.scan || !t.tmp_a ||
-      !t.tmp_b || !dorder)
+  if (!dorder || !tiler_scratch(tmp, (int)n, tiling == HOLO_TILE_PACKED, &t))
     return fail(HOLO_ERR_ALLOC, "tiler scratch");
   HOLO_TRY(tile_order(dxyz, (int)n, dorder, t, s, tiling));
   HOLO_CUDA(cudaMemcpyAsync(order, dorder, n * sizeof(int32_t), cudaMemcpyDefault, s));

@@ -177,12 +177,9 @@ int kernel_setup(int threads, int smem_bytes, int *ctas_per_sm) {
 void note_launches(int n);
 
 // tiler.cu
-int launch_bbox(const double *pos, int n, double *bbox6, double *scratch, int scratch_blocks,
-                cudaStream_t s);
 size_t sort_hist_entries(int n);
-// Device scratch of tile_order for n points: bbox[6], bbox_scratch[6 * 1024],
-// keys and keys2[n], hist[sort_hist_entries(n)], scan[that + 4096 + 16], tmp_a and
-// tmp_b[n].
+// Device scratch of tile_order for n points: bbox[6], bbox_scratch[6 * 152], keys and
+// keys2[n], hist[sort_hist_entries(n)], scan[4096], tmp_a and tmp_b[n].
 struct TileScratch {
   double *bbox, *bbox_scratch;
   uint16_t *keys, *keys2;
@@ -232,6 +229,42 @@ int launch_split(const SplitProblem &p, int variant, int grid, bool const_phase,
 int launch_split_batched(const SplitProblem *probs_dev, const WorkItem *items, int n_items,
                          int *queue, int variant, int grid, int *err, cudaStream_t s);
 int split_occupancy(int variant, bool mc, int *ctas_per_sm);
+
+// ---- boxes of a tile order ----------------------------------------------------------
+// Boxes of the tiles of 256, 512, .. 8192 consecutive points (levels 0 .. 5) of a tile
+// order, and what the planner needs to know about them.
+constexpr int kBoxLevels = 6;
+struct BoxStats {
+  double lo[3], hi[3];             // bounding box of all tiles
+  double hd[kBoxLevels][3];        // largest half extent per level and axis
+  double h[kBoxLevels];            // largest half diagonal per level
+};
+constexpr int kBoxStatDoubles = sizeof(BoxStats) / sizeof(double);
+inline int box_count(int n, int level) { return (n + (256 << level) - 1) / (256 << level); }
+inline size_t box_offset(int n, int level) {  // in boxes; level kBoxLevels: all of them
+  size_t o = 0;
+  for (int l = 0; l < level; ++l) o += box_count(n, l);
+  return o;
+}
+inline int box_level(int tile) {  // level of a tile size, -1 when it has none
+  for (int l = 0; l < kBoxLevels; ++l)
+    if (tile == 256 << l) return l;
+  return -1;
+}
+// tiler.cu: tile order, tile-ordered points (zeros up to n_pad), box pyramid and statistics
+// of one or two point sets, every step one launch for both; n >= 1.
+struct TileSet {
+  const double *pos;
+  int n, n_pad;
+  const int32_t *known;    // the set's order from another plan (then no sort), or null
+  int32_t *order;
+  double *pos_sorted;      // 3 * n_pad
+  double *boxes;           // 6 * box_offset(n, kBoxLevels)
+  BoxStats *parts;         // one per 8192 points
+  BoxStats *stats;
+  TileScratch scratch;     // of its own where it is sorted
+};
+int tile_sets(const TileSet *set, int count, int tiling, cudaStream_t s);
 
 // kernel_fp64.cu
 int launch_fp64(const Fp64Problem &p, int variant, int grid, bool const_phase, int *err,
@@ -290,6 +323,10 @@ struct holo_plan_s {
   double *pos_t = nullptr;       // 3 * M
   double *tiles_s = nullptr;     // 6 * n_stiles
   double *tiles_t = nullptr;     // 6 * n_ttiles
+  // split: boxes of the tiles of 256 .. 8192 points and their statistics (host)
+  double *boxes_s = nullptr, *boxes_t = nullptr;
+  holo::BoxStats stats_s{}, stats_t{};
+  double *odd_tiles = nullptr;   // boxes of source tiles that are none of these sizes
   int32_t *order_s = nullptr;    // N (split only)
   int32_t *order_t = nullptr;    // M (split only)
   float *geo_s = nullptr;        // split: float-float offsets from the tile centres

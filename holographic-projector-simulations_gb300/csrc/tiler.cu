@@ -16,72 +16,114 @@
 //     time, used where the Hilbert tiles' error bound rules out the fastest kernel.
 // All sorts are stable and ties keep input order: each order is deterministic
 // and does not depend on the tile size.
-#include <float.h>
+#include <algorithm>
 
 #include "internal.cuh"
 
 namespace holo {
 namespace {
 
-__device__ __forceinline__ void minmax3(double *lo, double *hi, const double *p) {
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = fmin(lo[d], p[d]);
-    hi[d] = fmax(hi[d], p[d]);
-  }
+// Doubles as 64-bit integers of the same order (NaN excluded): minima and maxima run on the
+// integer pipe, where FP64 compares would take a pair of the few FP64 lanes each.
+__device__ __forceinline__ long long ordered64(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
 }
+__device__ __forceinline__ double from_ordered64(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
+}
+constexpr long long kOrderedMax = 0x7fefffffffffffffLL;   // ordered64(DBL_MAX)
+constexpr long long kOrderedMin = ~0x7fefffffffffffffLL;  // ordered64(-DBL_MAX)
 
-// Block-wide min/max of 3 coordinates; result valid in thread 0.
-template <int T>
-__device__ void block_minmax(double *lo, double *hi) {
-  __shared__ double s_lo[T][3], s_hi[T][3];
-  for (int d = 0; d < 3; ++d) {
-    s_lo[threadIdx.x][d] = lo[d];
-    s_hi[threadIdx.x][d] = hi[d];
+struct Box64 {
+  long long lo[3], hi[3];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = kOrderedMax;
+      hi[d] = kOrderedMin;
+    }
   }
-  __syncthreads();
-  for (int w = T / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      for (int d = 0; d < 3; ++d) {
-        s_lo[threadIdx.x][d] = fmin(s_lo[threadIdx.x][d], s_lo[threadIdx.x + w][d]);
-        s_hi[threadIdx.x][d] = fmax(s_hi[threadIdx.x][d], s_hi[threadIdx.x + w][d]);
+  __device__ __forceinline__ void add(double x, double y, double z) {
+    const double p[3] = {x, y, z};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const long long k = ordered64(p[d]);
+      if ((__double_as_longlong(p[d]) & 0x7fffffffffffffffLL) <= 0x7ff0000000000000LL) {  // not NaN
+        lo[d] = min(lo[d], k);
+        hi[d] = max(hi[d], k);
       }
     }
-    __syncthreads();
   }
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = s_lo[0][d];
-    hi[d] = s_hi[0][d];
+  __device__ __forceinline__ void warp_reduce() {
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        lo[d] = min(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+        hi[d] = max(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+      }
+  }
+};
+
+// One or two point sets that a launch of the Hilbert tiling handles (blockIdx.y).
+struct SortSet {
+  const double *pos;
+  int n, parts;         // points; blocks of the box reduction
+  long long *box;       // [parts][6] ordered keys
+  uint16_t *keys;
+  uint32_t *hist;       // [blocks of kSortBlock][kCells]
+  uint32_t *totals;     // [kCells]
+  int32_t *order;
+};
+struct SortSets {
+  SortSet s[2];
+};
+
+// Box of 8 points per thread and block, and zeros for the histogram of the next kernel.
+__global__ void __launch_bounds__(256) k_box_parts(const SortSets sets) {
+  const SortSet &S = sets.s[blockIdx.y];
+  if ((int)blockIdx.x >= S.parts) return;
+  __shared__ Box64 w[8];
+  const int step = S.parts * 256, at = blockIdx.x * 256 + threadIdx.x;
+  Box64 b;
+  b.clear();
+  for (int i = at; i < S.n; i += step) {
+    const double *p = S.pos + 3 * (size_t)i;
+    b.add(p[0], p[1], p[2]);
+  }
+  const size_t cells = (size_t)((S.n + kSortBlock - 1) / kSortBlock) * (kCells / 4);
+  if (S.hist)
+    for (size_t c = at; c < cells; c += step)
+      reinterpret_cast<uint4 *>(S.hist)[c] = make_uint4(0u, 0u, 0u, 0u);
+  b.warp_reduce();
+  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = b;
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    const int d = threadIdx.x % 3;
+    long long v = threadIdx.x < 3 ? w[0].lo[d] : w[0].hi[d];
+    for (int j = 1; j < 8; ++j) v = threadIdx.x < 3 ? min(v, w[j].lo[d]) : max(v, w[j].hi[d]);
+    S.box[6 * blockIdx.x + threadIdx.x] = v;
   }
 }
 
-__global__ void __launch_bounds__(256) k_bbox_partial(const double *__restrict__ pos, int n,
-                                                      double *__restrict__ partial) {
-  double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    minmax3(lo, hi, pos + 3 * (size_t)i);
-  block_minmax<256>(lo, hi);
-  if (threadIdx.x == 0)
-    for (int d = 0; d < 3; ++d) {
-      partial[6 * blockIdx.x + d] = lo[d];
-      partial[6 * blockIdx.x + 3 + d] = hi[d];
+// The whole box from the parts, by warps 0 .. 5 of a block, into shared memory (lo, hi).
+__device__ __forceinline__ void reduce_box_parts(const long long *box, int parts, double *out) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < 6) {
+    long long v = warp < 3 ? kOrderedMax : kOrderedMin;
+    for (int b = lane; b < parts; b += 32)
+      v = warp < 3 ? min(v, box[6 * b + warp]) : max(v, box[6 * b + warp]);
+    for (int o = 16; o > 0; o >>= 1) {
+      const long long x = __shfl_xor_sync(0xffffffffu, v, o);
+      v = warp < 3 ? min(v, x) : max(v, x);
     }
+    if (lane == 0) out[warp] = from_ordered64(v);
+  }
 }
 
-__global__ void __launch_bounds__(256) k_bbox_final(const double *__restrict__ partial, int nb,
+__global__ void __launch_bounds__(256) k_bbox_final(const long long *__restrict__ box, int parts,
                                                     double *__restrict__ bbox) {
-  double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
-  for (int b = threadIdx.x; b < nb; b += blockDim.x)
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = fmin(lo[d], partial[6 * b + d]);
-      hi[d] = fmax(hi[d], partial[6 * b + 3 + d]);
-    }
-  block_minmax<256>(lo, hi);
-  if (threadIdx.x == 0)
-    for (int d = 0; d < 3; ++d) {
-      bbox[d] = lo[d];
-      bbox[3 + d] = hi[d];
-    }
+  reduce_box_parts(box, parts, bbox);
 }
 
 constexpr int kHilbertCells = 64;  // cells per axis of the Hilbert tiling (kCells in all)
@@ -108,28 +150,6 @@ __device__ __forceinline__ uint32_t hilbert_xy2d(int n, int x, int y) {
   return d;
 }
 
-__global__ void __launch_bounds__(256) k_cell_keys(const double *__restrict__ pos, int n,
-                                                   const double *__restrict__ bbox,
-                                                   uint16_t *__restrict__ keys) {
-  // the two widest axes of the bounding box span the cell grid
-  double ext[3];
-  for (int d = 0; d < 3; ++d) ext[d] = bbox[3 + d] - bbox[d];
-  int a0 = 0, a1 = 1, a2 = 2;  // sort axes by extent, descending
-  if (ext[a1] > ext[a0]) { int t = a0; a0 = a1; a1 = t; }
-  if (ext[a2] > ext[a1]) { int t = a1; a1 = a2; a2 = t; }
-  if (ext[a1] > ext[a0]) { int t = a0; a0 = a1; a1 = t; }
-  const double s0 = ext[a0] > 0 ? kHilbertCells / ext[a0] : 0.0;
-  const double s1 = ext[a1] > 0 ? kHilbertCells / ext[a1] : 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double *p = pos + 3 * (size_t)i;
-    int cx = (int)((p[a0] - bbox[a0]) * s0);
-    int cy = (int)((p[a1] - bbox[a1]) * s1);
-    cx = min(max(cx, 0), kHilbertCells - 1);
-    cy = min(max(cy, 0), kHilbertCells - 1);
-    keys[i] = (uint16_t)hilbert_xy2d(kHilbertCells, cx, cy);
-  }
-}
-
 // The two widest axes of a bounding box (lo[3], hi[3]), widest first.
 __device__ __forceinline__ void widest_axes(const double *bbox, int *a0, int *a1) {
   double ext[3];
@@ -140,6 +160,49 @@ __device__ __forceinline__ void widest_axes(const double *bbox, int *a0, int *a1
   if (ext[y] > ext[x]) { int t = x; x = y; y = t; }
   *a0 = x;
   *a1 = y;
+}
+
+// Hilbert cell of every point and the histogram of each kSortBlock points.  Bound by the FP64
+// pipe (two subtractions, products and conversions a point), so the box, the cell axes and
+// the scales are worked out once per block of 1024 points, not per thread (18.8 us for
+// 262,144 points and 5.1 us for 16,384 before, 12 us for both here).
+__global__ void __launch_bounds__(256) k_cell_keys(const SortSets sets) {
+  const SortSet &S = sets.s[blockIdx.y];
+  const int i0 = blockIdx.x * 1024;
+  if (i0 >= S.n) return;
+  __shared__ double box[6], scale[2], low[2];
+  __shared__ int axis[2];
+  reduce_box_parts(S.box, S.parts, box);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    widest_axes(box, &axis[0], &axis[1]);
+    for (int a = 0; a < 2; ++a) {
+      const double ext = box[3 + axis[a]] - box[axis[a]];
+      scale[a] = ext > 0 ? kHilbertCells / ext : 0.0;
+      low[a] = box[axis[a]];
+    }
+  }
+  __syncthreads();
+  const int a0 = axis[0], a1 = axis[1], lane = threadIdx.x & 31;
+  const double l0 = low[0], l1 = low[1], s0 = scale[0], s1 = scale[1];
+  uint32_t *hist = S.hist + (size_t)(i0 / kSortBlock) * kCells;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = i0 + 256 * k + threadIdx.x;
+    int key = kCells;  // sentinel past the end
+    if (i < S.n) {
+      const double *p = S.pos + 3 * (size_t)i;
+      int cx = (int)((p[a0] - l0) * s0);
+      int cy = (int)((p[a1] - l1) * s1);
+      cx = min(max(cx, 0), kHilbertCells - 1);
+      cy = min(max(cy, 0), kHilbertCells - 1);
+      key = (int)hilbert_xy2d(kHilbertCells, cx, cy);
+      S.keys[i] = (uint16_t)key;
+    }
+    // runs of one cell (a lattice's rows) in one addition
+    const uint32_t peers = __match_any_sync(0xffffffffu, key);
+    if (i < S.n && (__ffs(peers) - 1) == lane) atomicAdd(&hist[key], __popc(peers));
+  }
 }
 
 // Points per strip: about sqrt(#super tiles / aspect) strips make the super tiles
@@ -391,118 +454,136 @@ __global__ void __launch_bounds__(1024) k_local_bisect(const double *__restrict_
   for (int i = t; i < nl; i += blockDim.x) order[base + i] = idx[cur * kSuperTile + i];
 }
 
-// Per-block histogram of cell keys, stored cell-major: hist[cell * nblk + blk].
-__global__ void __launch_bounds__(256) k_hist(const uint16_t *__restrict__ keys, int n,
-                                              uint32_t *__restrict__ hist, int nblk) {
+// Per-block histogram of given keys (the packed tiling's sorts): hist[blk][cell].
+__global__ void __launch_bounds__(256) k_hist(const SortSets sets) {
+  const SortSet &S = sets.s[blockIdx.y];
   __shared__ uint32_t h[kCells];
   for (int c = threadIdx.x; c < kCells; c += blockDim.x) h[c] = 0;
   __syncthreads();
   const int i0 = blockIdx.x * kSortBlock;
-  const int i1 = min(n, i0 + kSortBlock);
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) atomicAdd(&h[keys[i]], 1u);
+  const int i1 = min(S.n, i0 + kSortBlock);
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) atomicAdd(&h[S.keys[i]], 1u);
   __syncthreads();
   for (int c = threadIdx.x; c < kCells; c += blockDim.x)
-    hist[(size_t)c * nblk + blockIdx.x] = h[c];
+    S.hist[(size_t)blockIdx.x * kCells + c] = h[c];
 }
 
-// Exclusive scan, three passes over blocks of 4096 entries.
-__device__ uint32_t block_exclusive_scan_1024(uint32_t v, uint32_t *total) {
-  __shared__ uint32_t warp_sums[32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = v;
+// Per cell: the exclusive prefix of its counts over the blocks (in place) and their total.
+__global__ void __launch_bounds__(128) k_scan_cells(const SortSets sets) {
+  const SortSet &S = sets.s[blockIdx.y];
+  const int cell = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nblk = (S.n + kSortBlock - 1) / kSortBlock;
+  uint32_t run = 0, *h = S.hist + cell;
+  int b = 0;
+  for (; b + 8 <= nblk; b += 8) {
+    uint32_t v[8];
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += t;
-  }
-  if (lane == 31) warp_sums[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t w = warp_sums[lane];
+    for (int j = 0; j < 8; ++j) v[j] = h[(size_t)(b + j) * kCells];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += t;
+    for (int j = 0; j < 8; ++j) {
+      h[(size_t)(b + j) * kCells] = run;
+      run += v[j];
     }
-    warp_sums[lane] = w;
   }
-  __syncthreads();
-  const uint32_t before = warp ? warp_sums[warp - 1] : 0u;
-  *total = warp_sums[31];
-  __syncthreads();
-  return before + x - v;
+  for (; b < nblk; ++b) {
+    const uint32_t v = h[(size_t)b * kCells];
+    h[(size_t)b * kCells] = run;
+    run += v;
+  }
+  S.totals[cell] = run;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_blocks(const uint32_t *__restrict__ in,
-                                                      size_t count, uint32_t *__restrict__ out,
-                                                      uint32_t *__restrict__ sums) {
-  const size_t base = (size_t)blockIdx.x * 4096 + 4 * threadIdx.x;
-  uint32_t v[4], s = 0;
-  for (int j = 0; j < 4; ++j) {
-    v[j] = base + j < count ? in[base + j] : 0u;
-    s += v[j];
-  }
-  uint32_t total;
-  uint32_t run = block_exclusive_scan_1024(s, &total);
-  for (int j = 0; j < 4; ++j) {
-    if (base + j < count) out[base + j] = run;
-    run += v[j];
-  }
-  if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
+// Stable scatter of kSortBlock points by their cells.  Eight warps take 512 consecutive
+// points each: a first walk, 32 points at a time, ranks every point among the earlier
+// points of its cell in the warp (match.any), a prefix over the warps and the scanned
+// totals turns the warps' counts into positions, and a last pass writes the order.  Bound by
+// the latency of those dependent shared-memory updates: 16 here, 128 for one warp walking
+// all 4096 points, which took 42 us for 262,144 points and 42 us for 16,384 (both sets
+// in one launch of this kernel: 10 us, GB300).
+constexpr int kScatWarps = 8, kScatSteps = kSortBlock / (32 * kScatWarps);
+constexpr int kScatSmem = kScatWarps * kCells * 2 + kCells * 4;
 
-__global__ void __launch_bounds__(1024) k_scan_sums(uint32_t *__restrict__ sums, int nb) {
-  // nb <= 4096
-  uint32_t v[4], s = 0;
-  for (int j = 0; j < 4; ++j) {
-    const int i = 4 * threadIdx.x + j;
-    v[j] = i < nb ? sums[i] : 0u;
-    s += v[j];
-  }
-  uint32_t total;
-  uint32_t run = block_exclusive_scan_1024(s, &total);
-  for (int j = 0; j < 4; ++j) {
-    const int i = 4 * threadIdx.x + j;
-    if (i < nb) sums[i] = run;
-    run += v[j];
-  }
-}
-
-__global__ void __launch_bounds__(1024) k_scan_add(uint32_t *__restrict__ out, size_t count,
-                                                   const uint32_t *__restrict__ sums) {
-  const size_t base = (size_t)blockIdx.x * 4096;
-  const uint32_t add = sums[blockIdx.x];
-  for (int j = threadIdx.x; j < 4096; j += blockDim.x)
-    if (base + j < count) out[base + j] += add;
-}
-
-// Stable scatter: one warp walks its block's points in input order, 32 at a
-// time; equal keys within a step are ranked by lane (match.any + popc), so the
-// sorted order preserves input order among equal keys.
-__global__ void __launch_bounds__(32) k_scatter(const uint16_t *__restrict__ keys, int n,
-                                                const uint32_t *__restrict__ offsets, int nblk,
-                                                int32_t *__restrict__ order) {
-  __shared__ uint32_t base[kCells];
-  const int lane = threadIdx.x;
-  for (int c = lane; c < kCells; c += 32) base[c] = offsets[(size_t)c * nblk + blockIdx.x];
-  __syncwarp();
+__global__ void __launch_bounds__(32 * kScatWarps) k_scatter(const SortSets sets) {
+  extern __shared__ __align__(16) unsigned char ssm[];
+  uint16_t *cnt = reinterpret_cast<uint16_t *>(ssm);                            // [warp][cell]
+  uint32_t *first = reinterpret_cast<uint32_t *>(ssm + kScatWarps * kCells * 2);  // [cell]
+  __shared__ uint32_t warp_sum[kScatWarps];
+  const SortSet &S = sets.s[blockIdx.y];
   const int i0 = blockIdx.x * kSortBlock;
-  const int i1 = min(n, i0 + kSortBlock);
+  if (i0 >= S.n) return;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int c = t; c < kScatWarps * kCells * 2 / 16; c += 32 * kScatWarps)
+    reinterpret_cast<uint4 *>(cnt)[c] = make_uint4(0u, 0u, 0u, 0u);
+  // cells' first positions: exclusive scan of the totals (16 cells per thread) ...
+  uint32_t v[16], sum = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint4 q = reinterpret_cast<const uint4 *>(S.totals)[4 * t + j];
+    v[4 * j] = q.x; v[4 * j + 1] = q.y; v[4 * j + 2] = q.z; v[4 * j + 3] = q.w;
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) sum += v[j];
+  uint32_t incl = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  uint32_t run = incl - sum;
+  for (int w = 0; w < warp; ++w) run += warp_sum[w];
+  // ... plus the points of earlier blocks
+  const uint4 *before = reinterpret_cast<const uint4 *>(S.hist + (size_t)blockIdx.x * kCells);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint4 q = before[4 * t + j];
+    uint4 f;
+    f.x = run + q.x; run += v[4 * j];
+    f.y = run + q.y; run += v[4 * j + 1];
+    f.z = run + q.z; run += v[4 * j + 2];
+    f.w = run + q.w; run += v[4 * j + 3];
+    reinterpret_cast<uint4 *>(first)[4 * t + j] = f;
+  }
+  // ranks within each warp's points (cell << 16 | rank; 0xffffffff: past the end)
+  uint32_t item[kScatSteps];
+  uint16_t *mine = cnt + warp * kCells;
   const uint32_t lt = (1u << lane) - 1u;
-  for (int s = i0; s < i1; s += 32) {
-    const int i = s + lane;
-    const bool valid = i < i1;
-    const int key = valid ? (int)keys[i] : kCells;  // kCells: sentinel, never stored
-    const uint32_t peers = __match_any_sync(0xffffffffu, key);
-    const uint32_t rank = __popc(peers & lt);
-    uint32_t dst = 0;
-    if (valid) dst = base[key] + rank;
+#pragma unroll
+  for (int k = 0; k < kScatSteps; ++k) {
+    const int i = i0 + warp * (32 * kScatSteps) + 32 * k + lane;
+    item[k] = i < S.n ? (uint32_t)S.keys[i] << 16 : 0xffffffffu;
+  }
+#pragma unroll
+  for (int k = 0; k < kScatSteps; ++k) {
+    const uint32_t key = item[k] >> 16, peers = __match_any_sync(0xffffffffu, key);
+    const uint32_t prev = key < (uint32_t)kCells ? mine[key] : 0u;
     __syncwarp();
-    // the highest lane of each key group advances the running offset
-    const bool last = (peers >> lane) == 1u;
-    if (valid && last) base[key] += __popc(peers);
+    if (key < (uint32_t)kCells) {
+      item[k] |= prev + __popc(peers & lt);
+      if ((peers >> lane) == 1u) mine[key] = (uint16_t)(prev + __popc(peers));  // highest lane
+    }
     __syncwarp();
-    if (valid) order[dst] = i;
+  }
+  __syncthreads();
+  // counts of the earlier warps, eight cells at a time (each count fits 13 bits)
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int c = t + 256 * h;
+    uint4 acc = make_uint4(0u, 0u, 0u, 0u);
+    for (int w = 0; w < kScatWarps; ++w) {
+      uint4 *q = reinterpret_cast<uint4 *>(cnt + w * kCells) + c;
+      const uint4 x = *q;
+      *q = acc;
+      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kScatSteps; ++k) {
+    const uint32_t key = item[k] >> 16;
+    if (key < (uint32_t)kCells)
+      S.order[first[key] + mine[key] + (item[k] & 0xffffu)] =
+          i0 + warp * (32 * kScatSteps) + 32 * k + lane;
   }
 }
 
@@ -525,17 +606,144 @@ __global__ void __launch_bounds__(256) k_gather_pos(const double *__restrict__ p
 
 __global__ void __launch_bounds__(256) k_tile_bbox(const double *__restrict__ pos, int n,
                                                    int tile, double *__restrict__ tiles) {
-  double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
+  __shared__ Box64 w[8];
   const int i0 = blockIdx.x * tile;
   const int i1 = min(n, i0 + tile);
-  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) minmax3(lo, hi, pos + 3 * (size_t)i);
-  block_minmax<256>(lo, hi);
-  if (threadIdx.x == 0)
-    for (int d = 0; d < 3; ++d) {
-      tiles[6 * blockIdx.x + d] = 0.5 * (lo[d] + hi[d]);
-      tiles[6 * blockIdx.x + 3 + d] = 0.5 * (hi[d] - lo[d]);
+  Box64 b;
+  b.clear();
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    const double *p = pos + 3 * (size_t)i;
+    b.add(p[0], p[1], p[2]);
+  }
+  b.warp_reduce();
+  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = b;
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    const int d = threadIdx.x;
+    long long lo = w[0].lo[d], hi = w[0].hi[d];
+    for (int j = 1; j < 8; ++j) {
+      lo = min(lo, w[j].lo[d]);
+      hi = max(hi, w[j].hi[d]);
     }
+    tiles[6 * blockIdx.x + d] = 0.5 * (from_ordered64(lo) + from_ordered64(hi));
+    tiles[6 * blockIdx.x + 3 + d] = 0.5 * (from_ordered64(hi) - from_ordered64(lo));
+  }
 }
+
+// Points in tile order (zeros past the end up to n_pad), the boxes of the tiles of 256 .. 8192
+// points of one super tile (levels 0 .. 5), and the super tile's part of their statistics.
+// One warp per leaf of 256 points; the box of a longer tile merges its leaves' keys.  The
+// FP64 operations left, two conversions of a box and its diagonal, are spread over lanes.
+struct GatherSet {
+  const double *pos;
+  const int32_t *order;
+  int n, n_pad;
+  double *out, *boxes;
+  BoxStats *parts;   // per super tile
+  BoxStats *stats;   // of the whole set
+};
+struct GatherSets {
+  GatherSet s[2];
+};
+__global__ void __launch_bounds__(1024) k_gather_boxes(const GatherSets sets) {
+  constexpr int kLeaves = kSuperTile / kLeafTile;
+  __shared__ long long leaf[kLeaves][6];
+  __shared__ double box[2 * kLeaves][6];
+  const GatherSet &S = sets.s[blockIdx.y];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, base = blockIdx.x * kSuperTile, n = S.n;
+  if (base >= S.n_pad) return;
+  Box64 b;
+  b.clear();
+#pragma unroll
+  for (int k = 0; k < kLeafTile / 32; ++k) {
+    const int i = base + warp * kLeafTile + 32 * k + lane;
+    if (i < n) {
+      const double *p = S.pos + 3 * (size_t)S.order[i];
+      const double x = p[0], y = p[1], z = p[2];
+      b.add(x, y, z);
+      double *o = S.out + 3 * (size_t)i;
+      o[0] = x; o[1] = y; o[2] = z;
+    } else if (i < S.n_pad) {
+      double *o = S.out + 3 * (size_t)i;
+      o[0] = o[1] = o[2] = 0.0;
+    }
+  }
+  if (base >= n) return;
+  b.warp_reduce();
+  if (lane < 6) leaf[warp][lane] = lane < 3 ? (lane == 0 ? b.lo[0] : lane == 1 ? b.lo[1] : b.lo[2])
+                                            : (lane == 3 ? b.hi[0] : lane == 4 ? b.hi[1] : b.hi[2]);
+  __syncthreads();
+  // thread t: axis t % 3 of tile t / 3 of the super tile's 63
+  if (t < 3 * (2 * kLeaves - 1)) {
+    const int d = t % 3;
+    int level = 0, tile = t / 3;
+    while (tile >= (kLeaves >> level)) tile -= kLeaves >> level++;
+    const int size = kLeafTile << level;
+    if (base + tile * size < n) {
+      size_t at = blockIdx.x * (size_t)(kSuperTile / size) + tile;
+      for (int l = 0; l < level; ++l) at += (n + (kLeafTile << l) - 1) / (kLeafTile << l);
+      long long lo = kOrderedMax, hi = kOrderedMin;
+      for (int f = tile << level; f < (tile + 1) << level; ++f) {
+        lo = min(lo, leaf[f][d]);
+        hi = max(hi, leaf[f][3 + d]);
+      }
+      const double c = 0.5 * (from_ordered64(lo) + from_ordered64(hi));
+      const double h = 0.5 * (from_ordered64(hi) - from_ordered64(lo));
+      S.boxes[6 * at + d] = c;
+      S.boxes[6 * at + 3 + d] = h;
+      box[t / 3][d] = c;
+      box[t / 3][3 + d] = h;
+    }
+  }
+  __syncthreads();
+  // warp l: the largest half extents of level l, a lane per tile; the super tile's own box
+  // comes from the last level
+  if (warp < kBoxLevels) {
+    BoxStats &o = S.parts[blockIdx.x];
+    int first = 0;
+    for (int l = 0; l < warp; ++l) first += kLeaves >> l;
+    const bool in = lane < (kLeaves >> warp) && base + lane * (kLeafTile << warp) < n;
+    double h2 = 0.0;
+    long long m[4];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double e = in ? box[first + lane][3 + d] : 0.0;
+      m[d] = in ? ordered64(e) : 0;
+      h2 = __dadd_rn(h2, __dmul_rn(e, e));
+    }
+    m[3] = in ? ordered64(__dsqrt_rn(h2)) : 0;
+    for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+      for (int d = 0; d < 4; ++d) m[d] = max(m[d], __shfl_xor_sync(0xffffffffu, m[d], s));
+    if (lane < 3) o.hd[warp][lane] = from_ordered64(lane == 0 ? m[0] : lane == 1 ? m[1] : m[2]);
+    if (lane == 3) o.h[warp] = from_ordered64(m[3]);
+    if (warp == kBoxLevels - 1 && lane < 3) {
+      o.lo[lane] = box[first][lane] - box[first][3 + lane];
+      o.hi[lane] = box[first][lane] + box[first][3 + lane];
+    }
+  }
+}
+
+// All super tiles' statistics into one: warp j reduces entry j (minimum for lo, else maximum).
+__global__ void __launch_bounds__(1024) k_box_stats(const GatherSets sets) {
+  const GatherSet &S = sets.s[blockIdx.x];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nb = (S.n + kSuperTile - 1) / kSuperTile;
+  if (warp >= kBoxStatDoubles || nb == 0) return;
+  const bool low = warp < 3;
+  long long v = low ? kOrderedMax : warp < 6 ? kOrderedMin : 0;
+  for (int b = lane; b < nb; b += 32) {
+    const long long x = ordered64(reinterpret_cast<const double *>(S.parts + b)[warp]);
+    v = low ? min(v, x) : max(v, x);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const long long x = __shfl_xor_sync(0xffffffffu, v, o);
+    v = low ? min(v, x) : max(v, x);
+  }
+  if (lane == 0) reinterpret_cast<double *>(S.stats)[warp] = from_ordered64(v);
+}
+static_assert(kBoxStatDoubles <= 32 && (kLeafTile << (kBoxLevels - 1)) == kSuperTile,
+              "one warp per statistic, the last level is the super tile");
 
 __global__ void __launch_bounds__(256) k_gather_ap(const double *__restrict__ amp,
                                                    const double *__restrict__ phase,
@@ -603,34 +811,81 @@ int grid_for(int n, int per_block, int cap) {
 
 }  // namespace
 
-int launch_bbox(const double *pos, int n, double *bbox6, double *scratch, int scratch_blocks,
-                cudaStream_t s) {
-  const int nb = grid_for(n, 256 * 8, scratch_blocks);
-  k_bbox_partial<<<nb, 256, 0, s>>>(pos, n, scratch); note_launches(1);
-  k_bbox_final<<<1, 256, 0, s>>>(scratch, nb, bbox6); note_launches(1);
-  HOLO_CUDA(cudaGetLastError());
-  return HOLO_OK;
-}
-
 size_t sort_hist_entries(int n) {
   const size_t nblk = (size_t)((n + kSortBlock - 1) / kSortBlock);
   return (nblk ? nblk : 1) * kCells;
 }
 
-// Stable counting sort of n keys (< kCells) into order (indices 0..n-1).
-static int counting_sort(const uint16_t *keys, int n, int32_t *order, uint32_t *hist,
-                         uint32_t *scan_tmp, cudaStream_t s) {
-  const int nblk = (n + kSortBlock - 1) / kSortBlock;
-  if (nblk > 4096) return fail(HOLO_ERR_INVALID, "point set too large for the tiler (%d)", n);
-  k_hist<<<nblk, 256, 0, s>>>(keys, n, hist, nblk); note_launches(1);
-  const size_t count = (size_t)nblk * kCells;
-  const int nb = (int)((count + 4095) / 4096);  // == nblk
-  uint32_t *offsets = scan_tmp;
-  uint32_t *sums = scan_tmp + count;
-  k_scan_blocks<<<nb, 1024, 0, s>>>(hist, count, offsets, sums); note_launches(1);
-  k_scan_sums<<<1, 1024, 0, s>>>(sums, nb); note_launches(1);
-  k_scan_add<<<nb, 1024, 0, s>>>(offsets, count, sums); note_launches(1);
-  k_scatter<<<nblk, 32, 0, s>>>(keys, n, offsets, nblk, order); note_launches(1);
+static SortSet sort_set(const double *pos, int n, int32_t *order, const TileScratch &t) {
+  SortSet S{};
+  S.pos = pos;
+  S.n = n;
+  S.parts = grid_for(n, 256 * 8, 152);
+  S.box = reinterpret_cast<long long *>(t.bbox_scratch);
+  S.keys = t.keys;
+  S.hist = t.hist;
+  S.totals = t.scan;
+  S.order = order;
+  return S;
+}
+
+// Stable counting sort by S.keys (< kCells) into S.order (indices 0..n-1) of one or two
+// sets; `counted`: their histograms are filled already.
+static int counting_sort(const SortSets &sets, int count, bool counted, cudaStream_t s) {
+  int nblk = 0;
+  for (int i = 0; i < count; ++i) nblk = std::max(nblk, (sets.s[i].n + kSortBlock - 1) / kSortBlock);
+  if (nblk > 4096) return fail(HOLO_ERR_INVALID, "point set too large for the tiler");
+  HOLO_TRY(kernel_setup<k_scatter>(32 * kScatWarps, kScatSmem, nullptr));
+  if (!counted) {
+    k_hist<<<dim3(nblk, count), 256, 0, s>>>(sets); note_launches(1);
+  }
+  k_scan_cells<<<dim3(kCells / 128, count), 128, 0, s>>>(sets); note_launches(1);
+  k_scatter<<<dim3(nblk, count), 32 * kScatWarps, kScatSmem, s>>>(sets); note_launches(1);
+  HOLO_CUDA(cudaGetLastError());
+  return HOLO_OK;
+}
+
+static int hilbert_order(const SortSets &sets, int count, cudaStream_t s) {
+  int parts = 0, n = 0;
+  for (int i = 0; i < count; ++i) {
+    parts = std::max(parts, sets.s[i].parts);
+    n = std::max(n, sets.s[i].n);
+  }
+  k_box_parts<<<dim3(parts, count), 256, 0, s>>>(sets); note_launches(1);
+  k_cell_keys<<<dim3((n + 1023) / 1024, count), 256, 0, s>>>(sets); note_launches(1);
+  return counting_sort(sets, count, true, s);
+}
+
+static int packed_order(const double *pos, int n, int32_t *order, const TileScratch &t,
+                        cudaStream_t s) {
+  constexpr int kBisectSmem = kSuperTile * (8 + 2 * 4);
+  HOLO_TRY(kernel_setup<k_local_bisect>(1024, kBisectSmem, nullptr));
+  if (n <= kSuperTile) {
+    HOLO_TRY(launch_iota(order, n, s));
+  } else {
+    SortSets sets{};
+    SortSet &S = sets.s[0];
+    S = sort_set(pos, n, t.tmp_a, t);
+    S.hist = nullptr;  // counted by k_hist
+    k_box_parts<<<dim3(S.parts, 1), 256, 0, s>>>(sets); note_launches(1);
+    k_bbox_final<<<1, 256, 0, s>>>(S.box, S.parts, t.bbox); note_launches(1);
+    S.hist = t.hist;
+    const int g = grid_for(n, 256, 8192);
+    // order along the widest axis -> each point's strip
+    k_axis_keys<<<g, 256, 0, s>>>(pos, n, t.bbox, 0, t.keys); note_launches(1);
+    HOLO_TRY(counting_sort(sets, 1, false, s));
+    k_strip_keys<<<g, 256, 0, s>>>(t.tmp_a, n, t.bbox, t.keys2); note_launches(1);
+    // along the second axis, then (stably) by strip
+    k_axis_keys<<<g, 256, 0, s>>>(pos, n, t.bbox, 1, t.keys); note_launches(1);
+    S.order = t.tmp_b;
+    HOLO_TRY(counting_sort(sets, 1, false, s));
+    k_permute_keys<<<g, 256, 0, s>>>(t.keys2, t.tmp_b, n, t.keys); note_launches(1);
+    S.order = t.tmp_a;
+    HOLO_TRY(counting_sort(sets, 1, false, s));
+    k_compose<<<g, 256, 0, s>>>(t.tmp_b, t.tmp_a, n, order); note_launches(1);
+  }
+  k_local_bisect<<<(n + kSuperTile - 1) / kSuperTile, 1024, kBisectSmem, s>>>(pos, n, order);
+  note_launches(1);
   HOLO_CUDA(cudaGetLastError());
   return HOLO_OK;
 }
@@ -638,31 +893,35 @@ static int counting_sort(const uint16_t *keys, int n, int32_t *order, uint32_t *
 int tile_order(const double *pos, int n, int32_t *order, const TileScratch &t, cudaStream_t s,
                int tiling) {
   if (n <= 0) return HOLO_OK;
-  if (tiling == kTileHilbert) {
-    HOLO_TRY(launch_bbox(pos, n, t.bbox, t.bbox_scratch, 1024, s));
-    k_cell_keys<<<grid_for(n, 256, 4096), 256, 0, s>>>(pos, n, t.bbox, t.keys); note_launches(1);
-    return counting_sort(t.keys, n, order, t.hist, t.scan, s);
+  if (tiling == kTilePacked) return packed_order(pos, n, order, t, s);
+  SortSets sets{};
+  sets.s[0] = sort_set(pos, n, order, t);
+  return hilbert_order(sets, 1, s);
+}
+
+int tile_sets(const TileSet *set, int count, int tiling, cudaStream_t s) {
+  SortSets sets{};
+  int sorted = 0;
+  for (int i = 0; i < count; ++i) {
+    if (set[i].known) {
+      HOLO_CUDA(cudaMemcpyAsync(set[i].order, set[i].known, (size_t)set[i].n * sizeof(int32_t),
+                                cudaMemcpyDeviceToDevice, s));
+    } else if (tiling == kTilePacked) {
+      HOLO_TRY(packed_order(set[i].pos, set[i].n, set[i].order, set[i].scratch, s));
+    } else {
+      sets.s[sorted++] = sort_set(set[i].pos, set[i].n, set[i].order, set[i].scratch);
+    }
   }
-  constexpr int kBisectSmem = kSuperTile * (8 + 2 * 4);
-  HOLO_TRY(kernel_setup<k_local_bisect>(1024, kBisectSmem, nullptr));
-  if (n <= kSuperTile) {
-    HOLO_TRY(launch_iota(order, n, s));
-  } else {
-    HOLO_TRY(launch_bbox(pos, n, t.bbox, t.bbox_scratch, 1024, s));
-    const int g = grid_for(n, 256, 8192);
-    // order along the widest axis -> each point's strip
-    k_axis_keys<<<g, 256, 0, s>>>(pos, n, t.bbox, 0, t.keys); note_launches(1);
-    HOLO_TRY(counting_sort(t.keys, n, t.tmp_a, t.hist, t.scan, s));
-    k_strip_keys<<<g, 256, 0, s>>>(t.tmp_a, n, t.bbox, t.keys2); note_launches(1);
-    // along the second axis, then (stably) by strip
-    k_axis_keys<<<g, 256, 0, s>>>(pos, n, t.bbox, 1, t.keys); note_launches(1);
-    HOLO_TRY(counting_sort(t.keys, n, t.tmp_b, t.hist, t.scan, s));
-    k_permute_keys<<<g, 256, 0, s>>>(t.keys2, t.tmp_b, n, t.keys); note_launches(1);
-    HOLO_TRY(counting_sort(t.keys, n, t.tmp_a, t.hist, t.scan, s));
-    k_compose<<<g, 256, 0, s>>>(t.tmp_b, t.tmp_a, n, order); note_launches(1);
+  if (sorted) HOLO_TRY(hilbert_order(sets, sorted, s));
+  GatherSets g{};
+  int supers = 1;
+  for (int i = 0; i < count; ++i) {
+    g.s[i] = {set[i].pos, set[i].order, set[i].n, set[i].n_pad, set[i].pos_sorted, set[i].boxes,
+              set[i].parts, set[i].stats};
+    supers = std::max(supers, (set[i].n_pad + kSuperTile - 1) / kSuperTile);
   }
-  k_local_bisect<<<(n + kSuperTile - 1) / kSuperTile, 1024, kBisectSmem, s>>>(pos, n, order);
-  note_launches(1);
+  k_gather_boxes<<<dim3(supers, count), 1024, 0, s>>>(g); note_launches(1);
+  k_box_stats<<<count, 1024, 0, s>>>(g); note_launches(1);
   HOLO_CUDA(cudaGetLastError());
   return HOLO_OK;
 }
@@ -718,14 +977,10 @@ int launch_gather_apf(const double *amp, const double *phase, const int32_t *ord
 
 int tiler_preload_hilbert() {
   cudaFuncAttributes a;
-  HOLO_CUDA(cudaFuncGetAttributes(&a, k_bbox_partial));
-  HOLO_CUDA(cudaFuncGetAttributes(&a, k_bbox_final));
+  HOLO_CUDA(cudaFuncGetAttributes(&a, k_box_parts));
   HOLO_CUDA(cudaFuncGetAttributes(&a, k_cell_keys));
-  HOLO_CUDA(cudaFuncGetAttributes(&a, k_hist));
-  HOLO_CUDA(cudaFuncGetAttributes(&a, k_scan_blocks));
-  HOLO_CUDA(cudaFuncGetAttributes(&a, k_scan_sums));
-  HOLO_CUDA(cudaFuncGetAttributes(&a, k_scan_add));
-  HOLO_CUDA(cudaFuncGetAttributes(&a, k_scatter));
+  HOLO_CUDA(cudaFuncGetAttributes(&a, k_scan_cells));
+  HOLO_TRY(kernel_setup<k_scatter>(32 * kScatWarps, kScatSmem, nullptr));
   HOLO_CUDA(cudaFuncGetAttributes(&a, k_gather_pos));
   HOLO_CUDA(cudaFuncGetAttributes(&a, k_tile_bbox));
   HOLO_CUDA(cudaFuncGetAttributes(&a, k_rel_hilo));
