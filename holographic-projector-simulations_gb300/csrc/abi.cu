@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <memory>
 
+#include "expand_plan.h"
 #include "internal.cuh"
 
 namespace holo {
@@ -361,6 +362,7 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
                         (6 * box_offset((int)N, kBoxLevels) + 6) * sizeof(double), s));
     HOLO_TRY(alloc_plan(pp, (void **)&p->boxes_t,
                         (6 * box_offset((int)M, kBoxLevels) + 6) * sizeof(double), s));
+    p->pair_kernel_only = forced_variant >= 0;
     auto order_both = [&](int tiling, const int32_t *ks, const int32_t *kt) -> int {
       p->tiling_s = ks ? known_tiling_s : tiling;
       p->tiling_t = kt ? known_tiling_t : tiling;
@@ -465,6 +467,25 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
   return HOLO_OK;
 }
 
+// Whether, and on which clusters, a transform of this plan at wave number k runs by cluster
+// expansions: where they take less time than the plan's pair kernel (~20 pairs per clock
+// and SM on the tensor-core builds, ~16 on the CUDA cores, over the waves of its work items).
+ExpandChoice plan_expansion(holo_plan_s *p, double k) {
+  if (p->precision != HOLO_SPLIT32 || p->pair_kernel_only || p->N == 0 || p->M == 0) return {};
+  const Variant V = split_variant(p->variant);
+  if (box_level(V.cs) < 0) return {};  // its tiles do not nest in the clusters
+  if (p->expand_k != k) {
+    const double items = (double)p->n_ttiles * p->splits, per_item = ceil((double)p->n_stiles / p->splits);
+    const double waves = ceil(items / std::max(1, p->grid));
+    const double clocks = waves * per_item * V.cs * V.tt() / (V.tc ? 20.0 : 16.0) *
+                          std::max(1.0, (double)p->grid / p->h->sm_count);
+    p->expand = expand_choose(p->stats_s, p->stats_t, p->N, p->M, box_level(V.cs), box_level(V.tt()),
+                              k, kPairOverhead + clocks / 1.9e9, p->h->sm_count);
+    p->expand_k = k;
+  }
+  return p->expand;
+}
+
 int plan_execute_impl(holo_plan_s *p, int sign, double lambda, const double *amp,
                       const double *phase, double2 *y, int flags, cudaStream_t s) {
   HOLO_TRY(check_sign(sign));
@@ -478,6 +499,8 @@ int plan_execute_impl(holo_plan_s *p, int sign, double lambda, const double *amp
   Scratch tmp(p->h, s);
   const double k = (2.0 * M_PI) / lambda;
   const bool cst = (flags & HOLO_FLAG_CONST_PHASE) != 0;
+  const ExpandChoice ch = cst ? ExpandChoice{} : plan_expansion(p, k);
+  if (ch.use) return expand_execute(p, ch, sign * k, amp, phase, y, s);
   double2 *ap = tmp.get<double2>(p->n_pad);
   double2 *partial = p->splits > 1 ? tmp.get<double2>((size_t)p->splits * p->M) : nullptr;
   if (!ap || (p->splits > 1 && !partial)) return fail(HOLO_ERR_ALLOC, "execute scratch");

@@ -230,7 +230,7 @@ int launch_split_batched(const SplitProblem *probs_dev, const WorkItem *items, i
                          int *queue, int variant, int grid, int *err, cudaStream_t s);
 int split_occupancy(int variant, bool mc, int *ctas_per_sm);
 
-// ---- boxes of a tile order ----------------------------------------------------------
+// ---- cluster expansions (kernel_expand.cu, expand_plan.cu) ---------------------------
 // Boxes of the tiles of 256, 512, .. 8192 consecutive points (levels 0 .. 5) of a tile
 // order, and what the planner needs to know about them.
 constexpr int kBoxLevels = 6;
@@ -265,6 +265,41 @@ struct TileSet {
   TileScratch scratch;     // of its own where it is sorted
 };
 int tile_sets(const TileSet *set, int count, int tiling, cudaStream_t s);
+
+constexpr int kExpandNodes = 128;  // node slots of a cluster
+// Device descriptor of one sum by cluster expansions; target clusters [t0, t0 + nTs).
+struct ExpandProblem {
+  const float *geo_s, *geo_t;        // float-float offsets from the variant's tile centres
+  const float2 *apf_s;               // (phase, amplitude), tile order
+  const double *tiles_s, *tiles_t;   // the variant's tiles (cs sources, tt targets)
+  const double *box_s, *box_t;       // the clusters' boxes (ns sources, nt targets)
+  const int32_t *order_t;
+  double2 *partial;                  // [ssplit][M] when ssplit > 1
+  double2 *y;
+  float *frames;                     // [nTs][nS][12]: (s k e hi, r0) (lo, b0 hi) (e, b0 lo)
+  float *basis;                      // [nTs][nS][8]: the perpendicular axes of each pair
+  float *half_s, *half_t;            // [cluster][4]: half extents along ax and ay, inverses
+  float *shift_s, *shift_t;          // [tile][8]: tile centre - cluster centre, float-float
+  float *cheb;                       // Chebyshev tables of both axes
+  float2 *moments;                   // [ksplit][nTs][nS][kExpandNodes]
+  float *coeffs;                     // [nTs][nS / 32][2][hi, lo][8][64 x 8]: MMA operand
+  int N, M, cs, tt, ns, nt, nS, nT, t0, nTs, slab;  // slab: target clusters per launch
+  int px, py, ax, ay;                // nodes along the coordinate axes ax and ay
+  int ksplit, ssplit;                // shares of a cluster's sources / of the source clusters
+  int cs_log2, tt_log2;
+  float kap;                         // s k / 2
+  double sk;
+};
+int launch_expand(const ExpandProblem &p, int *err, cudaStream_t s);
+// What a sum of N sources and M targets with these box statistics and wave number takes:
+// the cluster levels (at least least_s and least_t, the pair kernel's tiles) and node counts,
+// or use = false where the pair kernels are faster or no clusters hold the truncation bound.
+struct ExpandChoice {
+  bool use = false;
+  int ls = 0, lt = 0, px = 0, py = 0, ax = 0, ay = 0;
+};
+ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int M, int least_s,
+                           int least_t, double k, double direct_seconds, int sm_count);
 
 // kernel_fp64.cu
 int launch_fp64(const Fp64Problem &p, int variant, int grid, bool const_phase, int *err,
@@ -327,6 +362,9 @@ struct holo_plan_s {
   double *boxes_s = nullptr, *boxes_t = nullptr;
   holo::BoxStats stats_s{}, stats_t{};
   double *odd_tiles = nullptr;   // boxes of source tiles that are none of these sizes
+  bool pair_kernel_only = false; // a forced variant: always that kernel
+  double expand_k = 0.0;         // wave number of `expand` (0: not chosen yet)
+  holo::ExpandChoice expand;
   int32_t *order_s = nullptr;    // N (split only)
   int32_t *order_t = nullptr;    // M (split only)
   float *geo_s = nullptr;        // split: float-float offsets from the tile centres
@@ -362,6 +400,7 @@ int plan_create_impl(holo_handle h, const double *u_dev, size_t N, const double 
 int plan_execute_impl(holo_plan_s *p, int sign, double lambda, const double *amp_dev,
                       const double *phase_dev, double2 *y_dev, int flags, cudaStream_t s);
 void plan_release(holo_plan_s *p, cudaStream_t s);
+ExpandChoice plan_expansion(holo_plan_s *p, double k);
 // probe.cu: bracket a pair-evaluation kernel with events while profiling
 int profile_mark(holo_handle h, cudaStream_t s, bool begin);
 }  // namespace holo

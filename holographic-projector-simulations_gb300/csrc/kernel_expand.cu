@@ -1,0 +1,805 @@
+// kernel_expand.cu -- HOLO_SPLIT32 sums between clusters of points by separable expansions.
+//
+// The brute-force sum of superposition::per_block (cuda/superposition.cu:59-154) over every
+// pair of a target cluster T (centre T0) and a source cluster S (centre S0), regrouped.  With
+// D = T0 - S0, r0 = |D|, t' = t - T0, s' = s - S0 the phase of a pair splits into
+//   r = |D + t' - s'| = alpha(t) + beta(s) + psi(t, s),
+//   alpha = |D + t'|,  beta = |D - s'| - r0,  psi = r - alpha - beta,
+// where alpha and beta belong to one point and psi, the mixed part, is small and smooth: its
+// leading term is -(t'_perp . s'_perp) / r0, a few radians over clusters of thousands of
+// points.  G(t, s) = e^{i s k psi} / r is therefore interpolated in both points on px x py
+// Chebyshev nodes of the clusters' boxes (at most 128 of them), and the sum over the pair
+// of clusters becomes
+//   moments    mu_ab = sum_s T_a(x_s) T_b(y_s) a_s e^{i (phi_s + s k beta(s))}
+//   translate  nu    = M G M^T mu   (M: Chebyshev coefficients of the nodal interpolant)
+//   targets    y_t  += e^{i s k alpha(t)} sum_ab T_a(x_t) T_b(y_t) nu_ab:
+// (ns + nt) point evaluations and 128^2 node pairs instead of ns nt pairs.  Moments and
+// targets are products of a matrix of node weights (one row of T_a T_b per point) with one
+// column pair (re, im) per partner cluster: they run on the tensor cores (tcgen05 kind::tf32
+// as three products of TF32 splits, ~2^-21), while the CUDA cores form the phases, in the
+// float-float arithmetic of the pair kernels (split_frame.cuh).
+//
+// Truncation: for e^{i z x} on [-1, 1] the p-node interpolant is off by at most
+// 2 (z / 2)^p / p!; expand_choose (expand_plan.cu) takes the cheapest cluster sizes for which
+// that stays below 8e-7 along each axis, which measured 2e-7 of the field's norm or less.
+//
+// The TF32 accumulator of an MMA drops bits of the running sum at every step, a bias that
+// grows with the length of the chain: the moments kernel moves its accumulator to FP32
+// registers every 64 sources and keeps the small cross products of the splits in an
+// accumulator of their own; the target kernel adds the cross products and the high
+// orders, which are small, before the low ones.
+#include "internal.cuh"
+#include "ptx.cuh"
+
+namespace holo {
+namespace {
+
+#include "split_frame.cuh"
+#include "tc_operand.cuh"
+
+constexpr int kNodes = kExpandNodes;  // node slots of a cluster: rows of the weight matrices
+constexpr int kMaxP = 16;             // nodes along one axis
+constexpr int kGroupT = 64;           // target clusters per moments block (128 MMA columns)
+constexpr int kChunk = 16;            // sources per operand stage of the moments kernel
+constexpr int kSuper = 64;            // sources staged, and summed in the MMA accumulator, at once
+constexpr int kBlockT = 128;          // targets per block of the target kernel
+constexpr int kGroupS = 32;           // source clusters per MMA of the target kernel (64 columns)
+constexpr int kHalfFloats = 8192;     // one staged half (64 nodes, hi and lo) of nu: 32 KB
+
+// Block -> (problem, block of it): the last problem whose first block is <= b.
+template <bool BATCHED>
+__device__ __forceinline__ const ExpandProblem &find_problem(const ExpandProblem &P0,
+                                                             const ExpandProblem *probs,
+                                                             const int *offs, int n, int *item) {
+  if (!BATCHED) {
+    *item = blockIdx.x;
+    return P0;
+  }
+  int lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (offs[mid] <= (int)blockIdx.x) lo = mid; else hi = mid;
+  }
+  *item = blockIdx.x - offs[lo];
+  return probs[lo];
+}
+
+// FP32 frame of one cluster pair as the kernels read it: (s k e hi, r0) (s k e lo, b0 hi)
+// (e, b0 lo) with b0 = s k r0 mod 2 pi, and the axes e1, e2.
+__device__ __forceinline__ void store_frame(const ExpandProblem &P, int pair, const Frame &f) {
+  float4 *q = reinterpret_cast<float4 *>(P.frames + 12 * (size_t)pair);
+  q[0] = make_float4(f.ah[0], f.ah[1], f.ah[2], f.r0f);
+  q[1] = make_float4(f.al[0], f.al[1], f.al[2], f.b0h);
+  q[2] = make_float4(f.ef[0], f.ef[1], f.ef[2], f.b0l);
+  float4 *b = reinterpret_cast<float4 *>(P.basis + 8 * (size_t)pair);
+  b[0] = make_float4(f.e1[0], f.e1[1], f.e1[2], 0.f);
+  b[1] = make_float4(f.e2[0], f.e2[1], f.e2[2], 0.f);
+}
+
+// a = ah + al plus b = bh + bl as a float-float pair.
+__device__ __forceinline__ void add_ff(float ah, float al, float bh, float bl, float &h, float &l) {
+  float s, e;
+  two_sum(ah, bh, s, e);
+  e = __fadd_rn(e, __fadd_rn(al, bl));
+  h = __fadd_rn(s, e);
+  l = __fsub_rn(e, __fsub_rn(h, s));
+}
+
+// s k (c / 2q - c^2 / 8q^3) = kap (c / q) (1 - (c / q) / 4q), kap = s k / 2: the curvature
+// term rho of r = q + rho, c = |perpendicular offset|^2 (the next term, c^3 / 16 q^5, is
+// below 1e-7 rad where expand_choose admits the clusters).
+__device__ __forceinline__ float curvature(float kap, float c, float q, float &iq, float &h) {
+  iq = ptx::rcp_approx(q);
+  h = c * iq;
+  return kap * h * fmaf(-0.25f * h, iq, 1.f);
+}
+
+// ---- set-up: frames of all cluster pairs, offsets of the variant's tile centres from the
+// cluster centres, Chebyshev tables ----
+// Bound by the FP64 pipe's latency (a frame is ~150 dependent FP64 operations): one thread
+// per pair, so a few thousand pairs run in the time of one.
+template <bool BATCHED>
+__global__ void __launch_bounds__(128) k_expand_setup(const ExpandProblem P0,
+                                                      const ExpandProblem *__restrict__ probs,
+                                                      const int *__restrict__ offs, int n_probs) {
+  int item;
+  const ExpandProblem &P = find_problem<BATCHED>(P0, probs, offs, n_probs, &item);
+  int i = item * blockDim.x + threadIdx.x;
+  const int pairs = P.nTs * P.nS;
+  if (i < pairs) {
+    const int T = P.t0 + i / P.nS, S = i % P.nS;
+    Frame f;
+    build_frame(&f, P.box_t + 6 * (size_t)T, P.box_s + 6 * (size_t)S, P.sk);
+    store_frame(P, i, f);
+    return;
+  }
+  i -= pairs;
+  const int tiles_s = (P.N + P.cs - 1) / P.cs, tiles_t = (P.M + P.tt - 1) / P.tt;
+  if (i < tiles_s + tiles_t) {
+    const bool src = i < tiles_s;
+    const int j = src ? i : i - tiles_s;
+    const double *c = (src ? P.tiles_s : P.tiles_t) + 6 * (size_t)j;
+    const double *b = src ? P.box_s + 6 * (size_t)((long long)j * P.cs / P.ns)
+                          : P.box_t + 6 * (size_t)((long long)j * P.tt / P.nt);
+    float *o = (src ? P.shift_s : P.shift_t) + 8 * (size_t)j;
+    for (int d = 0; d < 3; ++d) {
+      const double x = c[d] - b[d];
+      o[d] = (float)x;
+      o[4 + d] = (float)(x - (double)o[d]);
+    }
+    return;
+  }
+  i -= tiles_s + tiles_t;
+  if (i < P.nS + P.nT) {
+    const bool src = i < P.nS;
+    const int j = src ? i : i - P.nS;
+    const double *b = (src ? P.box_s : P.box_t) + 6 * (size_t)j;
+    const float hx = (float)b[3 + P.ax], hy = (float)b[3 + P.ay];
+    reinterpret_cast<float4 *>(src ? P.half_s : P.half_t)[j] =
+        make_float4(hx, hy, hx > 0.f ? 1.f / hx : 0.f, hy > 0.f ? 1.f / hy : 0.f);
+    return;
+  }
+  i -= P.nS + P.nT;
+  if (i < 2 * kMaxP * kMaxP) {
+    // M[a][j] = (2 - delta_a0) / p cos(pi a (2 j + 1) / 2p); row kMaxP^2 + j: node j
+    const int axis = i / (kMaxP * kMaxP), a = i % (kMaxP * kMaxP) / kMaxP, j = i % kMaxP;
+    const int p = axis ? P.py : P.px;
+    float *tab = P.cheb + axis * (kMaxP * kMaxP + kMaxP);
+    if (a < p && j < p)
+      tab[a * kMaxP + j] = (a ? 2.f : 1.f) / (float)p *
+                           cospif((float)((a * (2 * j + 1)) % (4 * p)) / (float)(2 * p));
+    if (a == 0 && j < p) tab[kMaxP * kMaxP + j] = cospif((float)(2 * j + 1) / (float)(2 * p));
+  }
+}
+
+// Float offset of record i of tile-ordered point arrays relative to its cluster's centre.
+__device__ __forceinline__ void cluster_offset(const float *geo, const float *shift, int i,
+                                               int tile_log2, float h[3], float l[3]) {
+  const float2 *g = reinterpret_cast<const float2 *>(geo + 6 * (size_t)i);
+  const float4 *s = reinterpret_cast<const float4 *>(shift + 8 * (size_t)(i >> tile_log2));
+  const float2 g0 = g[0], g1 = g[1], g2 = g[2];
+  const float4 sh = s[0], sl = s[1];
+  add_ff(g0.x, g1.y, sh.x, sl.x, h[0], l[0]);
+  add_ff(g0.y, g2.x, sh.y, sl.y, h[1], l[1]);
+  add_ff(g1.x, g2.y, sh.z, sl.z, h[2], l[2]);
+}
+
+__device__ __forceinline__ float pick(const float v[3], int axis) {
+  return axis == 0 ? v[0] : axis == 1 ? v[1] : v[2];
+}
+
+// T_0 .. T_{p-1}(x) to out[k * stride].
+__device__ __forceinline__ void cheb_row(float x, int p, float *out, int stride) {
+  float t0 = 1.f, t1 = x;
+  for (int k = 0; k < p; ++k) {
+    out[k * stride] = t0;
+    const float t2 = fmaf(2.f * x, t1, -t0);
+    t0 = t1;
+    t1 = t2;
+  }
+}
+
+// ---- moments -------------------------------------------------------------------------------
+// One block: source cluster S, 64 target clusters, a share of S's sources; D[node][column] =
+// sum over sources of weight x (re | im of a e^{i (phi + s k beta)}) for 64 + 64 columns.
+// Per 16 sources every thread forms four sources' phasors for its target cluster (its frame
+// stays in registers) and eight products T_a T_b of its node row, both split into TF32 parts,
+// into one of two operand stages; one thread then issues the stage's six MMAs, and the other
+// stage is filled while they run.
+constexpr int kChebStride = kSuper + 4;  // 16-byte loads of eight rows hit eight bank groups
+struct MomentsSmem {
+  static constexpr size_t a = 0;                                // float [2][hi, lo][128*16]
+  static constexpr size_t b = a + 4 * kNodes * kChunk * 4;      // float [2][hi, lo][128*16]
+  static constexpr size_t cheb = b + 4 * 2 * kGroupT * kChunk * 4;  // float [2][16][68]
+  static constexpr size_t rec = cheb + 2 * kMaxP * kChebStride * 4;  // float [9][64]
+  static constexpr size_t bars = rec + 9 * kSuper * 4;          // uint64 [3]
+  static constexpr size_t misc = bars + 4 * 8;                  // uint32 taddr, abort
+  static constexpr size_t bytes = misc + 16;
+};
+constexpr int kMomThreads = 256;
+
+template <bool BATCHED>
+__global__ void __launch_bounds__(kMomThreads, 2)
+    k_expand_moments(const ExpandProblem P0, const ExpandProblem *__restrict__ probs,
+                     const int *__restrict__ offs, int n_probs, int *err) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  using L = MomentsSmem;
+  constexpr int kStage = 2 * kNodes * kChunk;  // floats of one operand stage (hi, lo)
+  float *sa = reinterpret_cast<float *>(smem + L::a), *sb = reinterpret_cast<float *>(smem + L::b);
+  float *cheb = reinterpret_cast<float *>(smem + L::cheb);
+  float *rec = reinterpret_cast<float *>(smem + L::rec);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::bars);  // free[2], full
+  uint32_t *taddr_slot = reinterpret_cast<uint32_t *>(smem + L::misc);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L::misc + 4);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int b = 0; b < 3; ++b) ptx::mbar_init(&bars[b], 1);
+    *abort_flag = 0;
+    ptx::fence_barrier_init();
+  }
+  if (warp == 0) ptx::tmem_alloc(taddr_slot, 256);
+
+  int item;
+  const ExpandProblem &P = find_problem<BATCHED>(P0, probs, offs, n_probs, &item);
+  const int ks = item % P.ksplit, nTG = (P.nTs + kGroupT - 1) / kGroupT;
+  const int tg = item / P.ksplit % nTG, S = item / P.ksplit / nTG;
+  const int first = S * P.ns, count = min(P.ns, P.N - first);
+  const int n_super = (count + kSuper - 1) / kSuper;
+  const int sc0 = (int)((long long)n_super * ks / P.ksplit);
+  const int sc1 = (int)((long long)n_super * (ks + 1) / P.ksplit);
+  const int px = P.px, py = P.py, np = px * py;
+  const float4 half = reinterpret_cast<const float4 *>(P.half_s)[S];
+  const float kap = P.kap;
+
+  // this thread's target cluster and its share of a chunk's sources
+  const int tq = tid & (kGroupT - 1), quad = tid >> 6, Tl = tg * kGroupT + tq;
+  float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f}, ef[3] = {0.f, 0.f, 0.f}, r0 = 1.f;
+  if (Tl < P.nTs) {
+    const float4 *f = reinterpret_cast<const float4 *>(P.frames + 12 * ((size_t)Tl * P.nS + S));
+    const float4 f0 = f[0], f1 = f[1], f2 = f[2];
+    ah[0] = f0.x; ah[1] = f0.y; ah[2] = f0.z; r0 = f0.w;
+    al[0] = f1.x; al[1] = f1.y; al[2] = f1.z;
+    ef[0] = f2.x; ef[1] = f2.y; ef[2] = f2.z;
+  }
+  // this thread's node row (a, b) of the weight operand and its half of a chunk's sources
+  const int row = tid & (kNodes - 1), khalf = tid >> 7;
+  const float rmask = row < np ? 1.f : 0.f;
+  const float *tab_x = cheb + (row < np ? row / py : 0) * kChebStride;
+  const float *tab_y = cheb + (kMaxP + (row < np ? row % py : 0)) * kChebStride;
+
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tbase = *taddr_slot;
+  constexpr uint32_t idesc = ptx::tc_idesc_tf32(kNodes, 2 * kGroupT);
+  // accumulators of this thread: node 32 (warp % 4) + lane, target clusters 32 (warp / 4) ..
+  const uint32_t trow = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * (warp >> 2));
+  float acc_re[32], acc_im[32];
+#pragma unroll
+  for (int j = 0; j < 32; ++j) acc_re[j] = acc_im[j] = 0.f;
+  auto flush = [&](uint32_t col) {
+    uint32_t v[16];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      ptx::tmem_ld16_nowait(trow + col + (uint32_t)(16 * (h & 1) + kGroupT * (h >> 1)), v);
+      ptx::tmem_wait16(v);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        if (h < 2)
+          acc_re[16 * h + j] += __uint_as_float(v[j]);
+        else
+          acc_im[16 * (h - 2) + j] += __uint_as_float(v[j]);
+      }
+    }
+  };
+
+  int g = 0;  // operand stages filled so far
+  for (int sc = sc0; sc < sc1; ++sc) {
+    // ---- stage 64 sources: offsets from the cluster centre, weights' factors ----
+    __syncthreads();
+    if (tid < 2 * kSuper) {
+      const int i = tid & (kSuper - 1), axis = tid >> 6, idx = first + sc * kSuper + i;
+      float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
+      float2 pa = make_float2(0.f, 0.f);
+      if (idx < P.N) {
+        cluster_offset(P.geo_s, P.shift_s, idx, P.cs_log2, h, l);
+        pa = P.apf_s[idx];
+      }
+      if (axis == 0) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          rec[d * kSuper + i] = h[d];
+          rec[(3 + d) * kSuper + i] = l[d];
+        }
+        rec[6 * kSuper + i] = fmaf(h[0], h[0], fmaf(h[1], h[1], h[2] * h[2]));
+        rec[7 * kSuper + i] = pa.x;
+        rec[8 * kSuper + i] = pa.y;
+        cheb_row(pick(h, P.ax) * half.z, px, cheb + i, kChebStride);
+      } else {
+        cheb_row(pick(h, P.ay) * half.w, py, cheb + kMaxP * kChebStride + i, kChebStride);
+      }
+    }
+    __syncthreads();
+    for (int c = 0; c < kSuper / kChunk; ++c, ++g) {
+      const int st = g & 1;
+      float *a_hi = sa + st * kStage, *a_lo = a_hi + kNodes * kChunk;
+      float *b_hi = sb + st * kStage, *b_lo = b_hi + kNodes * kChunk;
+      if (g >= 2) tc_wait(&bars[st], ((g >> 1) - 1) & 1u, abort_flag, err);
+      // ---- four phasors: sources 4 quad .. of the chunk for this thread's target cluster ----
+      {
+        float q[9][4];
+#pragma unroll
+        for (int f = 0; f < 9; ++f) {
+          const float4 v = *reinterpret_cast<const float4 *>(rec + f * kSuper + kChunk * c + 4 * quad);
+          q[f][0] = v.x; q[f][1] = v.y; q[f][2] = v.z; q[f][3] = v.w;
+        }
+        float re[4], im[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float th[3] = {q[0][j], q[1][j], q[2][j]}, tl[3] = {q[3][j], q[4][j], q[5][j]};
+          float s, e, s2, e2, iq, hq;
+          dot3_ff(ah, al, th, tl, s, e);
+          two_sum(q[7][j], -s, s2, e2);
+          const float ps = fmaf(ef[0], th[0], fmaf(ef[1], th[1], ef[2] * th[2]));
+          const float ph = reduce_two_pi_ff(s2, __fsub_rn(e2, e)) +
+                           curvature(kap, fmaf(-ps, ps, q[6][j]), r0 - ps, iq, hq);
+          re[j] = q[8][j] * ptx::cos_approx(ph);
+          im[j] = q[8][j] * ptx::sin_approx(ph);
+        }
+        const int o = (quad >> 1) * (2 * kGroupT * kTcK) + 32 * (quad & 1);
+        const int ore = o + tc_off(tq, 0), oim = o + tc_off(kGroupT + tq, 0);
+        float hi[4], lo[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          hi[j] = ptx::to_tf32_int(re[j]);
+          lo[j] = ptx::to_tf32_int(__fsub_rn(re[j], hi[j]));
+        }
+        *reinterpret_cast<float4 *>(b_hi + ore) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<float4 *>(b_lo + ore) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          hi[j] = ptx::to_tf32_int(im[j]);
+          lo[j] = ptx::to_tf32_int(__fsub_rn(im[j], hi[j]));
+        }
+        *reinterpret_cast<float4 *>(b_hi + oim) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<float4 *>(b_lo + oim) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      // ---- eight weights: node row `row`, sources 8 khalf .. of the chunk ----
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = kChunk * c + 8 * khalf + 4 * h;
+        const float4 x = *reinterpret_cast<const float4 *>(tab_x + k);
+        const float4 y = *reinterpret_cast<const float4 *>(tab_y + k);
+        const float w[4] = {rmask * x.x * y.x, rmask * x.y * y.y, rmask * x.z * y.z,
+                            rmask * x.w * y.w};
+        float hi[4], lo[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          hi[j] = ptx::to_tf32_int(w[j]);
+          lo[j] = ptx::to_tf32_int(__fsub_rn(w[j], hi[j]));
+        }
+        const int o = khalf * (kNodes * kTcK) + tc_off(row, 4 * h);
+        *reinterpret_cast<float4 *>(a_hi + o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<float4 *>(a_lo + o) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      ptx::fence_proxy_async_smem();
+      ptx::tc_fence_before();
+      __syncthreads();
+      if (tid == 0 && !*abort_flag) {
+        ptx::tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < kChunk / kTcK; ++k) {
+          const uint64_t dah = ptx::tc_smem_desc(a_hi + k * kNodes * kTcK, kTcLbo, kTcSbo);
+          const uint64_t dal = ptx::tc_smem_desc(a_lo + k * kNodes * kTcK, kTcLbo, kTcSbo);
+          const uint64_t dbh = ptx::tc_smem_desc(b_hi + k * kNodes * kTcK, kTcLbo, kTcSbo);
+          const uint64_t dbl = ptx::tc_smem_desc(b_lo + k * kNodes * kTcK, kTcLbo, kTcSbo);
+          ptx::tc_mma_tf32(tbase, dah, dbh, idesc, c > 0 || k > 0);
+          ptx::tc_mma_tf32(tbase + 128, dah, dbl, idesc, g > 0 || k > 0);
+          ptx::tc_mma_tf32(tbase + 128, dal, dbh, idesc, 1u);
+        }
+        ptx::tc_commit(&bars[st]);
+        if (c == kSuper / kChunk - 1) ptx::tc_commit(&bars[2]);
+      }
+    }
+    // ---- the 64 sources' sums into registers (the next MMA overwrites them after the
+    // barrier that follows these loads) ----
+    if (__all_sync(0xffffffffu, tc_wait(&bars[2], (sc - sc0) & 1u, abort_flag, err))) {
+      ptx::tc_fence_after();
+      flush(0);
+      ptx::tc_fence_before();
+    }
+  }
+  if (sc1 > sc0 && !*abort_flag) {
+    __syncwarp();
+    ptx::tc_fence_after();
+    flush(128);
+  }
+  const int node = 32 * (warp & 3) + lane;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    const int T = tg * kGroupT + 32 * (warp >> 2) + j;
+    if (T < P.nTs)
+      P.moments[((size_t)ks * P.nTs * P.nS + (size_t)T * P.nS + S) * kNodes + node] =
+          make_float2(acc_re[j], acc_im[j]);
+  }
+  // every commit has arrived before the block ends
+  if (tid == 0)
+    for (int b = 0; b < 2; ++b)
+      if (g > b) ptx::mbar_wait_bounded(&bars[b], ((g - 1 - b) >> 1) & 1u, kWaitCycles);
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  if (warp == 0) ptx::tmem_dealloc(tbase, 256);
+}
+
+// ---- translate -----------------------------------------------------------------------------
+// One block per cluster pair, one thread per node: moments to nodal weights, the px py x px py
+// products with G formed on the fly (one reciprocal, sine and cosine per node pair: bound by
+// the MUFU and FP32 pipes together), then back to Chebyshev coefficients, written as the TF32
+// operand that the target kernel stages.
+template <bool BATCHED>
+__global__ void __launch_bounds__(kNodes) k_expand_translate(
+    const ExpandProblem P0, const ExpandProblem *__restrict__ probs, const int *__restrict__ offs,
+    int n_probs) {
+  __shared__ float2 va[kNodes], vb[kNodes];
+  __shared__ float tab[2][kMaxP * kMaxP + kMaxP];
+  __shared__ float4 node_a[kNodes], node_b[kNodes];
+  int item;
+  const ExpandProblem &P = find_problem<BATCHED>(P0, probs, offs, n_probs, &item);
+  const int Tl = item / P.nS, S = item % P.nS, n = threadIdx.x;
+  const int px = P.px, py = P.py, np = px * py;
+  const size_t pairs = (size_t)P.nTs * P.nS;
+  for (int i = n; i < 2 * (kMaxP * kMaxP + kMaxP); i += kNodes)
+    tab[i / (kMaxP * kMaxP + kMaxP)][i % (kMaxP * kMaxP + kMaxP)] = P.cheb[i];
+  float2 mu = make_float2(0.f, 0.f);
+  for (int k = 0; k < P.ksplit; ++k) {
+    const float2 v = P.moments[(k * pairs + item) * kNodes + n];
+    mu.x += v.x;
+    mu.y += v.y;
+  }
+  va[n] = mu;
+  const float4 *f = reinterpret_cast<const float4 *>(P.frames + 12 * (size_t)item);
+  const float4 *fb = reinterpret_cast<const float4 *>(P.basis + 8 * (size_t)item);
+  const float4 f0 = f[0], f2 = f[2], f3 = fb[0], f4 = fb[1];
+  const float kap = P.kap, r0 = f0.w;
+  const int a = n / py, b = n % py;  // Chebyshev order or node along each axis
+  const float *mx = tab[0], *my = tab[1];
+  __syncthreads();
+  // nodal weights: M^T mu M, one axis at a time
+  if (n < np) {
+    float2 s = make_float2(0.f, 0.f);
+    for (int j = 0; j < py; ++j) {
+      const float m = my[j * kMaxP + b];
+      const float2 v = va[a * py + j];
+      s.x = fmaf(m, v.x, s.x);
+      s.y = fmaf(m, v.y, s.y);
+    }
+    vb[n] = s;
+  }
+  __syncthreads();
+  // node n of both clusters: offsets in the pair's frame
+  float tx = 0.f, ty = 0.f, tz = 0.f, ct = 0.f, rt = 0.f;
+  if (n < np) {
+    float2 s = make_float2(0.f, 0.f);
+    for (int i = 0; i < px; ++i) {
+      const float m = mx[i * kMaxP + a];
+      const float2 v = vb[i * py + b];
+      s.x = fmaf(m, v.x, s.x);
+      s.y = fmaf(m, v.y, s.y);
+    }
+    const float x = mx[kMaxP * kMaxP + a], y = my[kMaxP * kMaxP + b];
+    const float ex[3] = {f2.x, f2.y, f2.z}, e1[3] = {f3.x, f3.y, f3.z}, e2[3] = {f4.x, f4.y, f4.z};
+    const float4 ht = reinterpret_cast<const float4 *>(P.half_t)[P.t0 + Tl];
+    const float4 hs = reinterpret_cast<const float4 *>(P.half_s)[S];
+    float iq, h;
+    const float ux = x * ht.x, uy = y * ht.y;
+    const float e1x = pick(e1, P.ax), e1y = pick(e1, P.ay), e2x = pick(e2, P.ax);
+    const float e2y = pick(e2, P.ay), exx = pick(ex, P.ax), exy = pick(ex, P.ay);
+    tx = fmaf(e1x, ux, e1y * uy);
+    ty = fmaf(e2x, ux, e2y * uy);
+    tz = fmaf(exx, ux, exy * uy);
+    ct = fmaf(tx, tx, ty * ty);
+    rt = curvature(kap, ct, r0 + tz, iq, h);
+    const float wx = x * hs.x, wy = y * hs.y;
+    const float sx = fmaf(e1x, wx, e1y * wy), sy = fmaf(e2x, wx, e2y * wy);
+    const float sz = fmaf(exx, wx, exy * wy), cs = fmaf(sx, sx, sy * sy);
+    node_a[n] = make_float4(-2.f * sx, -2.f * sy, sz, cs);
+    node_b[n] = make_float4(s.x, s.y, curvature(kap, cs, r0 - sz, iq, h), 0.f);
+  }
+  __syncthreads();
+  // V_n = sum_j e^{i s k psi} / r W_j
+  float vre = 0.f, vim = 0.f;
+  const float qt = r0 + tz;
+#pragma unroll 4
+  for (int j = 0; j < np; ++j) {
+    const float4 s = node_a[j], w = node_b[j];
+    float iq, h;
+    const float c = fmaf(tx, s.x, fmaf(ty, s.y, ct + s.w));
+    const float psi = curvature(kap, c, qt - s.z, iq, h) - rt - w.z;
+    const float ir = iq * fmaf(-0.5f * h, iq, 1.f);  // 1 / r to c / q^2
+    const float cr = ir * ptx::cos_approx(psi), ci = ir * ptx::sin_approx(psi);
+    vre = fmaf(cr, w.x, fmaf(-ci, w.y, vre));
+    vim = fmaf(cr, w.y, fmaf(ci, w.x, vim));
+  }
+  va[n] = make_float2(vre, vim);
+  __syncthreads();
+  // Chebyshev coefficients of the nodal values: M V M^T
+  if (n < np) {
+    float2 s = make_float2(0.f, 0.f);
+    for (int i = 0; i < px; ++i) {
+      const float m = mx[a * kMaxP + i];
+      const float2 v = va[i * py + b];
+      s.x = fmaf(m, v.x, s.x);
+      s.y = fmaf(m, v.y, s.y);
+    }
+    vb[n] = s;
+  }
+  __syncthreads();
+  float2 nu = make_float2(0.f, 0.f);
+  if (n < np)
+    for (int j = 0; j < py; ++j) {
+      const float m = my[b * kMaxP + j];
+      const float2 v = vb[a * py + j];
+      nu.x = fmaf(m, v.x, nu.x);
+      nu.y = fmaf(m, v.y, nu.y);
+    }
+  // operand rows S % 32 (re) and 32 + S % 32 (im), depth n: halves of 64 nodes, hi then lo
+  const int nSG = (P.nS + kGroupS - 1) / kGroupS;
+  float *o = P.coeffs + (((size_t)Tl * nSG + S / kGroupS) * 2 + (n >> 6)) * kHalfFloats +
+             (size_t)((n & 63) >> 3) * (2 * kGroupS * kTcK);
+  const int re = tc_off(S % kGroupS, n & 7), im = tc_off(kGroupS + S % kGroupS, n & 7);
+  const float rh = ptx::to_tf32_int(nu.x), ih = ptx::to_tf32_int(nu.y);
+  o[re] = rh;
+  o[im] = ih;
+  o[kHalfFloats / 2 + re] = ptx::to_tf32_int(__fsub_rn(nu.x, rh));
+  o[kHalfFloats / 2 + im] = ptx::to_tf32_int(__fsub_rn(nu.y, ih));
+}
+
+// ---- targets -------------------------------------------------------------------------------
+// One block: 128 targets of one cluster against a share of the source clusters, 32 at a time:
+// D[target][column] = sum over 128 nodes of weight x coefficient for 32 + 32 columns.  The
+// weights of the targets stay in shared memory for the whole block (128 KB, both TF32 parts);
+// a load warp brings the coefficients by bulk copies, in halves of 64 nodes, and the
+// frames of 32 pairs; 16 consumer warps read D (two TMEM buffers), each thread its target and
+// 8 clusters, rotate by e^{i s k alpha} and sum.
+struct TargetsSmem {
+  static constexpr size_t a = 0;                                    // float [hi, lo][128*128]
+  static constexpr size_t b = a + 2 * kBlockT * kNodes * 4;         // float [2][kHalfFloats]
+  static constexpr size_t cheb = b + 2 * kHalfFloats * 4;           // float [2][16][128]
+  static constexpr size_t frames = cheb + 2 * kMaxP * kBlockT * 4;  // float [2][32][12]
+  static constexpr size_t bars = frames + 2 * kGroupS * 12 * 4;     // uint64 [12]
+  static constexpr size_t misc = bars + 12 * 8;                     // uint32 taddr, abort
+  static constexpr size_t bytes = misc + 16;
+};
+static_assert(TargetsSmem::bytes <= 227 * 1024, "target kernel: shared memory");
+constexpr int kTgtConsumers = 16;                        // then the MMA warp and the load warp
+constexpr int kTgtThreads = 32 * (kTgtConsumers + 2);
+
+template <bool BATCHED>
+__global__ void __launch_bounds__(kTgtThreads, 1)
+    k_expand_targets(const ExpandProblem P0, const ExpandProblem *__restrict__ probs,
+                     const int *__restrict__ offs, int n_probs, int *err) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  using L = TargetsSmem;
+  float *a_hi = reinterpret_cast<float *>(smem + L::a), *a_lo = a_hi + kBlockT * kNodes;
+  float *sb = reinterpret_cast<float *>(smem + L::b);
+  float *cheb = reinterpret_cast<float *>(smem + L::cheb);
+  float *sframes = reinterpret_cast<float *>(smem + L::frames);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::bars);
+  uint64_t *bfull = bars, *bfree = bars + 2, *dfull = bars + 4, *dfree = bars + 6,
+           *ffull = bars + 8, *ffree = bars + 10;
+  uint32_t *taddr_slot = reinterpret_cast<uint32_t *>(smem + L::misc);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L::misc + 4);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool consumer = warp < kTgtConsumers, mma_warp = warp == kTgtConsumers;
+
+  int item;
+  const ExpandProblem &P = find_problem<BATCHED>(P0, probs, offs, n_probs, &item);
+  const int blk = item / P.ssplit, sp = item % P.ssplit;
+  const int m0 = P.t0 * P.nt + blk * kBlockT, Tl = blk * kBlockT / P.nt;
+  const int nSG = (P.nS + kGroupS - 1) / kGroupS;
+  const int g0 = (int)((long long)nSG * sp / P.ssplit), g1 = (int)((long long)nSG * (sp + 1) / P.ssplit);
+  const int px = P.px, py = P.py, np = px * py;
+
+  // half i: nodes 64 .. 127 (i even) or 0 .. 63 (i odd) of cluster group g0 + i / 2
+  const int nh = 2 * (g1 - g0);
+  auto load = [&](int i) {
+    const int st = i & 1, g = g0 + (i >> 1);
+    ptx::mbar_arrive_expect_tx(&bfull[st], kHalfFloats * 4);
+    ptx::bulk_g2s(sb + st * kHalfFloats,
+                  P.coeffs + (((size_t)Tl * nSG + g) * 2 + (1 - st)) * kHalfFloats, kHalfFloats * 4,
+                  &bfull[st]);
+    if (st == 0) {
+      const int d = (i >> 1) & 1, bytes = 48 * min(kGroupS, P.nS - g * kGroupS);
+      ptx::mbar_arrive_expect_tx(&ffull[d], bytes);
+      ptx::bulk_g2s(sframes + d * kGroupS * 12,
+                    P.frames + 12 * ((size_t)Tl * P.nS + g * kGroupS), bytes, &ffull[d]);
+    }
+  };
+  if (tid == 32 * (kTgtConsumers + 1)) {
+    for (int b = 0; b < 2; ++b) {
+      ptx::mbar_init(&bfull[b], 1);
+      ptx::mbar_init(&bfree[b], 1);
+      ptx::mbar_init(&dfull[b], 1);
+      ptx::mbar_init(&dfree[b], kTgtConsumers);
+      ptx::mbar_init(&ffull[b], 1);
+      ptx::mbar_init(&ffree[b], kTgtConsumers);
+    }
+    *abort_flag = 0;
+    ptx::fence_barrier_init();
+    for (int i = 0; i < min(nh, 2); ++i) load(i);
+  }
+  if (mma_warp) ptx::tmem_alloc(taddr_slot, 128);
+
+  // ---- weights of the block's targets ----
+  float th[3] = {0.f, 0.f, 0.f}, tl[3] = {0.f, 0.f, 0.f};  // consumers: target 32 (warp % 4) + lane
+  {
+    const int t = m0 + (tid & (kBlockT - 1));
+    if (consumer && t < P.M) cluster_offset(P.geo_t, P.shift_t, t, P.tt_log2, th, tl);
+    const float4 half = reinterpret_cast<const float4 *>(P.half_t)[P.t0 + Tl];
+    if (tid < kBlockT)
+      cheb_row(pick(th, P.ax) * half.z, px, cheb + tid, kBlockT);
+    else if (tid < 2 * kBlockT)
+      cheb_row(pick(th, P.ay) * half.w, py, cheb + kMaxP * kBlockT + tid - kBlockT, kBlockT);
+  }
+  __syncthreads();
+  if (consumer) {
+    const int row = tid & (kBlockT - 1), n0 = 32 * (tid >> 7);
+    int a = n0 / py, b = n0 % py;
+    for (int q = 0; q < 8; ++q) {
+      float hi[4], lo[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float w = n0 + 4 * q + j < np
+                            ? cheb[a * kBlockT + row] * cheb[(kMaxP + b) * kBlockT + row] : 0.f;
+        if (++b == py) {
+          b = 0;
+          ++a;
+        }
+        hi[j] = ptx::to_tf32_int(w);
+        lo[j] = ptx::to_tf32_int(__fsub_rn(w, hi[j]));
+      }
+      const int n = n0 + 4 * q, o = (n >> 3) * (kBlockT * kTcK) + tc_off(row, n & 7);
+      *reinterpret_cast<float4 *>(a_hi + o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<float4 *>(a_lo + o) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+    }
+  }
+  ptx::fence_proxy_async_smem();
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tbase = *taddr_slot;
+  constexpr uint32_t idesc = ptx::tc_idesc_tf32(kBlockT, 2 * kGroupS);
+
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);  // (re hi, re lo, im hi, im lo)
+  if (mma_warp) {
+    if (lane == 0) {
+      int issued = 0;
+      for (int i = 0; i < nh; ++i) {
+        const int st = i & 1, gi = i >> 1, d = gi & 1;
+        if (!tc_wait(&bfull[st], gi & 1u, abort_flag, err)) break;
+        if (st == 0 && gi >= 2 && !tc_wait(&dfree[d], ((gi >> 1) - 1) & 1u, abort_flag, err)) break;
+        ptx::tc_fence_after();
+        const float *bh = sb + st * kHalfFloats, *bl = bh + kHalfFloats / 2;
+        const uint32_t dt = tbase + (uint32_t)(2 * kGroupS * d);
+        const int k0 = 8 * (1 - st);
+        for (int k = 7; k >= 0; --k) {  // the cross products of the TF32 parts
+          const uint64_t ah = ptx::tc_smem_desc(a_hi + (k0 + k) * kBlockT * kTcK, kTcLbo, kTcSbo);
+          const uint64_t al = ptx::tc_smem_desc(a_lo + (k0 + k) * kBlockT * kTcK, kTcLbo, kTcSbo);
+          ptx::tc_mma_tf32(dt, ah, ptx::tc_smem_desc(bl + k * 2 * kGroupS * kTcK, kTcLbo, kTcSbo),
+                           idesc, st > 0 || k < 7);
+          ptx::tc_mma_tf32(dt, al, ptx::tc_smem_desc(bh + k * 2 * kGroupS * kTcK, kTcLbo, kTcSbo),
+                           idesc, 1u);
+        }
+        for (int k = 7; k >= 0; --k)
+          ptx::tc_mma_tf32(dt, ptx::tc_smem_desc(a_hi + (k0 + k) * kBlockT * kTcK, kTcLbo, kTcSbo),
+                           ptx::tc_smem_desc(bh + k * 2 * kGroupS * kTcK, kTcLbo, kTcSbo), idesc, 1u);
+        ptx::tc_commit(&bfree[st]);
+        if (st) ptx::tc_commit(&dfull[d]);
+        ++issued;
+      }
+      // the MMAs in flight end before the block does
+      for (int i = max(0, issued - 2); i < issued; ++i)
+        ptx::mbar_wait_bounded(&bfree[i & 1], (i >> 1) & 1u, kWaitCycles);
+    }
+    __syncwarp();
+  } else if (!consumer) {
+    if (lane == 0) {
+      int loaded = min(nh, 2);
+      for (int i = 2; i < nh; ++i, ++loaded) {  // half i goes where half i - 2 was
+        if (!tc_wait(&bfree[i & 1], ((i >> 1) - 1) & 1u, abort_flag, err)) break;
+        if (!(i & 1) && i >= 4 && !tc_wait(&ffree[(i >> 1) & 1], ((i >> 2) - 1) & 1u, abort_flag, err))
+          break;
+        load(i);
+      }
+      // and so do the copies
+      for (int i = max(0, loaded - 2); i < loaded; ++i)
+        ptx::mbar_wait_bounded(&bfull[i & 1], (i >> 1) & 1u, kWaitCycles);
+      for (int g = max(0, (loaded + 1) / 2 - 2); g < (loaded + 1) / 2; ++g)
+        ptx::mbar_wait_bounded(&ffull[g & 1], (g >> 1) & 1u, kWaitCycles);
+    }
+    __syncwarp();
+  } else {
+    const int cg = warp >> 2;
+    const float kap = P.kap;
+    const float t2 = fmaf(th[0], th[0], fmaf(th[1], th[1], th[2] * th[2]));
+    const uint32_t trow = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(8 * cg);
+    for (int g = g0; g < g1; ++g) {
+      const int gi = g - g0, d = gi & 1, left = min(8, P.nS - g * kGroupS - 8 * cg);
+      if (!__all_sync(0xffffffffu, tc_wait(&dfull[d], (gi >> 1) & 1u, abort_flag, err) &&
+                                       tc_wait(&ffull[d], (gi >> 1) & 1u, abort_flag, err)))
+        break;
+      ptx::tc_fence_after();
+      uint32_t vr[8], vi[8];
+      ptx::tmem_ld8_nowait(trow + (uint32_t)(2 * kGroupS * d), vr);
+      ptx::tmem_ld8_nowait(trow + (uint32_t)(2 * kGroupS * d + kGroupS), vi);
+      ptx::tmem_wait8(vr);
+      ptx::tmem_wait8(vi);
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&dfree[d]);
+      const float4 *f = reinterpret_cast<const float4 *>(sframes + (d * kGroupS + 8 * cg) * 12);
+      float gr = 0.f, gim = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (j < left) {
+          const float4 f0 = f[3 * j], f1 = f[3 * j + 1], f2 = f[3 * j + 2];
+          const float ah[3] = {f0.x, f0.y, f0.z}, al[3] = {f1.x, f1.y, f1.z};
+          float s, e, s2, e2, iq, hq;
+          dot3_ff(ah, al, th, tl, s, e);
+          two_sum(s, f1.w, s2, e2);
+          const float tz = fmaf(f2.x, th[0], fmaf(f2.y, th[1], f2.z * th[2]));
+          const float ph = reduce_two_pi_ff(s2, __fadd_rn(__fadd_rn(e, e2), f2.w)) +
+                           curvature(kap, fmaf(-tz, tz, t2), f0.w + tz, iq, hq);
+          const float cr = ptx::cos_approx(ph), sr = ptx::sin_approx(ph);
+          const float re = __uint_as_float(vr[j]), im = __uint_as_float(vi[j]);
+          gr = fmaf(re, cr, fmaf(-im, sr, gr));
+          gim = fmaf(re, sr, fmaf(im, cr, gim));
+        }
+      }
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&ffree[d]);
+      float h, e;
+      two_sum(sum.x, gr, h, e);
+      sum.x = h;
+      sum.y = __fadd_rn(sum.y, e);
+      two_sum(sum.z, gim, h, e);
+      sum.z = h;
+      sum.w = __fadd_rn(sum.w, e);
+    }
+  }
+  // ---- the four warps of a target add their clusters' sums ----
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  if (mma_warp) ptx::tmem_dealloc(tbase, 128);
+  float4 *part = reinterpret_cast<float4 *>(cheb);  // [4][128], the Chebyshev factors are done
+  if (consumer) part[(warp >> 2) * kBlockT + 32 * (warp & 3) + lane] = sum;
+  __syncthreads();
+  if (tid < kBlockT && m0 + tid < P.M) {
+    double re = 0.0, im = 0.0;
+    for (int c = 0; c < 4; ++c) {
+      const float4 v = part[c * kBlockT + tid];
+      re += (double)v.x + (double)v.y;
+      im += (double)v.z + (double)v.w;
+    }
+    const int t = m0 + tid;
+    if (P.ssplit == 1)
+      P.y[P.order_t[t]] = make_double2(re, im);
+    else
+      P.partial[(size_t)sp * P.M + t] = make_double2(re, im);
+  }
+}
+
+}  // namespace
+
+int expand_setup_blocks(const ExpandProblem &p) {
+  const long long n = (long long)p.nTs * p.nS + (p.N + p.cs - 1) / p.cs + (p.M + p.tt - 1) / p.tt +
+                      p.nS + p.nT + 2 * kMaxP * kMaxP;
+  return (int)((n + 127) / 128);
+}
+int expand_moments_blocks(const ExpandProblem &p) {
+  return p.nS * ((p.nTs + kGroupT - 1) / kGroupT) * p.ksplit;
+}
+int expand_translate_blocks(const ExpandProblem &p) { return p.nS * p.nTs; }
+int expand_targets_blocks(const ExpandProblem &p) {
+  const long long m0 = (long long)p.t0 * p.nt, m1 = (long long)(p.t0 + p.nTs) * p.nt;
+  const long long m = (m1 < p.M ? m1 : p.M) - m0;
+  return (int)((m + kBlockT - 1) / kBlockT) * p.ssplit;
+}
+
+int launch_expand(const ExpandProblem &p, int *err, cudaStream_t s) {
+  HOLO_TRY((kernel_setup<k_expand_moments<false>>(kMomThreads, (int)MomentsSmem::bytes, nullptr)));
+  HOLO_TRY((kernel_setup<k_expand_targets<false>>(kTgtThreads, (int)TargetsSmem::bytes, nullptr)));
+  k_expand_setup<false><<<expand_setup_blocks(p), 128, 0, s>>>(p, nullptr, nullptr, 1);
+  k_expand_moments<false><<<expand_moments_blocks(p), kMomThreads, MomentsSmem::bytes, s>>>(
+      p, nullptr, nullptr, 1, err);
+  k_expand_translate<false><<<expand_translate_blocks(p), kNodes, 0, s>>>(p, nullptr, nullptr, 1);
+  k_expand_targets<false><<<expand_targets_blocks(p), kTgtThreads, TargetsSmem::bytes, s>>>(
+      p, nullptr, nullptr, 1, err);
+  note_launches(4);
+  HOLO_CUDA(cudaGetLastError());
+  return HOLO_OK;
+}
+
+}  // namespace holo

@@ -47,11 +47,10 @@ namespace holo {
 namespace {
 
 #include "split_frame.cuh"
+#include "tc_operand.cuh"
 
 constexpr int kTcTT = 512;                    // targets per CTA (4 blocks of 128)
-constexpr int kTcM = 128, kTcK = 8;
 constexpr int kTcCols = 512;                  // TMEM columns allocated: two accumulator buffers
-constexpr uint32_t kTcLbo = 128, kTcSbo = 256;  // operand layout (bytes), see tc_off
 
 // Shape of one build: CG column groups of consumer warps per TMEM lane group (4 lane
 // groups of 32 targets), NB sources per MMA block (TMEM columns per buffer), CS = NBLK NB
@@ -67,14 +66,6 @@ struct TcShape {
   static constexpr int Cols = NB / CG;            // columns per consumer warp per block
   static constexpr int Chunks = Cols / 16;        // 16-column loads per block
 };
-
-// Float offset of element (row r, feature k) of a K-major tf32 operand with K = 8:
-// core matrices of 8 rows x 4 features (16 B rows, 128 B), the two along K 128 B
-// apart (LBO), 8-row groups 256 B apart (SBO).  Rows of one 128- or 256-row block
-// are contiguous, so block b starts at row 128 b / 256 b.
-__host__ __device__ __forceinline__ int tc_off(int r, int k) {
-  return (r >> 3) * 64 + (k >> 2) * 32 + (r & 7) * 4 + (k & 3);
-}
 
 template <int CG, int NBLK>
 struct TcSmem {
@@ -133,19 +124,6 @@ __device__ __forceinline__ void store_row_split(float *hi, float *lo, int r, con
   *reinterpret_cast<float4 *>(hi + tc_off(r, 4)) = make_float4(h[4], h[5], h[6], h[7]);
   *reinterpret_cast<float4 *>(lo + tc_off(r, 0)) = make_float4(l[0], l[1], l[2], l[3]);
   *reinterpret_cast<float4 *>(lo + tc_off(r, 4)) = make_float4(l[4], l[5], l[6], l[7]);
-}
-
-// Bounded wait that gives up at once when the CTA has aborted; sleep_ns > 0: poll with
-// that much sleep in between.
-__device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
-                                        int *err, unsigned sleep_ns = 0) {
-  if (*abort_flag) return false;
-  if (sleep_ns ? ptx::mbar_wait_bounded_sleep(bar, parity, kWaitCycles, sleep_ns)
-               : ptx::mbar_wait_bounded(bar, parity, kWaitCycles))
-    return true;
-  *abort_flag = 1;
-  atomicExch(err, kDevErrTimeout);
-  return false;
 }
 
 // Build flags: kTcScalar -- the MUFU pairs accumulated in scalar FP32 (no packing);
