@@ -325,10 +325,27 @@ static int tile_error_bound(holo_plan_s *p, int cs, int tt, double *bound, doubl
   return HOLO_OK;
 }
 
+// Tiles, splits and grid of the plan's kernel variant.
+static int plan_grid(holo_plan_s *p) {
+  const bool split = p->precision == HOLO_SPLIT32;
+  const Variant V = split ? split_variant(p->variant) : fp64_variant(p->variant);
+  p->n_stiles = (p->N + V.cs - 1) / V.cs;
+  if (!split) p->n_pad = std::max(p->n_stiles, 1) * V.cs;
+  p->n_ttiles = (p->M + V.tt() - 1) / V.tt();
+  int occ = 0;
+  HOLO_TRY(split ? split_occupancy(p->variant, false, &occ) : fp64_occupancy(p->variant, &occ));
+  const int G = std::max(1, occ) * p->h->sm_count;
+  const size_t scratch_cap = (size_t)1 << 30;  // partial sums at most 1 GiB
+  const int max_splits = (int)std::max<size_t>(1, scratch_cap / (std::max<size_t>(p->M, 1) * 16));
+  p->splits = choose_splits(p->n_ttiles, p->n_stiles, G, p->M, max_splits);
+  p->grid = std::max(1, std::min(G, p->n_ttiles * p->splits));
+  return HOLO_OK;
+}
+
 int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, size_t M,
                      int precision, int forced_variant, cudaStream_t s, holo_plan_s **out,
                      const int32_t *known_order_s, const int32_t *known_order_t,
-                     int known_tiling_s, int known_tiling_t) {
+                     int known_tiling_s, int known_tiling_t, double k_once) {
   if (precision != HOLO_FP64 && precision != HOLO_SPLIT32)
     return fail(HOLO_ERR_INVALID, "unknown precision %d", precision);
   HOLO_TRY(check_sizes(N, M));
@@ -413,7 +430,13 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
     size_t ci = 0;
     HOLO_TRY(order_both(kTileHilbert, known_order_s, known_order_t));
     HOLO_TRY(choose(&ci));
-    if (ci > 0 && forced_variant < 0) {
+    bool expands = false;
+    if (ci > 0 && forced_variant < 0 && k_once > 0.0) {
+      p->variant = variant;
+      HOLO_TRY(plan_grid(pp));
+      expands = plan_expansion(pp, k_once).use;
+    }
+    if (ci > 0 && forced_variant < 0 && !expands) {
       size_t cp = 0;
       HOLO_TRY(order_both(kTilePacked, nullptr, nullptr));
       HOLO_TRY(choose(&cp));
@@ -425,21 +448,8 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
   }
   const Variant V = precision == HOLO_SPLIT32 ? split_variant(variant) : fp64_variant(variant);
   p->variant = variant;
-  p->n_stiles = (int)((N + V.cs - 1) / V.cs);
-  if (precision != HOLO_SPLIT32) p->n_pad = std::max(p->n_stiles, 1) * V.cs;
-  p->n_ttiles = (int)((M + V.tt() - 1) / V.tt());
-
-  int occ = 0;
-  if (precision == HOLO_SPLIT32) {
-    HOLO_TRY(split_occupancy(variant, false, &occ));
-  } else {
-    HOLO_TRY(fp64_occupancy(variant, &occ));
-  }
-  const int G = std::max(1, occ) * h->sm_count;
-  const size_t scratch_cap = (size_t)1 << 30;  // partial sums at most 1 GiB
-  const int max_splits = (int)std::max<size_t>(1, scratch_cap / (std::max<size_t>(M, 1) * 16));
-  p->splits = choose_splits(p->n_ttiles, p->n_stiles, G, M, max_splits);
-  p->grid = std::max(1, std::min(G, p->n_ttiles * p->splits));
+  p->expand_k = 0.0;  // chosen for another tiling, if at all
+  HOLO_TRY(plan_grid(p.get()));
 
   if (precision == HOLO_SPLIT32) {
     // float-float offsets of every point from its tile's centre (tiles of the
@@ -456,6 +466,10 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
     if (M) HOLO_CUDA(cudaMemcpyAsync(p->pos_t, v, 3 * M * sizeof(double), cudaMemcpyDeviceToDevice, s));
   }
   // keep original-order positions for the adjoint's transposed plan
+  if (k_once > 0.0) {
+    *out = p.release();
+    return HOLO_OK;
+  }
   double *u_keep = nullptr, *v_keep = nullptr;
   HOLO_TRY(alloc_plan(p.get(), (void **)&u_keep, 3 * std::max<size_t>(N, 1) * sizeof(double), s));
   HOLO_TRY(alloc_plan(p.get(), (void **)&v_keep, 3 * std::max<size_t>(M, 1) * sizeof(double), s));
@@ -470,7 +484,7 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
 // Whether, and on which clusters, a transform of this plan at wave number k runs by cluster
 // expansions: where they take less time than the plan's pair kernel (~20 pairs per clock
 // and SM on the tensor-core builds, ~16 on the CUDA cores, over the waves of its work items).
-ExpandChoice plan_expansion(holo_plan_s *p, double k) {
+ExpandChoice plan_expansion(holo_plan_s *p, double k, double launches) {
   if (p->precision != HOLO_SPLIT32 || p->pair_kernel_only || p->N == 0 || p->M == 0) return {};
   const Variant V = split_variant(p->variant);
   if (box_level(V.cs) < 0) return {};  // its tiles do not nest in the clusters
@@ -480,7 +494,7 @@ ExpandChoice plan_expansion(holo_plan_s *p, double k) {
     const double clocks = waves * per_item * V.cs * V.tt() / (V.tc ? 20.0 : 16.0) *
                           std::max(1.0, (double)p->grid / p->h->sm_count);
     p->expand = expand_choose(p->stats_s, p->stats_t, p->N, p->M, box_level(V.cs), box_level(V.tt()),
-                              k, kPairOverhead + clocks / 1.9e9, p->h->sm_count);
+                              k, clocks / 1.9e9, launches, p->h->sm_count);
     p->expand_k = k;
   }
   return p->expand;
@@ -896,7 +910,8 @@ static int one_shot(holo_handle h, int sign, double lambda, const double *amp,
       return fail(HOLO_ERR_INVALID, "targets_per_block %d: use 256, 512, 1024 or 2048", block);
   }
   holo_plan_s *p = nullptr;
-  HOLO_TRY(plan_create_impl(h, du, N, dv, M, precision, forced_variant, s, &p));
+  HOLO_TRY(plan_create_impl(h, du, N, dv, M, precision, forced_variant, s, &p, nullptr, nullptr,
+                            kTileHilbert, kTileHilbert, (2.0 * M_PI) / lambda));
   const int rc = mc ? plan_execute_mc_impl(p, sign, lambda, da, dp, (double2 *)dy, seed, sub, block, s)
                     : plan_execute_impl(p, sign, lambda, da, dp, (double2 *)dy, 0, s);
   plan_release(p, s);
@@ -1056,7 +1071,9 @@ static int project_dev(holo_handle h, double lambda, const double *xa, const dou
   double *partials = tmp.get<double>(1024);
   if (!y || !mx || !partials) return fail(HOLO_ERR_ALLOC, "project scratch");
   holo_plan_s *p1 = nullptr;
-  HOLO_TRY(plan_create_impl(h, u, N, v, M, precision, -1, s, &p1));
+  const double k = (2.0 * M_PI) / lambda;
+  HOLO_TRY(plan_create_impl(h, u, N, v, M, precision, -1, s, &p1, nullptr, nullptr, kTileHilbert,
+                            kTileHilbert, k));
   // p1 lives until the reference-wave and z plans have taken its tile order of v
   std::unique_ptr<holo_plan_s, void (*)(holo_plan_s *)> keep(p1, [](holo_plan_s *q) {
     plan_release(q, q->last_stream);
@@ -1082,7 +1099,7 @@ static int project_dev(holo_handle h, double lambda, const double *xa, const dou
     HOLO_CUDA(cudaMemcpyAsync(src, host_src, sizeof(host_src), cudaMemcpyHostToDevice, s));
     holo_plan_s *pr = nullptr;
     HOLO_TRY(plan_create_impl(h, src, 1, v, M, precision, -1, s, &pr, nullptr, order_v,
-                              holo::kTileHilbert, tiling_v));
+                              holo::kTileHilbert, tiling_v, k));
     rc = plan_execute_impl(pr, HOLO_FORWARDS, lambda, src + 3, src + 4, yref, 0, s);
     plan_release(pr, s);
     HOLO_TRY(rc);
@@ -1095,7 +1112,8 @@ static int project_dev(holo_handle h, double lambda, const double *xa, const dou
   double2 *z = tmp.get<double2>(P);
   if (!z) return fail(HOLO_ERR_ALLOC, "project scratch");
   holo_plan_s *p2 = nullptr;
-  HOLO_TRY(plan_create_impl(h, v, M, w, P, precision, -1, s, &p2, order_v, nullptr, tiling_v));
+  HOLO_TRY(plan_create_impl(h, v, M, w, P, precision, -1, s, &p2, order_v, nullptr, tiling_v,
+                            kTileHilbert, k));
   rc = plan_execute_impl(p2, HOLO_FORWARDS, lambda, ya, yp, z, 0, s);
   plan_release(p2, s);
   HOLO_TRY(rc);

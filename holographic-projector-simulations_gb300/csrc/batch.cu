@@ -6,12 +6,14 @@
 // the same kernel variant form a group, whose (target tile, source range) work
 // items go into one device work queue sorted longest-first, drained by one
 // persistent split-precision kernel with an atomic counter (no CTA waits on
-// another).  Gathers, the queue reset, one queue kernel per group and the
-// cross-split reductions are captured once into a CUDA graph;
-// holo_batch_execute replays it.
+// another).  Problems that run by cluster expansions share one launch of each of
+// their four kernels, whose blocks find their problem by its first block.  Gathers
+// (one launch), the queue reset, the queue and expansion kernels and the cross-split
+// reductions are captured once into a CUDA graph; holo_batch_execute replays it.
 #include <algorithm>
 #include <memory>
 
+#include "expand_plan.h"
 #include "internal.cuh"
 
 using namespace holo;
@@ -73,6 +75,40 @@ int describe_problem(holo_batch_s *b, const holo_problem &q, holo_plan_s *p, int
   return HOLO_OK;
 }
 
+// Scratch and descriptor of problem i, which fills `share` of the GPU, by cluster expansions;
+// P is what the reduction of its partial sums needs.
+int describe_expansion(holo_batch_s *b, const holo_problem &q, holo_plan_s *p, const ExpandChoice &ch,
+                       double share, ExpandProblem *E, SplitProblem *P, cudaStream_t s) {
+  const double sk = q.sign * ((2.0 * M_PI) / q.lambda);
+  ExpandScratch size, tmp;
+  expand_describe(p, ch, sk, (double2 *)q.y_re_im, share, size);
+  tmp.base = (unsigned char *)pool_alloc(b->h, size.bytes, s);
+  if (!tmp.base) return fail(HOLO_ERR_ALLOC, "batch expansion scratch of %zu bytes", size.bytes);
+  b->owned.push_back(tmp.base);
+  *E = expand_describe(p, ch, sk, (double2 *)q.y_re_im, share, tmp);
+  E->nTs = std::min(E->slab, E->nT);
+  *P = SplitProblem{};
+  P->apf_s = E->apf_s;
+  P->order_t = p->order_t;
+  P->partial = E->partial;
+  P->y = E->y;
+  P->N = p->N;
+  P->M = p->M;
+  P->splits = E->ssplit;
+  return HOLO_OK;
+}
+
+// A device copy of host data, kept by the batch.
+template <typename T>
+int keep_copy(holo_batch_s *b, const std::vector<T> &host, T **dev, cudaStream_t s) {
+  *dev = (T *)pool_alloc(b->h, sizeof(T) * std::max<size_t>(host.size(), 1), s);
+  if (!*dev) return fail(HOLO_ERR_ALLOC, "batch descriptors");
+  b->owned.push_back(*dev);
+  if (!host.empty())
+    HOLO_CUDA(cudaMemcpyAsync(*dev, host.data(), sizeof(T) * host.size(), cudaMemcpyHostToDevice, s));
+  return HOLO_OK;
+}
+
 int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, cudaStream_t s) {
   holo_handle h = b->h;
   // every problem planned on its own: tile shape and pair model as for a
@@ -80,16 +116,42 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
   // sequence of per-problem launches)
   for (int i = 0; i < n; ++i) {
     holo_plan_s *p = nullptr;
-    HOLO_TRY(plan_create_impl(h, pr[i].u_xyz, pr[i].N, pr[i].v_xyz, pr[i].M, precision, -1, s,
-                              &p));
+    HOLO_TRY(plan_create_impl(h, pr[i].u_xyz, pr[i].N, pr[i].v_xyz, pr[i].M, precision, -1, s, &p,
+                              nullptr, nullptr, kTileHilbert, kTileHilbert,
+                              (2.0 * M_PI) / pr[i].lambda));
     b->plans.push_back(p);
     b->total_pairs += (long long)pr[i].N * (long long)pr[i].M;
   }
   if (precision != HOLO_SPLIT32) return HOLO_OK;
 
-  std::vector<Group> groups;
-  std::vector<int> group_of(n);
+  std::vector<SplitProblem> probs(n);
+  std::vector<ExpandProblem> expands, slabbed;  // slabbed: more scratch than one launch takes
+  std::vector<ExpandChoice> choice(n);
+  double seconds = 1e-12;
   for (int i = 0; i < n; ++i) {
+    choice[i] = plan_expansion(b->plans[i], (2.0 * M_PI) / pr[i].lambda, 0.0);
+    if (choice[i].use) seconds += choice[i].seconds;
+  }
+  for (int i = 0; i < n; ++i) {
+    if (!choice[i].use) continue;
+    ExpandProblem E;
+    HOLO_TRY(describe_expansion(b, pr[i], b->plans[i], choice[i], choice[i].seconds / seconds, &E,
+                                &probs[i], s));
+    (E.nTs == E.nT ? expands : slabbed).push_back(E);
+  }
+  const int ne = (int)expands.size();
+  std::vector<int> offs(4 * (size_t)(ne + 1), 0);
+  int totals[4] = {0, 0, 0, 0};
+  for (int i = 0; i < ne; ++i) {
+    int blocks[4];
+    expand_blocks(expands[i], blocks);
+    for (int k = 0; k < 4; ++k) offs[(size_t)k * (ne + 1) + i + 1] = totals[k] += blocks[k];
+  }
+
+  std::vector<Group> groups;
+  std::vector<int> group_of(n, -1);
+  for (int i = 0; i < n; ++i) {
+    if (choice[i].use) continue;
     size_t g = 0;
     const int v = b->plans[i]->variant;
     while (g < groups.size() && groups[g].variant != v) ++g;
@@ -99,7 +161,6 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
     }
     group_of[i] = (int)g;
   }
-  std::vector<SplitProblem> probs(n);
   std::vector<int> offsets(n + 1, 0);
   for (int i = 0; i < n; ++i) offsets[i + 1] = offsets[i] + b->plans[i]->M;
   for (size_t g = 0; g < groups.size(); ++g) {
@@ -125,30 +186,32 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
     });
     G.grid = std::max(1, std::min(slots, (int)G.items.size()));
   }
-  const int ng = (int)groups.size();
-  SplitProblem *probs_dev = (SplitProblem *)pool_alloc(h, sizeof(SplitProblem) * std::max(n, 1), s);
-  int *queues = (int *)pool_alloc(h, sizeof(int) * std::max(ng, 1), s);
-  int *offsets_dev = (int *)pool_alloc(h, sizeof(int) * (n + 1), s);
-  if (!probs_dev || !queues || !offsets_dev) return fail(HOLO_ERR_ALLOC, "batch descriptors");
-  b->owned.push_back(probs_dev);
-  b->owned.push_back(queues);
-  b->owned.push_back(offsets_dev);
-  for (Group &G : groups) {
-    G.items_dev = (WorkItem *)pool_alloc(h, sizeof(WorkItem) * std::max<size_t>(G.items.size(), 1), s);
-    if (!G.items_dev) return fail(HOLO_ERR_ALLOC, "batch work items");
-    b->owned.push_back(G.items_dev);
-    if (!G.items.empty())
-      HOLO_CUDA(cudaMemcpyAsync(G.items_dev, G.items.data(), sizeof(WorkItem) * G.items.size(),
-                                cudaMemcpyHostToDevice, s));
+  std::vector<GatherApf> gathers(n);
+  int gather_blocks = 0;
+  for (int i = 0; i < n; ++i) {
+    const holo_plan_s *p = b->plans[i];
+    gathers[i] = {pr[i].amp, pr[i].phase, p->order_s, p->N, p->n_pad,
+                  const_cast<float2 *>(probs[i].apf_s), gather_blocks};
+    gather_blocks += (p->n_pad + 1023) / 1024;
   }
-  if (n > 0)
-    HOLO_CUDA(cudaMemcpyAsync(probs_dev, probs.data(), sizeof(SplitProblem) * n,
-                              cudaMemcpyHostToDevice, s));
-  HOLO_CUDA(cudaMemcpyAsync(offsets_dev, offsets.data(), sizeof(int) * (n + 1),
-                            cudaMemcpyHostToDevice, s));
+  const int ng = (int)groups.size();
+  SplitProblem *probs_dev = nullptr;
+  ExpandProblem *expands_dev = nullptr;
+  GatherApf *gathers_dev = nullptr;
+  int *offsets_dev = nullptr, *offs_dev = nullptr;
+  int *queues = (int *)pool_alloc(h, sizeof(int) * std::max(ng, 1), s);
+  if (!queues) return fail(HOLO_ERR_ALLOC, "batch descriptors");
+  b->owned.push_back(queues);
+  HOLO_TRY(keep_copy(b, probs, &probs_dev, s));
+  HOLO_TRY(keep_copy(b, expands, &expands_dev, s));
+  HOLO_TRY(keep_copy(b, gathers, &gathers_dev, s));
+  HOLO_TRY(keep_copy(b, offsets, &offsets_dev, s));
+  HOLO_TRY(keep_copy(b, offs, &offs_dev, s));
+  for (Group &G : groups) HOLO_TRY(keep_copy(b, G.items, &G.items_dev, s));
   HOLO_CUDA(cudaStreamSynchronize(s));  // host vectors above are about to go away
 
-  // ---- capture the graph: gathers, queue reset, one queue kernel per group, reductions ----
+  // ---- capture the graph: gathers, queue reset, one queue kernel per group, expansions,
+  // reductions ----
   cudaStream_t cap;
   HOLO_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
   int rc = HOLO_OK;
@@ -157,15 +220,19 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
     cudaStreamDestroy(cap);
     return cuda_fail(e, "cudaStreamBeginCapture", __FILE__, __LINE__);
   }
-  for (int i = 0; i < n && rc == HOLO_OK; ++i)
-    rc = launch_gather_apf(pr[i].amp, pr[i].phase, b->plans[i]->order_s, b->plans[i]->N,
-                           b->plans[i]->n_pad, const_cast<float2 *>(probs[i].apf_s), cap);
+  rc = launch_gather_apf_batched(gathers_dev, n, gather_blocks, cap);
   if (rc == HOLO_OK && ng > 0 && cudaMemsetAsync(queues, 0, sizeof(int) * ng, cap) != cudaSuccess)
     rc = fail(HOLO_ERR_CUDA, "queue reset during capture");
   for (int g = 0; g < ng && rc == HOLO_OK; ++g)
     if (!groups[g].items.empty())
       rc = launch_split_batched(probs_dev, groups[g].items_dev, (int)groups[g].items.size(),
                                 queues + g, groups[g].variant, groups[g].grid, h->dev_err, cap);
+  if (rc == HOLO_OK) rc = launch_expand_batched(expands_dev, offs_dev, totals, ne, h->dev_err, cap);
+  for (ExpandProblem &E : slabbed)
+    for (E.t0 = 0; E.t0 < E.nT && rc == HOLO_OK; E.t0 += E.slab) {
+      E.nTs = std::min(E.slab, E.nT - E.t0);
+      rc = launch_expand(E, h->dev_err, cap);
+    }
   if (rc == HOLO_OK) rc = launch_reduce_batched(probs_dev, offsets_dev, n, offsets[n], cap);
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(cap, &graph);

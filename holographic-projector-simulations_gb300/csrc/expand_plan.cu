@@ -32,7 +32,8 @@ int nodes_for(double z, double eta) {
 }  // namespace
 
 ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int M, int least_s,
-                           int least_t, double k, double direct_seconds, int sm_count) {
+                           int least_t, double k, double direct_seconds, double launches,
+                           int sm_count) {
   ExpandChoice best;
   double gap2 = 0.0, e[3];
   for (int d = 0; d < 3; ++d) {
@@ -84,11 +85,12 @@ ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int 
       const double clocks = kMomentClocks * (double)N * ceil(nT / 64) * 64 +
                             kTargetClocks * ceil((double)M / 128) * 128 * ceil(nS / 32) * 32 +
                             kNodePairClocks * nS * nT * 128.0 * ch.px * ch.py;
-      const double seconds = kExpandOverhead + clocks / (sm_count * 1.9e9);
+      const double seconds = launches + clocks / (sm_count * 1.9e9);
       if (seconds < best_s) {
         best_s = seconds;
         best = ch;
         best.use = true;
+        best.seconds = seconds;
       }
     }
   }
@@ -96,7 +98,7 @@ ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int 
 }
 
 ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk, double2 *y,
-                              ExpandScratch &tmp) {
+                              double share, ExpandScratch &tmp) {
   const Variant V = split_variant(p->variant);
   ExpandProblem P{};
   P.geo_s = p->geo_s;
@@ -129,7 +131,7 @@ ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk,
   const size_t most = std::max<size_t>(1, ((size_t)1 << 30) / row);
   P.slab = most >= (size_t)P.nT ? P.nT : most >= 64 ? (int)(most / 64 * 64) : (int)most;
   // enough moments blocks for three waves of two per SM, enough target blocks for two of one
-  const int sms = p->h->sm_count;
+  const int sms = std::max(1, (int)(share * p->h->sm_count));
   const int mom = P.nS * ((P.slab + 63) / 64);
   P.ksplit = std::max(1, std::min({(6 * sms + mom - 1) / mom, P.ns / 64, 8}));
   const int blocks = (int)(((long long)P.slab * P.nt + 127) / 128);
@@ -153,7 +155,7 @@ ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk,
 int expand_execute(holo_plan_s *p, const ExpandChoice &ch, double sk, const double *amp,
                    const double *phase, double2 *y, cudaStream_t s) {
   ExpandScratch size;
-  expand_describe(p, ch, sk, y, size);
+  expand_describe(p, ch, sk, y, 1.0, size);
   struct Buffer {
     void *p;
     cudaStream_t s;
@@ -162,7 +164,7 @@ int expand_execute(holo_plan_s *p, const ExpandChoice &ch, double sk, const doub
   if (!buf.p) return fail(HOLO_ERR_ALLOC, "expansion scratch of %zu bytes", size.bytes);
   ExpandScratch tmp;
   tmp.base = static_cast<unsigned char *>(buf.p);
-  ExpandProblem P = expand_describe(p, ch, sk, y, tmp);
+  ExpandProblem P = expand_describe(p, ch, sk, y, 1.0, tmp);
   HOLO_TRY(launch_gather_apf(amp, phase, p->order_s, p->N, p->n_pad, const_cast<float2 *>(P.apf_s), s));
   HOLO_TRY(profile_mark(p->h, s, true));
   for (P.t0 = 0; P.t0 < P.nT; P.t0 += P.slab) {

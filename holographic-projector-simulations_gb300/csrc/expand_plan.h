@@ -6,9 +6,8 @@
 namespace holo {
 
 // SM clocks of the expansion kernels (GB300), per point evaluation of the moments and
-// targets kernels and per pair of nodes of the translation; seconds of their launches.
+// targets kernels and per pair of nodes of the translation.
 constexpr double kMomentClocks = 1.6, kTargetClocks = 2.0, kNodePairClocks = 0.3;
-constexpr double kExpandOverhead = 30e-6, kPairOverhead = 10e-6;
 
 // One device buffer for all of a sum's scratch: a first pass over the takes adds up the size,
 // a second one hands out the addresses.
@@ -23,9 +22,10 @@ struct ExpandScratch {
   }
 };
 
-// The descriptor of a sum (all but its slab) with its buffers taken from `tmp`.
+// The descriptor of a sum (all but its slab) with its buffers taken from `tmp`; share: the
+// part of the GPU that it should fill (1 alone, its part of the work in a batch).
 ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk, double2 *y,
-                              ExpandScratch &tmp);
+                              double share, ExpandScratch &tmp);
 int expand_execute(holo_plan_s *p, const ExpandChoice &ch, double sk, const double *amp,
                    const double *phase, double2 *y, cudaStream_t s);
 

@@ -209,6 +209,15 @@ int launch_rel_hilo(const double *pos_sorted, int n, int n_out, const double *ti
                     float *out, cudaStream_t s);
 int launch_gather_apf(const double *amp, const double *phase, const int32_t *order, int n,
                       int n_pad, float2 *out, cudaStream_t s);
+// The gather of many problems in one launch; first: their first blocks of 1024 records.
+struct GatherApf {
+  const double *amp, *phase;
+  const int32_t *order;
+  int n, n_pad;
+  float2 *out;
+  int first;
+};
+int launch_gather_apf_batched(const GatherApf *sets_dev, int n_sets, int blocks, cudaStream_t s);
 
 // kernel_split.cu
 // kernel_tc.cu: the tensor-core split kernel (pair model 3) on source tiles of `cs`
@@ -291,15 +300,22 @@ struct ExpandProblem {
   double sk;
 };
 int launch_expand(const ExpandProblem &p, int *err, cudaStream_t s);
+// The same kernels over many problems (each one slab), one launch each: offs holds, for each
+// of the four kernels, the first block of every problem and the total (4 x (n + 1) ints).
+void expand_blocks(const ExpandProblem &p, int blocks[4]);
+int launch_expand_batched(const ExpandProblem *probs_dev, const int *offs_dev, const int *totals,
+                          int n, int *err, cudaStream_t s);
 // What a sum of N sources and M targets with these box statistics and wave number takes:
 // the cluster levels (at least least_s and least_t, the pair kernel's tiles) and node counts,
 // or use = false where the pair kernels are faster or no clusters hold the truncation bound.
 struct ExpandChoice {
   bool use = false;
+  double seconds = 0.0;  // estimate
   int ls = 0, lt = 0, px = 0, py = 0, ax = 0, ay = 0;
 };
 ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int M, int least_s,
-                           int least_t, double k, double direct_seconds, int sm_count);
+                           int least_t, double k, double direct_seconds, double launches,
+                           int sm_count);
 
 // kernel_fp64.cu
 int launch_fp64(const Fp64Problem &p, int variant, int grid, bool const_phase, int *err,
@@ -390,17 +406,22 @@ namespace holo {
 void *pool_alloc(holo_handle h, size_t bytes, cudaStream_t s);
 void pool_free(void *p, cudaStream_t s);
 int size_bucket(size_t N, size_t M);
+// k_once: the wave number of the one transform this plan is for (0: a plan to keep, with the
+// positions its adjoint would need); where that runs by cluster expansions the Hilbert tiles
+// do, whatever their bound for the pair kernels.
 // known_order_s / known_order_t: the tile order of the same source / target array
 // from another split plan (copied instead of recomputed), of tiling known_tiling_s/t
 int plan_create_impl(holo_handle h, const double *u_dev, size_t N, const double *v_dev,
                      size_t M, int precision, int forced_variant, cudaStream_t s,
                      holo_plan_s **out, const int32_t *known_order_s = nullptr,
                      const int32_t *known_order_t = nullptr, int known_tiling_s = kTileHilbert,
-                     int known_tiling_t = kTileHilbert);
+                     int known_tiling_t = kTileHilbert, double k_once = 0.0);
 int plan_execute_impl(holo_plan_s *p, int sign, double lambda, const double *amp_dev,
                       const double *phase_dev, double2 *y_dev, int flags, cudaStream_t s);
 void plan_release(holo_plan_s *p, cudaStream_t s);
-ExpandChoice plan_expansion(holo_plan_s *p, double k);
+// launches: seconds that the expansions' launches cost beyond the pair kernel's (0 in a batch)
+constexpr double kExpandLaunches = 20e-6;
+ExpandChoice plan_expansion(holo_plan_s *p, double k, double launches = kExpandLaunches);
 // probe.cu: bracket a pair-evaluation kernel with events while profiling
 int profile_mark(holo_handle h, cudaStream_t s, bool begin);
 }  // namespace holo

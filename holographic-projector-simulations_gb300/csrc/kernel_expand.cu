@@ -773,33 +773,44 @@ __global__ void __launch_bounds__(kTgtThreads, 1)
 
 }  // namespace
 
-int expand_setup_blocks(const ExpandProblem &p) {
+void expand_blocks(const ExpandProblem &p, int blocks[4]) {
   const long long n = (long long)p.nTs * p.nS + (p.N + p.cs - 1) / p.cs + (p.M + p.tt - 1) / p.tt +
                       p.nS + p.nT + 2 * kMaxP * kMaxP;
-  return (int)((n + 127) / 128);
-}
-int expand_moments_blocks(const ExpandProblem &p) {
-  return p.nS * ((p.nTs + kGroupT - 1) / kGroupT) * p.ksplit;
-}
-int expand_translate_blocks(const ExpandProblem &p) { return p.nS * p.nTs; }
-int expand_targets_blocks(const ExpandProblem &p) {
+  blocks[0] = (int)((n + 127) / 128);
+  blocks[1] = p.nS * ((p.nTs + kGroupT - 1) / kGroupT) * p.ksplit;
+  blocks[2] = p.nS * p.nTs;
   const long long m0 = (long long)p.t0 * p.nt, m1 = (long long)(p.t0 + p.nTs) * p.nt;
   const long long m = (m1 < p.M ? m1 : p.M) - m0;
-  return (int)((m + kBlockT - 1) / kBlockT) * p.ssplit;
+  blocks[3] = (int)((m + kBlockT - 1) / kBlockT) * p.ssplit;
 }
 
-int launch_expand(const ExpandProblem &p, int *err, cudaStream_t s) {
-  HOLO_TRY((kernel_setup<k_expand_moments<false>>(kMomThreads, (int)MomentsSmem::bytes, nullptr)));
-  HOLO_TRY((kernel_setup<k_expand_targets<false>>(kTgtThreads, (int)TargetsSmem::bytes, nullptr)));
-  k_expand_setup<false><<<expand_setup_blocks(p), 128, 0, s>>>(p, nullptr, nullptr, 1);
-  k_expand_moments<false><<<expand_moments_blocks(p), kMomThreads, MomentsSmem::bytes, s>>>(
-      p, nullptr, nullptr, 1, err);
-  k_expand_translate<false><<<expand_translate_blocks(p), kNodes, 0, s>>>(p, nullptr, nullptr, 1);
-  k_expand_targets<false><<<expand_targets_blocks(p), kTgtThreads, TargetsSmem::bytes, s>>>(
-      p, nullptr, nullptr, 1, err);
+template <bool BATCHED>
+static int launch_all(const ExpandProblem &p, const ExpandProblem *probs, const int *offs,
+                      const int *blocks, int n, int *err, cudaStream_t s) {
+  HOLO_TRY((kernel_setup<k_expand_moments<BATCHED>>(kMomThreads, (int)MomentsSmem::bytes, nullptr)));
+  HOLO_TRY((kernel_setup<k_expand_targets<BATCHED>>(kTgtThreads, (int)TargetsSmem::bytes, nullptr)));
+  const int step = BATCHED ? n + 1 : 0;
+  k_expand_setup<BATCHED><<<blocks[0], 128, 0, s>>>(p, probs, offs, n);
+  k_expand_moments<BATCHED><<<blocks[1], kMomThreads, MomentsSmem::bytes, s>>>(p, probs, offs + step,
+                                                                              n, err);
+  k_expand_translate<BATCHED><<<blocks[2], kNodes, 0, s>>>(p, probs, offs + 2 * step, n);
+  k_expand_targets<BATCHED><<<blocks[3], kTgtThreads, TargetsSmem::bytes, s>>>(
+      p, probs, offs + 3 * step, n, err);
   note_launches(4);
   HOLO_CUDA(cudaGetLastError());
   return HOLO_OK;
+}
+
+int launch_expand(const ExpandProblem &p, int *err, cudaStream_t s) {
+  int blocks[4];
+  expand_blocks(p, blocks);
+  return launch_all<false>(p, nullptr, nullptr, blocks, 1, err, s);
+}
+
+int launch_expand_batched(const ExpandProblem *probs_dev, const int *offs_dev, const int *totals,
+                          int n, int *err, cudaStream_t s) {
+  if (n <= 0) return HOLO_OK;
+  return launch_all<true>(ExpandProblem{}, probs_dev, offs_dev, totals, n, err, s);
 }
 
 }  // namespace holo

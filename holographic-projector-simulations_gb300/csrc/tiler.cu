@@ -782,20 +782,35 @@ __global__ void __launch_bounds__(256) k_rel_hilo(const double *__restrict__ pos
 }
 
 // (phase reduced to [-pi, pi], amplitude) in float, tile order.
+__device__ __forceinline__ float2 apf_record(const double *amp, const double *phase,
+                                             const int32_t *order, int n, int i) {
+  if (i >= n) return make_float2(0.f, 0.f);
+  const int j = order ? order[i] : i;
+  const double p = phase[j];
+  const double q = rint(p * kInvTwoPi);  // two-constant Cody-Waite reduction
+  const double r = fma(-q, kTwoPiLo, fma(-q, kTwoPiHi, p));
+  return make_float2((float)r, (float)amp[j]);
+}
 __global__ void __launch_bounds__(256) k_gather_apf(const double *__restrict__ amp,
                                                     const double *__restrict__ phase,
                                                     const int32_t *__restrict__ order, int n,
                                                     int n_pad, float2 *__restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_pad; i += gridDim.x * blockDim.x) {
-    if (i < n) {
-      const int j = order ? order[i] : i;
-      const double p = phase[j];
-      const double q = rint(p * kInvTwoPi);  // two-constant Cody-Waite reduction
-      const double r = fma(-q, kTwoPiLo, fma(-q, kTwoPiHi, p));
-      out[i] = make_float2((float)r, (float)amp[j]);
-    } else {
-      out[i] = make_float2(0.f, 0.f);
-    }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_pad; i += gridDim.x * blockDim.x)
+    out[i] = apf_record(amp, phase, order, n, i);
+}
+__global__ void __launch_bounds__(256) k_gather_apf_batched(const GatherApf *__restrict__ sets,
+                                                            int n_sets) {
+  int lo = 0, hi = n_sets;  // the last set whose first block is <= this one
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (sets[mid].first <= (int)blockIdx.x) lo = mid; else hi = mid;
+  }
+  const GatherApf G = sets[lo];
+  const int i0 = (blockIdx.x - G.first) * 1024 + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = i0 + 256 * k;
+    if (i < G.n_pad) G.out[i] = apf_record(G.amp, G.phase, G.order, G.n, i);
   }
 }
 
@@ -971,6 +986,13 @@ int launch_gather_apf(const double *amp, const double *phase, const int32_t *ord
                       int n_pad, float2 *out, cudaStream_t s) {
   if (n_pad <= 0) return HOLO_OK;
   k_gather_apf<<<grid_for(n_pad, 256, 8192), 256, 0, s>>>(amp, phase, order, n, n_pad, out); note_launches(1);
+  HOLO_CUDA(cudaGetLastError());
+  return HOLO_OK;
+}
+
+int launch_gather_apf_batched(const GatherApf *sets_dev, int n_sets, int blocks, cudaStream_t s) {
+  if (n_sets <= 0 || blocks <= 0) return HOLO_OK;
+  k_gather_apf_batched<<<blocks, 256, 0, s>>>(sets_dev, n_sets); note_launches(1);
   HOLO_CUDA(cudaGetLastError());
   return HOLO_OK;
 }
