@@ -227,11 +227,11 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
     if (!groups[g].items.empty())
       rc = launch_split_batched(probs_dev, groups[g].items_dev, (int)groups[g].items.size(),
                                 queues + g, groups[g].variant, groups[g].grid, h->dev_err, cap);
-  if (rc == HOLO_OK) rc = launch_expand_batched(expands_dev, offs_dev, totals, ne, h->dev_err, cap);
+  if (rc == HOLO_OK) rc = launch_expand_batched(expands_dev, offs_dev, totals, ne, h->sm_count, h->dev_err, cap);
   for (ExpandProblem &E : slabbed)
     for (E.t0 = 0; E.t0 < E.nT && rc == HOLO_OK; E.t0 += E.slab) {
       E.nTs = std::min(E.slab, E.nT - E.t0);
-      rc = launch_expand(E, h->dev_err, cap);
+      rc = launch_expand(E, h->sm_count, h->dev_err, cap);
     }
   if (rc == HOLO_OK) rc = launch_reduce_batched(probs_dev, offsets_dev, n, offsets[n], cap);
   cudaGraph_t graph = nullptr;

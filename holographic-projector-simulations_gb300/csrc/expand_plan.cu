@@ -31,6 +31,49 @@ int nodes_for(double z, double eta) {
 
 }  // namespace
 
+// Shares of a cluster's sources, and of the source clusters, that give every SM work: three
+// waves of two moments blocks, two target items.
+static int moment_shares(int nS, int nT, int ns, int sms) {
+  const int blocks = nS * ((nT + 63) / 64);
+  return std::max(1, std::min({(6 * sms + blocks - 1) / blocks, ns / 64, 32}));
+}
+static int target_shares(int nS, int M, int sms) {
+  const int blocks = (M + 127) / 128;
+  return std::max(1, std::min((2 * sms + blocks - 1) / blocks, (nS + 31) / 32));
+}
+
+// SM clocks that the three kernels take (GB300, the constants of expand_plan.h): whole waves of
+// moments blocks, of target items and of translation blocks.
+static double expand_clocks(const ExpandChoice &ch, int N, int M, int sms) {
+  const int ns = 256 << ch.ls, nS = box_count(N, ch.ls), nT = box_count(M, ch.lt);
+  const int ksplit = moment_shares(nS, nT, ns, sms), ssplit = target_shares(nS, M, sms);
+  const double blocks = (double)nS * ((nT + 63) / 64) * ksplit;
+  const double stages = ceil(ceil(std::min(ns, N) / 64.0) / ksplit);
+  const double moments = kMomentStage * stages * (blocks <= sms ? 1.0 : 2.0 * ceil(blocks / (2.0 * sms)));
+  const double items = ceil((M + 127) / 128 * (double)ssplit / sms);
+  const double targets = items * (kTargetItem + kTargetGroup * ceil((nS + 31) / 32 / (double)ssplit));
+  const double translate = std::max(kNodePairClocks * 128.0 * ch.px * ch.py * nS * nT / sms,
+                                    kTranslateLatency * ch.px * ch.py);
+  return moments + targets + translate;
+}
+
+int expand_quads(int px, int py, uint32_t *quads) {
+  const int qx = px / 4, rx = px % 4, qy = py / 4;
+  int n = 0;
+  auto add = [&](uint32_t which, uint32_t scalar, uint32_t quad) {
+    if (quads && n < 32) quads[n] = which << 16 | scalar << 8 | quad;
+    ++n;
+  };
+  for (int a = 0; a < px; ++a)
+    for (int q = 0; q < qy; ++q) add(0, a, q);
+  for (int b = 4 * qy; b < py; ++b) {
+    for (int q = 0; q < qx; ++q) add(1, b, q);
+  }
+  if (rx)
+    for (int b = 4 * qy; b < py; ++b) add(1, b, qx);
+  return n;
+}
+
 ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int M, int least_s,
                            int least_t, double k, double direct_seconds, double launches,
                            int sm_count) {
@@ -60,7 +103,7 @@ ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int 
       if (!(k * src.hd[ls][f] * ht / gap < 1e-7 && k * tgt.hd[lt][f] * hs / gap < 1e-7)) continue;
       // FP32 rounding of the curvature term, (hs + ht)^2 / 2r, and its truncated series
       const double c = (hs + ht) * (hs + ht) / gap;
-      if (!(k * c * ldexp(1.0, -23) < 2e-6 && k * c * pow(rel, 4) / 16.0 < 1e-7)) continue;
+      if (!(k * c * ldexp(1.0, -23) < 3e-6 && k * c * pow(rel, 4) / 16.0 < 1e-7)) continue;
       ExpandChoice ch;
       ch.ls = ls;
       ch.lt = lt;
@@ -80,12 +123,12 @@ ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int 
       ch.px = nodes(ch.ax, ch.ay);
       ch.py = nodes(ch.ay, ch.ax);
       if (!ch.px || !ch.py || ch.px * ch.py > kExpandNodes) continue;
-      const double nS = box_count(N, ls), nT = box_count(M, lt);
-      // SM clocks per unit of work, measured (kernel_expand.cu)
-      const double clocks = kMomentClocks * (double)N * ceil(nT / 64) * 64 +
-                            kTargetClocks * ceil((double)M / 128) * 128 * ceil(nS / 32) * 32 +
-                            kNodePairClocks * nS * nT * 128.0 * ch.px * ch.py;
-      const double seconds = launches + clocks / (sm_count * 1.9e9);
+      if (expand_quads(ch.px, ch.py, nullptr) > 32) {
+        std::swap(ch.px, ch.py);
+        std::swap(ch.ax, ch.ay);
+        if (expand_quads(ch.px, ch.py, nullptr) > 32) continue;
+      }
+      const double seconds = launches + expand_clocks(ch, N, M, sm_count) / 1.9e9;
       if (seconds < best_s) {
         best_s = seconds;
         best = ch;
@@ -123,6 +166,7 @@ ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk,
   P.py = ch.py;
   P.ax = ch.ax;
   P.ay = ch.ay;
+  P.n_quads = expand_quads(P.px, P.py, P.quads);
   P.sk = sk;
   P.kap = (float)(0.5 * sk);
   // target clusters per launch: at most 1 GiB of frames, moments and coefficients
@@ -130,13 +174,9 @@ ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk,
   const size_t row = (size_t)P.nS * (80 + 4 * 1024) + (size_t)groups_s * 65536;
   const size_t most = std::max<size_t>(1, ((size_t)1 << 30) / row);
   P.slab = most >= (size_t)P.nT ? P.nT : most >= 64 ? (int)(most / 64 * 64) : (int)most;
-  // enough moments blocks for three waves of two per SM, enough target blocks for two of one
   const int sms = std::max(1, (int)(share * p->h->sm_count));
-  const int mom = P.nS * ((P.slab + 63) / 64);
-  P.ksplit = std::max(1, std::min({(6 * sms + mom - 1) / mom, P.ns / 64, 8}));
-  const int blocks = (int)(((long long)P.slab * P.nt + 127) / 128);
-  const int tgt = std::min(blocks, (P.M + 127) / 128);
-  P.ssplit = std::max(1, std::min((2 * sms + tgt - 1) / tgt, groups_s));
+  P.ksplit = moment_shares(P.nS, P.slab, P.ns, sms);
+  P.ssplit = target_shares(P.nS, std::min(P.slab * P.nt, P.M), sms);
   const size_t pairs = (size_t)P.slab * P.nS;
   P.apf_s = tmp.take<float2>(p->n_pad);
   P.frames = tmp.take<float>(12 * pairs);
@@ -169,7 +209,7 @@ int expand_execute(holo_plan_s *p, const ExpandChoice &ch, double sk, const doub
   HOLO_TRY(profile_mark(p->h, s, true));
   for (P.t0 = 0; P.t0 < P.nT; P.t0 += P.slab) {
     P.nTs = std::min(P.slab, P.nT - P.t0);
-    HOLO_TRY(launch_expand(P, p->h->dev_err, s));
+    HOLO_TRY(launch_expand(P, p->h->sm_count, p->h->dev_err, s));
   }
   if (P.ssplit > 1) HOLO_TRY(launch_reduce(P.partial, P.ssplit, P.M, P.order_t, y, s));
   return profile_mark(p->h, s, false);

@@ -5,9 +5,11 @@
 
 namespace holo {
 
-// SM clocks of the expansion kernels (GB300), per point evaluation of the moments and
-// targets kernels and per pair of nodes of the translation.
-constexpr double kMomentClocks = 1.6, kTargetClocks = 2.0, kNodePairClocks = 0.3;
+// SM clocks of the expansion kernels (GB300): a moments block's 64 sources x 64 target clusters
+// alone on an SM (half the rate for each of two), a target item's set-up and its 32 source
+// clusters, one pair of nodes of the translation at full load, and per node pair of a thread.
+constexpr double kMomentStage = 7000.0, kTargetItem = 5000.0, kTargetGroup = 5000.0,
+                 kNodePairClocks = 0.27, kTranslateLatency = 80.0;
 
 // One device buffer for all of a sum's scratch: a first pass over the takes adds up the size,
 // a second one hands out the addresses.

@@ -294,17 +294,22 @@ struct ExpandProblem {
   float *coeffs;                     // [nTs][nS / 32][2][hi, lo][8][64 x 8]: MMA operand
   int N, M, cs, tt, ns, nt, nS, nT, t0, nTs, slab;  // slab: target clusters per launch
   int px, py, ax, ay;                // nodes along the coordinate axes ax and ay
+  // the orders (a, b) of the coefficients in MMA depth, four at a time: entry q holds
+  // (which << 16) | (scalar << 8) | quad -- T_scalar of one axis times four consecutive
+  // T of the other (which: 0 the four along ay, 1 along ax; orders past the last are 0)
+  int n_quads;
+  uint32_t quads[32];
   int ksplit, ssplit;                // shares of a cluster's sources / of the source clusters
   int cs_log2, tt_log2;
   float kap;                         // s k / 2
   double sk;
 };
-int launch_expand(const ExpandProblem &p, int *err, cudaStream_t s);
+int launch_expand(const ExpandProblem &p, int sms, int *err, cudaStream_t s);
 // The same kernels over many problems (each one slab), one launch each: offs holds, for each
 // of the four kernels, the first block of every problem and the total (4 x (n + 1) ints).
 void expand_blocks(const ExpandProblem &p, int blocks[4]);
 int launch_expand_batched(const ExpandProblem *probs_dev, const int *offs_dev, const int *totals,
-                          int n, int *err, cudaStream_t s);
+                          int n, int sms, int *err, cudaStream_t s);
 // What a sum of N sources and M targets with these box statistics and wave number takes:
 // the cluster levels (at least least_s and least_t, the pair kernel's tiles) and node counts,
 // or use = false where the pair kernels are faster or no clusters hold the truncation bound.
@@ -313,6 +318,8 @@ struct ExpandChoice {
   double seconds = 0.0;  // estimate
   int ls = 0, lt = 0, px = 0, py = 0, ax = 0, ay = 0;
 };
+// The quads of px x py orders into `quads` (may be null); their count (more than 32: no layout).
+int expand_quads(int px, int py, uint32_t *quads);
 ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int M, int least_s,
                            int least_t, double k, double direct_seconds, double launches,
                            int sm_count);

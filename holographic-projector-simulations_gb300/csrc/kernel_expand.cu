@@ -28,6 +28,8 @@
 // registers every 64 sources and keeps the small cross products of the splits in an
 // accumulator of their own; the target kernel adds the cross products and the high
 // orders, which are small, before the low ones.
+#include <algorithm>
+
 #include "internal.cuh"
 #include "ptx.cuh"
 
@@ -85,13 +87,30 @@ __device__ __forceinline__ void add_ff(float ah, float al, float bh, float bl, f
   l = __fsub_rn(e, __fsub_rn(h, s));
 }
 
-// s k (c / 2q - c^2 / 8q^3) = kap (c / q) (1 - (c / q) / 4q), kap = s k / 2: the curvature
-// term rho of r = q + rho, c = |perpendicular offset|^2 (the next term, c^3 / 16 q^5, is
-// below 1e-7 rad where expand_choose admits the clusters).
-__device__ __forceinline__ float curvature(float kap, float c, float q, float &iq, float &h) {
-  iq = ptx::rcp_approx(q);
-  h = c * iq;
+// s k rho of r = q + rho, rho = c / (q + r), c = |perpendicular offset|^2, to c^2:
+// kap (c / q) (1 - c / 4q^2), kap = s k / 2 (the next term, c^3 / 16 q^5, is below 1e-7 rad where
+// expand_choose admits the clusters).
+__device__ __forceinline__ float curvature(float kap, float c, float q) {
+  const float iq = ptx::rcp_approx(q), h = c * iq;
   return kap * h * fmaf(-0.25f * h, iq, 1.f);
+}
+
+// Mean error of cos.approx over a turn (GB300, 6.7e7 uniform angles; sin.approx has none).  Over
+// sources of random phase every other error averages out, but this one adds up: over a
+// cluster of 4096 it is sqrt(4096) 4e-8 = 2.6e-6 of the moment, more than all the rest
+// (1.5e-6 of the 512^2 -> 1024^2 field with it, 6e-7 without).
+constexpr float kCosBias = 4.034e-8f;
+
+// (S + E + c) mod 2 pi for the curvature term c of some radians, |S| < 2^16: the turns are counted
+// with c included and c is added where the reduced sum is small, so that the result stays
+// within about [-pi, pi], where sin.approx is at its most exact (its product with 1 / 2 pi rounds
+// by up to 7e-7 rad beyond a turn).
+__device__ __forceinline__ float reduce_two_pi_with(float S, float E, float c) {
+  const float n = __fsub_rn(fmaf(__fadd_rn(S, c), 0.159154943f, 12582912.0f), 12582912.0f);
+  float r = __fadd_rn(fmaf(-n, 6.28125f, S), c);
+  r = fmaf(-n, 1.935307169e-3f, r);   // fl32(2 pi - C1)
+  r = fmaf(-n, 1.025313168e-11f, r);  // fl32(2 pi - C1 - C2)
+  return __fadd_rn(r, E);
 }
 
 // ---- set-up: frames of all cluster pairs, offsets of the variant's tile centres from the
@@ -317,13 +336,13 @@ __global__ void __launch_bounds__(kMomThreads, 2)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float th[3] = {q[0][j], q[1][j], q[2][j]}, tl[3] = {q[3][j], q[4][j], q[5][j]};
-          float s, e, s2, e2, iq, hq;
+          float s, e, s2, e2;
           dot3_ff(ah, al, th, tl, s, e);
           two_sum(q[7][j], -s, s2, e2);
           const float ps = fmaf(ef[0], th[0], fmaf(ef[1], th[1], ef[2] * th[2]));
-          const float ph = reduce_two_pi_ff(s2, __fsub_rn(e2, e)) +
-                           curvature(kap, fmaf(-ps, ps, q[6][j]), r0 - ps, iq, hq);
-          re[j] = q[8][j] * ptx::cos_approx(ph);
+          const float ph = reduce_two_pi_with(
+              s2, __fsub_rn(e2, e), curvature(kap, fmaf(-ps, ps, q[6][j]), r0 - ps));
+          re[j] = fmaf(q[8][j], ptx::cos_approx(ph), -kCosBias * q[8][j]);
           im[j] = q[8][j] * ptx::sin_approx(ph);
         }
         const int o = (quad >> 1) * (2 * kGroupT * kTcK) + 32 * (quad & 1);
@@ -471,7 +490,6 @@ __global__ void __launch_bounds__(kNodes) k_expand_translate(
     const float ex[3] = {f2.x, f2.y, f2.z}, e1[3] = {f3.x, f3.y, f3.z}, e2[3] = {f4.x, f4.y, f4.z};
     const float4 ht = reinterpret_cast<const float4 *>(P.half_t)[P.t0 + Tl];
     const float4 hs = reinterpret_cast<const float4 *>(P.half_s)[S];
-    float iq, h;
     const float ux = x * ht.x, uy = y * ht.y;
     const float e1x = pick(e1, P.ax), e1y = pick(e1, P.ay), e2x = pick(e2, P.ax);
     const float e2y = pick(e2, P.ay), exx = pick(ex, P.ax), exy = pick(ex, P.ay);
@@ -479,23 +497,25 @@ __global__ void __launch_bounds__(kNodes) k_expand_translate(
     ty = fmaf(e2x, ux, e2y * uy);
     tz = fmaf(exx, ux, exy * uy);
     ct = fmaf(tx, tx, ty * ty);
-    rt = curvature(kap, ct, r0 + tz, iq, h);
+    rt = curvature(kap, ct, r0 + tz);
     const float wx = x * hs.x, wy = y * hs.y;
     const float sx = fmaf(e1x, wx, e1y * wy), sy = fmaf(e2x, wx, e2y * wy);
     const float sz = fmaf(exx, wx, exy * wy), cs = fmaf(sx, sx, sy * sy);
     node_a[n] = make_float4(-2.f * sx, -2.f * sy, sz, cs);
-    node_b[n] = make_float4(s.x, s.y, curvature(kap, cs, r0 - sz, iq, h), 0.f);
+    node_b[n] = make_float4(s.x, s.y, curvature(kap, cs, r0 - sz), 0.f);
   }
   __syncthreads();
-  // V_n = sum_j e^{i s k psi} / r W_j
+  // V_n = sum_j e^{i s k psi} / r W_j, psi = c u - c_t u_t - c_s u_s with c = c_t + c_s - 2 t.s
+  // (the same regrouped into small differences, -2 t.s u + c_t (u - u_t) + c_s (u - u_s), took 16 %
+  // longer and was no more exact in the field)
   float vre = 0.f, vim = 0.f;
   const float qt = r0 + tz;
 #pragma unroll 4
   for (int j = 0; j < np; ++j) {
     const float4 s = node_a[j], w = node_b[j];
-    float iq, h;
-    const float c = fmaf(tx, s.x, fmaf(ty, s.y, ct + s.w));
-    const float psi = curvature(kap, c, qt - s.z, iq, h) - rt - w.z;
+    const float c = fmaf(tx, s.x, fmaf(ty, s.y, ct + s.w)), iq = ptx::rcp_approx(qt - s.z);
+    const float h = c * iq;
+    const float psi = kap * h * fmaf(-0.25f * h, iq, 1.f) - rt - w.z;
     const float ir = iq * fmaf(-0.5f * h, iq, 1.f);  // 1 / r to c / q^2
     const float cr = ir * ptx::cos_approx(psi), ci = ir * ptx::sin_approx(psi);
     vre = fmaf(cr, w.x, fmaf(-ci, w.y, vre));
@@ -515,260 +535,394 @@ __global__ void __launch_bounds__(kNodes) k_expand_translate(
     vb[n] = s;
   }
   __syncthreads();
+  // thread n: the coefficient of slot n of the MMA depth
   float2 nu = make_float2(0.f, 0.f);
-  if (n < np)
-    for (int j = 0; j < py; ++j) {
-      const float m = my[b * kMaxP + j];
-      const float2 v = vb[a * py + j];
-      nu.x = fmaf(m, v.x, nu.x);
-      nu.y = fmaf(m, v.y, nu.y);
-    }
-  // operand rows S % 32 (re) and 32 + S % 32 (im), depth n: halves of 64 nodes, hi then lo
-  const int nSG = (P.nS + kGroupS - 1) / kGroupS;
-  float *o = P.coeffs + (((size_t)Tl * nSG + S / kGroupS) * 2 + (n >> 6)) * kHalfFloats +
-             (size_t)((n & 63) >> 3) * (2 * kGroupS * kTcK);
-  const int re = tc_off(S % kGroupS, n & 7), im = tc_off(kGroupS + S % kGroupS, n & 7);
+  if (n < 4 * P.n_quads) {
+    const uint32_t quad = P.quads[n >> 2];
+    const int one = (quad >> 8) & 255, four = 4 * (quad & 255) + (n & 3);
+    const int oa = quad >> 16 ? four : one, ob = quad >> 16 ? one : four;
+    if (oa < px && ob < py)
+      for (int j = 0; j < py; ++j) {
+        const float m = my[ob * kMaxP + j];
+        const float2 v = vb[oa * py + j];
+        nu.x = fmaf(m, v.x, nu.x);
+        nu.y = fmaf(m, v.y, nu.y);
+      }
+  }
+  // operand rows S % 32 (re), 32 + S % 32 (im) and, 64 rows on, their TF32 remainders; depth n
+  const int nSG = (P.nS + kGroupS - 1) / kGroupS, row = S % kGroupS;
+  float *o = P.coeffs + ((size_t)Tl * nSG + S / kGroupS) * 2 * kHalfFloats +
+             (size_t)(n >> 3) * (4 * kGroupS * kTcK);
   const float rh = ptx::to_tf32_int(nu.x), ih = ptx::to_tf32_int(nu.y);
-  o[re] = rh;
-  o[im] = ih;
-  o[kHalfFloats / 2 + re] = ptx::to_tf32_int(__fsub_rn(nu.x, rh));
-  o[kHalfFloats / 2 + im] = ptx::to_tf32_int(__fsub_rn(nu.y, ih));
+  o[tc_off(row, n & 7)] = rh;
+  o[tc_off(kGroupS + row, n & 7)] = ih;
+  o[tc_off(2 * kGroupS + row, n & 7)] = ptx::to_tf32_int(__fsub_rn(nu.x, rh));
+  o[tc_off(3 * kGroupS + row, n & 7)] = ptx::to_tf32_int(__fsub_rn(nu.y, ih));
 }
 
 // ---- targets -------------------------------------------------------------------------------
-// One block: 128 targets of one cluster against a share of the source clusters, 32 at a time:
-// D[target][column] = sum over 128 nodes of weight x coefficient for 32 + 32 columns.  The
-// weights of the targets stay in shared memory for the whole block (128 KB, both TF32 parts);
-// a load warp brings the coefficients by bulk copies, in halves of 64 nodes, and the
-// frames of 32 pairs; 16 consumer warps read D (two TMEM buffers), each thread its target and
-// 8 clusters, rotate by e^{i s k alpha} and sum.
+// Work items are blocks of 128 targets of one cluster against a share of the source clusters:
+// D[target][column] = sum over nodes of weight x coefficient, 32 clusters (32 + 32 columns)
+// at a time.  Persistent CTAs, one per SM, with a role per warp so that an item's weights are
+// built and its coefficients fetched while the previous item's phases are formed:
+//   builders (8 warps)   the weights of the next item's targets into tensor memory (the MMAs' A
+//                        operand, both TF32 parts) once the MMAs of this one are complete,
+//                        the targets' offsets, and the results of the item before
+//   load warp            coefficients (halves of 64 nodes) and frames by bulk copies
+//   MMA warp             one thread issues the products into one of two TMEM buffers
+//   consumers (16 warps) read D, rotate by e^{i s k alpha}, sum: each thread one target and
+//                        8 clusters of every 32
+// Bound by the consumers' FP32 and MUFU work (~3,000 clocks per 32 clusters); a block per
+// item without roles took 12,000 clocks of set-up and tail per item (see the figures at
+// expand_plan.h).  Hand-offs are mbarrier phases; those a waiter may trail by two items come in
+// pairs.
 struct TargetsSmem {
-  static constexpr size_t a = 0;                                    // float [hi, lo][128*128]
-  static constexpr size_t b = a + 2 * kBlockT * kNodes * 4;         // float [2][kHalfFloats]
-  static constexpr size_t cheb = b + 2 * kHalfFloats * 4;           // float [2][16][128]
-  static constexpr size_t frames = cheb + 2 * kMaxP * kBlockT * 4;  // float [2][32][12]
-  static constexpr size_t bars = frames + 2 * kGroupS * 12 * 4;     // uint64 [12]
-  static constexpr size_t misc = bars + 12 * 8;                     // uint32 taddr, abort
+  static constexpr int kStages = 4;                                 // halves of coefficients
+  static constexpr size_t b = 0;                                    // float [4][kHalfFloats]
+  static constexpr size_t quad = b + kStages * kHalfFloats * 4;     // float4 [8][128]: four orders
+  static constexpr size_t cheb = quad + 8 * kBlockT * 16;           // float [24][128]
+  static constexpr size_t rec = cheb + 24 * kBlockT * 4;            // float [2][7][128]
+  static constexpr size_t part = rec + 2 * 7 * kBlockT * 4;         // float4 [4][128]
+  static constexpr size_t frames = part + 4 * kBlockT * 16;         // float [2][32][12]
+  static constexpr size_t bars = frames + 2 * kGroupS * 12 * 4;     // uint64 [21]
+  static constexpr size_t misc = bars + 22 * 8;                     // uint32 taddr, abort
   static constexpr size_t bytes = misc + 16;
 };
 static_assert(TargetsSmem::bytes <= 227 * 1024, "target kernel: shared memory");
-constexpr int kTgtConsumers = 16;                        // then the MMA warp and the load warp
-constexpr int kTgtThreads = 32 * (kTgtConsumers + 2);
+constexpr int kTgtConsumers = 16, kTgtBuilders = 8;
+constexpr int kTgtThreads = 32 * (kTgtConsumers + 2 + kTgtBuilders);
 
 template <bool BATCHED>
 __global__ void __launch_bounds__(kTgtThreads, 1)
     k_expand_targets(const ExpandProblem P0, const ExpandProblem *__restrict__ probs,
-                     const int *__restrict__ offs, int n_probs, int *err) {
+                     const int *__restrict__ offs, int n_items, int *err) {
   extern __shared__ __align__(128) unsigned char smem[];
   using L = TargetsSmem;
-  float *a_hi = reinterpret_cast<float *>(smem + L::a), *a_lo = a_hi + kBlockT * kNodes;
+  constexpr int kStages = L::kStages;
   float *sb = reinterpret_cast<float *>(smem + L::b);
+  float4 *squad = reinterpret_cast<float4 *>(smem + L::quad);
   float *cheb = reinterpret_cast<float *>(smem + L::cheb);
+  float *srec = reinterpret_cast<float *>(smem + L::rec);
+  float4 *part = reinterpret_cast<float4 *>(smem + L::part);
   float *sframes = reinterpret_cast<float *>(smem + L::frames);
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::bars);
-  uint64_t *bfull = bars, *bfree = bars + 2, *dfull = bars + 4, *dfree = bars + 6,
-           *ffull = bars + 8, *ffree = bars + 10;
+  uint64_t *bfull = bars, *bfree = bars + 4, *dfull = bars + 8, *dfree = bars + 10,
+           *ffull = bars + 12, *ffree = bars + 14, *a_ready = bars + 16, *a_free = bars + 18,
+           *parts_ready = bars + 19, *parts_free = bars + 20;
   uint32_t *taddr_slot = reinterpret_cast<uint32_t *>(smem + L::misc);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L::misc + 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool consumer = warp < kTgtConsumers, mma_warp = warp == kTgtConsumers;
-
-  int item;
-  const ExpandProblem &P = find_problem<BATCHED>(P0, probs, offs, n_probs, &item);
-  const int blk = item / P.ssplit, sp = item % P.ssplit;
-  const int m0 = P.t0 * P.nt + blk * kBlockT, Tl = blk * kBlockT / P.nt;
-  const int nSG = (P.nS + kGroupS - 1) / kGroupS;
-  const int g0 = (int)((long long)nSG * sp / P.ssplit), g1 = (int)((long long)nSG * (sp + 1) / P.ssplit);
-  const int px = P.px, py = P.py, np = px * py;
-
-  // half i: nodes 64 .. 127 (i even) or 0 .. 63 (i odd) of cluster group g0 + i / 2
-  const int nh = 2 * (g1 - g0);
-  auto load = [&](int i) {
-    const int st = i & 1, g = g0 + (i >> 1);
-    ptx::mbar_arrive_expect_tx(&bfull[st], kHalfFloats * 4);
-    ptx::bulk_g2s(sb + st * kHalfFloats,
-                  P.coeffs + (((size_t)Tl * nSG + g) * 2 + (1 - st)) * kHalfFloats, kHalfFloats * 4,
-                  &bfull[st]);
-    if (st == 0) {
-      const int d = (i >> 1) & 1, bytes = 48 * min(kGroupS, P.nS - g * kGroupS);
-      ptx::mbar_arrive_expect_tx(&ffull[d], bytes);
-      ptx::bulk_g2s(sframes + d * kGroupS * 12,
-                    P.frames + 12 * ((size_t)Tl * P.nS + g * kGroupS), bytes, &ffull[d]);
-    }
-  };
-  if (tid == 32 * (kTgtConsumers + 1)) {
-    for (int b = 0; b < 2; ++b) {
+  const bool consumer = warp < kTgtConsumers, mma_warp = warp == kTgtConsumers,
+             load_warp = warp == kTgtConsumers + 1;
+  if (tid == 0) {
+    for (int b = 0; b < kStages; ++b) {
       ptx::mbar_init(&bfull[b], 1);
       ptx::mbar_init(&bfree[b], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(&dfull[b], 1);
       ptx::mbar_init(&dfree[b], kTgtConsumers);
       ptx::mbar_init(&ffull[b], 1);
       ptx::mbar_init(&ffree[b], kTgtConsumers);
+      ptx::mbar_init(&a_ready[b], 32 * kTgtBuilders);
     }
+    ptx::mbar_init(a_free, 1);
+    ptx::mbar_init(parts_ready, kTgtConsumers);
+    ptx::mbar_init(parts_free, kBlockT);
     *abort_flag = 0;
     ptx::fence_barrier_init();
-    for (int i = 0; i < min(nh, 2); ++i) load(i);
   }
-  if (mma_warp) ptx::tmem_alloc(taddr_slot, 128);
-
-  // ---- weights of the block's targets ----
-  float th[3] = {0.f, 0.f, 0.f}, tl[3] = {0.f, 0.f, 0.f};  // consumers: target 32 (warp % 4) + lane
-  {
-    const int t = m0 + (tid & (kBlockT - 1));
-    if (consumer && t < P.M) cluster_offset(P.geo_t, P.shift_t, t, P.tt_log2, th, tl);
-    const float4 half = reinterpret_cast<const float4 *>(P.half_t)[P.t0 + Tl];
-    if (tid < kBlockT)
-      cheb_row(pick(th, P.ax) * half.z, px, cheb + tid, kBlockT);
-    else if (tid < 2 * kBlockT)
-      cheb_row(pick(th, P.ay) * half.w, py, cheb + kMaxP * kBlockT + tid - kBlockT, kBlockT);
-  }
-  __syncthreads();
-  if (consumer) {
-    const int row = tid & (kBlockT - 1), n0 = 32 * (tid >> 7);
-    int a = n0 / py, b = n0 % py;
-    for (int q = 0; q < 8; ++q) {
-      float hi[4], lo[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float w = n0 + 4 * q + j < np
-                            ? cheb[a * kBlockT + row] * cheb[(kMaxP + b) * kBlockT + row] : 0.f;
-        if (++b == py) {
-          b = 0;
-          ++a;
-        }
-        hi[j] = ptx::to_tf32_int(w);
-        lo[j] = ptx::to_tf32_int(__fsub_rn(w, hi[j]));
-      }
-      const int n = n0 + 4 * q, o = (n >> 3) * (kBlockT * kTcK) + tc_off(row, n & 7);
-      *reinterpret_cast<float4 *>(a_hi + o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-      *reinterpret_cast<float4 *>(a_lo + o) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-    }
-  }
-  ptx::fence_proxy_async_smem();
+  if (mma_warp) ptx::tmem_alloc(taddr_slot, 512);  // D[2] 128 columns, weights hi and lo 128
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tbase = *taddr_slot;
-  constexpr uint32_t idesc = ptx::tc_idesc_tf32(kBlockT, 2 * kGroupS);
 
-  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);  // (re hi, re lo, im hi, im lo)
-  if (mma_warp) {
-    if (lane == 0) {
-      int issued = 0;
-      for (int i = 0; i < nh; ++i) {
-        const int st = i & 1, gi = i >> 1, d = gi & 1;
-        if (!tc_wait(&bfull[st], gi & 1u, abort_flag, err)) break;
-        if (st == 0 && gi >= 2 && !tc_wait(&dfree[d], ((gi >> 1) - 1) & 1u, abort_flag, err)) break;
-        ptx::tc_fence_after();
-        const float *bh = sb + st * kHalfFloats, *bl = bh + kHalfFloats / 2;
-        const uint32_t dt = tbase + (uint32_t)(2 * kGroupS * d);
-        const int k0 = 8 * (1 - st);
-        for (int k = 7; k >= 0; --k) {  // the cross products of the TF32 parts
-          const uint64_t ah = ptx::tc_smem_desc(a_hi + (k0 + k) * kBlockT * kTcK, kTcLbo, kTcSbo);
-          const uint64_t al = ptx::tc_smem_desc(a_lo + (k0 + k) * kBlockT * kTcK, kTcLbo, kTcSbo);
-          ptx::tc_mma_tf32(dt, ah, ptx::tc_smem_desc(bl + k * 2 * kGroupS * kTcK, kTcLbo, kTcSbo),
-                           idesc, st > 0 || k < 7);
-          ptx::tc_mma_tf32(dt, al, ptx::tc_smem_desc(bh + k * 2 * kGroupS * kTcK, kTcLbo, kTcSbo),
-                           idesc, 1u);
-        }
-        for (int k = 7; k >= 0; --k)
-          ptx::tc_mma_tf32(dt, ptx::tc_smem_desc(a_hi + (k0 + k) * kBlockT * kTcK, kTcLbo, kTcSbo),
-                           ptx::tc_smem_desc(bh + k * 2 * kGroupS * kTcK, kTcLbo, kTcSbo), idesc, 1u);
-        ptx::tc_commit(&bfree[st]);
-        if (st) ptx::tc_commit(&dfull[d]);
-        ++issued;
+  // item -> problem (items of a CTA only go up, so the search goes on from the last one),
+  // target cluster (of the slab), first target, source cluster groups [g0, g1)
+  int prob = 0, first = 0, next = BATCHED ? offs[1] : n_items;
+  struct Item {
+    int Tl, m0, sp, nSG, g0, g1;
+  };
+  auto locate = [&](int item, Item &w) -> const ExpandProblem & {
+    if (BATCHED)
+      while (item >= next) {
+        first = next;
+        ++prob;
+        next = offs[prob + 1];
       }
-      // the MMAs in flight end before the block does
-      for (int i = max(0, issued - 2); i < issued; ++i)
-        ptx::mbar_wait_bounded(&bfree[i & 1], (i >> 1) & 1u, kWaitCycles);
+    const ExpandProblem &P = BATCHED ? probs[prob] : P0;
+    const int blk = (item - first) / P.ssplit;
+    w.sp = (item - first) % P.ssplit;
+    w.m0 = P.t0 * P.nt + blk * kBlockT;
+    w.Tl = blk * kBlockT / P.nt;
+    w.nSG = (P.nS + kGroupS - 1) / kGroupS;
+    w.g0 = (int)((long long)w.nSG * w.sp / P.ssplit);
+    w.g1 = (int)((long long)w.nSG * (w.sp + 1) / P.ssplit);
+    return P;
+  };
+
+  Item w;
+  if (mma_warp) {
+    const uint32_t leader = lane == 0;
+    constexpr uint32_t idesc = ptx::tc_idesc_tf32(kBlockT, 4 * kGroupS);
+    constexpr uint32_t idesc_lo = ptx::tc_idesc_tf32(kBlockT, 2 * kGroupS);
+    // one k step of 8 nodes further: 8 columns of weights, 4096 bytes of coefficients
+    constexpr uint64_t kStepB = 4 * kGroupS * kTcK * 4 / 16;
+    const uint32_t ta = tbase + 256;
+    const uint64_t db0 = ptx::tc_smem_desc(sb, kTcLbo, kTcSbo);
+    uint32_t hc = 0, gc = 0, it = 0;  // halves, groups and items so far
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++it) {
+      const ExpandProblem &P = locate(item, w);
+      const int steps = (P.n_quads + 1) / 2;
+      if (!tc_wait(&a_ready[it & 1], (it >> 1) & 1u, abort_flag, err)) break;
+      for (int g = w.g0; g < w.g1 && !*abort_flag; ++g, ++gc) {
+        const uint32_t d = gc & 1, dt = tbase + 4 * kGroupS * d;
+        if (gc >= 2 && !tc_wait(&dfree[d], ((gc >> 1) - 1) & 1u, abort_flag, err)) break;
+        uint32_t acc = 0;
+        for (int half = steps > 8; half >= 0; --half, ++hc) {
+          const uint32_t st = hc % kStages;
+          if (!tc_wait(&bfull[st], (hc / kStages) & 1u, abort_flag, err)) break;
+          ptx::tc_fence_after();
+          const uint64_t b = db0 + st * (kHalfFloats * 4 / 16);
+          const uint32_t a = ta + 64 * half;
+          const int n = min(8, steps - 8 * half);
+#pragma unroll
+          for (int k = 7; k >= 0; --k) {
+            if (k >= n) continue;
+            // hi x (hi | lo), then lo x hi onto the second product
+            ptx::tc_mma_tf32_ta(dt, a + 8 * k, b + k * kStepB, idesc, acc, leader);
+            ptx::tc_mma_tf32_ta(dt + 2 * kGroupS, a + 128 + 8 * k, b + k * kStepB, idesc_lo, 1u, leader);
+            acc = 1u;
+          }
+          ptx::tc_commit(&bfree[st], leader);
+        }
+        ptx::tc_commit(&dfull[d], leader);
+      }
+      ptx::tc_commit(a_free, leader);
     }
+    // the MMAs in flight end before the CTA does
+    if (it > 0) ptx::mbar_wait_bounded(a_free, (it - 1) & 1u, kWaitCycles);
+    for (uint32_t h = hc > kStages ? hc - kStages : 0; h < hc; ++h)
+      ptx::mbar_wait_bounded(&bfree[h % kStages], (h / kStages) & 1u, kWaitCycles);
     __syncwarp();
-  } else if (!consumer) {
+  } else if (load_warp) {
     if (lane == 0) {
-      int loaded = min(nh, 2);
-      for (int i = 2; i < nh; ++i, ++loaded) {  // half i goes where half i - 2 was
-        if (!tc_wait(&bfree[i & 1], ((i >> 1) - 1) & 1u, abort_flag, err)) break;
-        if (!(i & 1) && i >= 4 && !tc_wait(&ffree[(i >> 1) & 1], ((i >> 2) - 1) & 1u, abort_flag, err))
-          break;
-        load(i);
+      uint32_t hc = 0, gc = 0;
+      for (int item = blockIdx.x; item < n_items && !*abort_flag; item += gridDim.x) {
+        const ExpandProblem &P = locate(item, w);
+        const int steps = (P.n_quads + 1) / 2;
+        for (int g = w.g0; g < w.g1 && !*abort_flag; ++g, ++gc) {
+          const uint32_t d = gc & 1;
+          if (gc >= 2 && !tc_wait(&ffree[d], ((gc >> 1) - 1) & 1u, abort_flag, err)) break;
+          const uint32_t bytes = 48 * min(kGroupS, P.nS - g * kGroupS);
+          ptx::mbar_arrive_expect_tx(&ffull[d], bytes);
+          ptx::bulk_g2s(sframes + d * kGroupS * 12,
+                        P.frames + 12 * ((size_t)w.Tl * P.nS + g * kGroupS), bytes, &ffull[d]);
+          for (int half = steps > 8; half >= 0; --half, ++hc) {
+            const uint32_t st = hc % kStages, bytes_b = 4 * 4 * kGroupS * kTcK * min(8, steps - 8 * half);
+            if (hc >= kStages && !tc_wait(&bfree[st], (hc / kStages - 1) & 1u, abort_flag, err)) break;
+            ptx::mbar_arrive_expect_tx(&bfull[st], bytes_b);
+            ptx::bulk_g2s(sb + st * kHalfFloats,
+                          P.coeffs + (((size_t)w.Tl * w.nSG + g) * 2 + half) * kHalfFloats, bytes_b,
+                          &bfull[st]);
+          }
+        }
       }
       // and so do the copies
-      for (int i = max(0, loaded - 2); i < loaded; ++i)
-        ptx::mbar_wait_bounded(&bfull[i & 1], (i >> 1) & 1u, kWaitCycles);
-      for (int g = max(0, (loaded + 1) / 2 - 2); g < (loaded + 1) / 2; ++g)
+      for (uint32_t h = hc > kStages ? hc - kStages : 0; h < hc; ++h)
+        ptx::mbar_wait_bounded(&bfull[h % kStages], (h / kStages) & 1u, kWaitCycles);
+      for (uint32_t g = gc > 2 ? gc - 2 : 0; g < gc; ++g)
         ptx::mbar_wait_bounded(&ffull[g & 1], (g >> 1) & 1u, kWaitCycles);
     }
     __syncwarp();
-  } else {
-    const int cg = warp >> 2;
-    const float kap = P.kap;
-    const float t2 = fmaf(th[0], th[0], fmaf(th[1], th[1], th[2] * th[2]));
+  } else if (consumer) {
+    const int cg = warp >> 2, row = 32 * (warp & 3) + lane;
     const uint32_t trow = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(8 * cg);
-    for (int g = g0; g < g1; ++g) {
-      const int gi = g - g0, d = gi & 1, left = min(8, P.nS - g * kGroupS - 8 * cg);
-      if (!__all_sync(0xffffffffu, tc_wait(&dfull[d], (gi >> 1) & 1u, abort_flag, err) &&
-                                       tc_wait(&ffull[d], (gi >> 1) & 1u, abort_flag, err)))
-        break;
-      ptx::tc_fence_after();
-      uint32_t vr[8], vi[8];
-      ptx::tmem_ld8_nowait(trow + (uint32_t)(2 * kGroupS * d), vr);
-      ptx::tmem_ld8_nowait(trow + (uint32_t)(2 * kGroupS * d + kGroupS), vi);
-      ptx::tmem_wait8(vr);
-      ptx::tmem_wait8(vi);
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&dfree[d]);
-      const float4 *f = reinterpret_cast<const float4 *>(sframes + (d * kGroupS + 8 * cg) * 12);
-      float gr = 0.f, gim = 0.f;
+    uint32_t gc = 0, it = 0;
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++it) {
+      const ExpandProblem &P = locate(item, w);
+      const float kap = P.kap;
+      const int nS = P.nS;
+      if (!__all_sync(0xffffffffu, tc_wait(&a_ready[it & 1], (it >> 1) & 1u, abort_flag, err))) break;
+      const float *r = srec + (it & 1) * 7 * kBlockT + row;
+      const float th[3] = {r[0], r[kBlockT], r[2 * kBlockT]};
+      const float tl[3] = {r[3 * kBlockT], r[4 * kBlockT], r[5 * kBlockT]};
+      const float t2 = r[6 * kBlockT];
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);  // (re hi, re lo, im hi, im lo)
+      bool ok = true;
+      for (int g = w.g0; g < w.g1; ++g, ++gc) {
+        const uint32_t d = gc & 1, ph2 = (gc >> 1) & 1u;
+        const int left = min(8, nS - g * kGroupS - 8 * cg);
+        ok = __all_sync(0xffffffffu, tc_wait(&dfull[d], ph2, abort_flag, err) &&
+                                         tc_wait(&ffull[d], ph2, abort_flag, err));
+        if (!ok) break;
+        ptx::tc_fence_after();
+        uint32_t vr[8], vi[8], wr[8], wi[8];
+        ptx::tmem_ld8_nowait(trow + 4 * kGroupS * d, vr);
+        ptx::tmem_ld8_nowait(trow + 4 * kGroupS * d + kGroupS, vi);
+        ptx::tmem_ld8_nowait(trow + 4 * kGroupS * d + 2 * kGroupS, wr);
+        ptx::tmem_ld8_nowait(trow + 4 * kGroupS * d + 3 * kGroupS, wi);
+        ptx::tmem_wait8(vr);
+        ptx::tmem_wait8(vi);
+        ptx::tmem_wait8(wr);
+        ptx::tmem_wait8(wi);
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&dfree[d]);
+        const float4 *f = reinterpret_cast<const float4 *>(sframes + (d * kGroupS + 8 * cg) * 12);
+        float gr = 0.f, gim = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (j < left) {
-          const float4 f0 = f[3 * j], f1 = f[3 * j + 1], f2 = f[3 * j + 2];
-          const float ah[3] = {f0.x, f0.y, f0.z}, al[3] = {f1.x, f1.y, f1.z};
-          float s, e, s2, e2, iq, hq;
-          dot3_ff(ah, al, th, tl, s, e);
-          two_sum(s, f1.w, s2, e2);
-          const float tz = fmaf(f2.x, th[0], fmaf(f2.y, th[1], f2.z * th[2]));
-          const float ph = reduce_two_pi_ff(s2, __fadd_rn(__fadd_rn(e, e2), f2.w)) +
-                           curvature(kap, fmaf(-tz, tz, t2), f0.w + tz, iq, hq);
-          const float cr = ptx::cos_approx(ph), sr = ptx::sin_approx(ph);
-          const float re = __uint_as_float(vr[j]), im = __uint_as_float(vi[j]);
-          gr = fmaf(re, cr, fmaf(-im, sr, gr));
-          gim = fmaf(re, sr, fmaf(im, cr, gim));
+        for (int j = 0; j < 8; ++j) {
+          if (j < left) {
+            const float4 f0 = f[3 * j], f1 = f[3 * j + 1], f2 = f[3 * j + 2];
+            const float ah[3] = {f0.x, f0.y, f0.z}, al[3] = {f1.x, f1.y, f1.z};
+            float s, e, s2, e2;
+            dot3_ff(ah, al, th, tl, s, e);
+            two_sum(s, f1.w, s2, e2);
+            const float tz = fmaf(f2.x, th[0], fmaf(f2.y, th[1], f2.z * th[2]));
+            const float ph =
+                reduce_two_pi_with(s2, __fadd_rn(__fadd_rn(e, e2), f2.w),
+                                   curvature(kap, fmaf(-tz, tz, t2), f0.w + tz));
+            const float cr = ptx::cos_approx(ph), sr = ptx::sin_approx(ph);
+            const float re = __uint_as_float(vr[j]) + __uint_as_float(wr[j]);
+            const float im = __uint_as_float(vi[j]) + __uint_as_float(wi[j]);
+            gr = fmaf(re, cr, fmaf(-im, sr, gr));
+            gim = fmaf(re, sr, fmaf(im, cr, gim));
+          }
+        }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&ffree[d]);
+        float h, e;
+        two_sum(sum.x, gr, h, e);
+        sum.x = h;
+        sum.y = __fadd_rn(sum.y, e);
+        two_sum(sum.z, gim, h, e);
+        sum.z = h;
+        sum.w = __fadd_rn(sum.w, e);
+      }
+      if (!ok) break;
+      if (it > 0 &&
+          !__all_sync(0xffffffffu, tc_wait(parts_free, (it - 1) & 1u, abort_flag, err)))
+        break;
+      part[cg * kBlockT + row] = sum;
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(parts_ready);
+    }
+  } else {
+    // ---- builders: thread (row, half): 64 nodes of one target's weights.  After a timeout
+    // they go on (every wait then returns at once): their barrier needs all of them ----
+    // (a warp reaches the 32 TMEM lanes of its index mod 4: rows follow from that)
+    const int bt = tid - 32 * (kTgtConsumers + 2), row = 32 * (warp & 3) + lane, half = bt >> 7;
+    auto bar_builders = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
+    static_assert(32 * kTgtBuilders == 256, "builders' named barrier");
+    uint32_t it = 0;
+    // the four warps of a target add their clusters' sums; results of an item
+    int out_t = -1, out_sp = 0;
+    const ExpandProblem *out_p = nullptr;
+    auto write_out = [&](uint32_t i) {
+      if (half) return;
+      const int order = out_t >= 0 && out_p->ssplit == 1 ? out_p->order_t[out_t] : 0;
+      if (!tc_wait(parts_ready, i & 1u, abort_flag, err)) return;
+      float4 s = part[row];
+#pragma unroll
+      for (int c = 1; c < 4; ++c) {
+        const float4 v = part[c * kBlockT + row];
+        float h, e;
+        two_sum(s.x, v.x, h, e);
+        s.x = h;
+        s.y = __fadd_rn(s.y, __fadd_rn(v.y, e));
+        two_sum(s.z, v.z, h, e);
+        s.z = h;
+        s.w = __fadd_rn(s.w, __fadd_rn(v.w, e));
+      }
+      ptx::mbar_arrive(parts_free);
+      if (out_t >= 0) {
+        const double2 v = make_double2((double)s.x + (double)s.y, (double)s.z + (double)s.w);
+        if (out_p->ssplit == 1)
+          out_p->y[order] = v;
+        else
+          out_p->partial[(size_t)out_sp * out_p->M + out_t] = v;
+      }
+    };
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++it) {
+      const ExpandProblem &P = locate(item, w);
+      const int px = P.px, py = P.py, np = px * py, t = w.m0 + row;
+      float th[3] = {0.f, 0.f, 0.f}, tl[3] = {0.f, 0.f, 0.f};
+      if (t < P.M) cluster_offset(P.geo_t, P.shift_t, t, P.tt_log2, th, tl);
+      const float4 hx = reinterpret_cast<const float4 *>(P.half_t)[P.t0 + w.Tl];
+      // the builders' reads of the last item's factors are behind the barrier below; its
+      // records' buffer was released with the parts of item - 2
+      {
+        // T_0 .. T_{p-1} along one axis, as scalars and as fours (zero past the last)
+        const int p = half ? py : px;
+        const float x = half ? pick(th, P.ay) * hx.w : pick(th, P.ax) * hx.z;
+        float *o = cheb + (half ? px : 0) * kBlockT + row;
+        float4 *q = squad + (half ? 0 : 4) * kBlockT + row;
+        float t0 = 1.f, t1 = x;
+        for (int k = 0; k < p; k += 4) {
+          float v[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            v[j] = k + j < p ? t0 : 0.f;
+            if (k + j < p) o[(k + j) * kBlockT] = t0;
+            const float t2 = fmaf(2.f * x, t1, -t0);
+            t0 = t1;
+            t1 = t2;
+          }
+          q[(k / 4) * kBlockT] = make_float4(v[0], v[1], v[2], v[3]);
         }
       }
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&ffree[d]);
-      float h, e;
-      two_sum(sum.x, gr, h, e);
-      sum.x = h;
-      sum.y = __fadd_rn(sum.y, e);
-      two_sum(sum.z, gim, h, e);
-      sum.z = h;
-      sum.w = __fadd_rn(sum.w, e);
+      if (half == 0) {
+        float *r = srec + (it & 1) * 7 * kBlockT + row;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          r[d * kBlockT] = th[d];
+          r[(3 + d) * kBlockT] = tl[d];
+        }
+        r[6 * kBlockT] = fmaf(th[0], th[0], fmaf(th[1], th[1], th[2] * th[2]));
+      }
+      bar_builders();
+      if (it > 0) tc_wait(a_free, (it - 1) & 1u, abort_flag, err);
+      ptx::tc_fence_after();
+      // two quads (8 columns) at a time: one factor times four; the tensor cores drop the low
+      // 13 bits, so the product itself is the high part and what it loses, rounded, the low
+      const uint32_t acol = tbase + 256 + ((uint32_t)(32 * (warp & 3)) << 16);
+      const int q1 = min(16 * half + 16, (P.n_quads + 1) / 2 * 2);
+      for (int q = 16 * half; q < q1; q += 2) {
+        float hi[8], lo[8];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t c = P.quads[q + j];
+          const bool along_x = c >> 16;
+          const float s = cheb[((along_x ? px : 0) + (int)((c >> 8) & 255)) * kBlockT + row];
+          const float4 f = squad[((along_x ? 4 : 0) + (int)(c & 255)) * kBlockT + row];
+          const float v[4] = {s * f.x, s * f.y, s * f.z, s * f.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            hi[4 * j + e] = v[e];
+            const float r = __fsub_rn(v[e], __uint_as_float(__float_as_uint(v[e]) & 0xffffe000u));
+            lo[4 * j + e] = __uint_as_float(__float_as_uint(r) + 0x1000u);
+          }
+        }
+        ptx::tmem_st8(acol + 4 * q, hi);
+        ptx::tmem_st8(acol + 128 + 4 * q, lo);
+      }
+      ptx::tmem_wait_st();
+      ptx::tc_fence_before();
+      ptx::mbar_arrive(&a_ready[it & 1]);
+      if (it > 0) write_out(it - 1);
+      bar_builders();  // the factors are rewritten next; both halves of the results are out
+      out_t = t < P.M ? t : -1;
+      out_sp = w.sp;
+      out_p = &P;
     }
+    if (it > 0) write_out(it - 1);
   }
-  // ---- the four warps of a target add their clusters' sums ----
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  if (mma_warp) ptx::tmem_dealloc(tbase, 128);
-  float4 *part = reinterpret_cast<float4 *>(cheb);  // [4][128], the Chebyshev factors are done
-  if (consumer) part[(warp >> 2) * kBlockT + 32 * (warp & 3) + lane] = sum;
-  __syncthreads();
-  if (tid < kBlockT && m0 + tid < P.M) {
-    double re = 0.0, im = 0.0;
-    for (int c = 0; c < 4; ++c) {
-      const float4 v = part[c * kBlockT + tid];
-      re += (double)v.x + (double)v.y;
-      im += (double)v.z + (double)v.w;
-    }
-    const int t = m0 + tid;
-    if (P.ssplit == 1)
-      P.y[P.order_t[t]] = make_double2(re, im);
-    else
-      P.partial[(size_t)sp * P.M + t] = make_double2(re, im);
-  }
+  if (mma_warp) ptx::tmem_dealloc(tbase, 512);
 }
 
 }  // namespace
@@ -786,7 +940,7 @@ void expand_blocks(const ExpandProblem &p, int blocks[4]) {
 
 template <bool BATCHED>
 static int launch_all(const ExpandProblem &p, const ExpandProblem *probs, const int *offs,
-                      const int *blocks, int n, int *err, cudaStream_t s) {
+                      const int *blocks, int n, int sms, int *err, cudaStream_t s) {
   HOLO_TRY((kernel_setup<k_expand_moments<BATCHED>>(kMomThreads, (int)MomentsSmem::bytes, nullptr)));
   HOLO_TRY((kernel_setup<k_expand_targets<BATCHED>>(kTgtThreads, (int)TargetsSmem::bytes, nullptr)));
   const int step = BATCHED ? n + 1 : 0;
@@ -794,23 +948,23 @@ static int launch_all(const ExpandProblem &p, const ExpandProblem *probs, const 
   k_expand_moments<BATCHED><<<blocks[1], kMomThreads, MomentsSmem::bytes, s>>>(p, probs, offs + step,
                                                                               n, err);
   k_expand_translate<BATCHED><<<blocks[2], kNodes, 0, s>>>(p, probs, offs + 2 * step, n);
-  k_expand_targets<BATCHED><<<blocks[3], kTgtThreads, TargetsSmem::bytes, s>>>(
-      p, probs, offs + 3 * step, n, err);
+  k_expand_targets<BATCHED><<<std::min(blocks[3], sms), kTgtThreads, TargetsSmem::bytes, s>>>(
+      p, probs, offs + 3 * step, blocks[3], err);
   note_launches(4);
   HOLO_CUDA(cudaGetLastError());
   return HOLO_OK;
 }
 
-int launch_expand(const ExpandProblem &p, int *err, cudaStream_t s) {
+int launch_expand(const ExpandProblem &p, int sms, int *err, cudaStream_t s) {
   int blocks[4];
   expand_blocks(p, blocks);
-  return launch_all<false>(p, nullptr, nullptr, blocks, 1, err, s);
+  return launch_all<false>(p, nullptr, nullptr, blocks, 1, sms, err, s);
 }
 
 int launch_expand_batched(const ExpandProblem *probs_dev, const int *offs_dev, const int *totals,
-                          int n, int *err, cudaStream_t s) {
+                          int n, int sms, int *err, cudaStream_t s) {
   if (n <= 0) return HOLO_OK;
-  return launch_all<true>(ExpandProblem{}, probs_dev, offs_dev, totals, n, err, s);
+  return launch_all<true>(ExpandProblem{}, probs_dev, offs_dev, totals, n, sms, err, s);
 }
 
 }  // namespace holo

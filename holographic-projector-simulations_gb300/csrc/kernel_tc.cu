@@ -109,23 +109,6 @@ __device__ __forceinline__ void split_range_tc(int n, int splits, int s, int *b,
   *e = (int)(((long long)n * (s + 1)) / splits);
 }
 
-// Row r of an operand pair (hi, lo): the 8 features split into TF32 high parts and
-// TF32 remainders, written as four 16-byte stores (features 0-3 and 4-7 of a row
-// are contiguous; eight consecutive rows fill 128 bytes, so a warp's stores are
-// free of bank conflicts).
-__device__ __forceinline__ void store_row_split(float *hi, float *lo, int r, const float *x) {
-  float h[kTcK], l[kTcK];
-#pragma unroll
-  for (int k = 0; k < kTcK; ++k) {
-    h[k] = ptx::to_tf32_int(x[k]);
-    l[k] = ptx::to_tf32_int(__fsub_rn(x[k], h[k]));
-  }
-  *reinterpret_cast<float4 *>(hi + tc_off(r, 0)) = make_float4(h[0], h[1], h[2], h[3]);
-  *reinterpret_cast<float4 *>(hi + tc_off(r, 4)) = make_float4(h[4], h[5], h[6], h[7]);
-  *reinterpret_cast<float4 *>(lo + tc_off(r, 0)) = make_float4(l[0], l[1], l[2], l[3]);
-  *reinterpret_cast<float4 *>(lo + tc_off(r, 4)) = make_float4(l[4], l[5], l[6], l[7]);
-}
-
 // Build flags: kTcScalar -- the MUFU pairs accumulated in scalar FP32 (no packing);
 // kTcHalfUnroll -- the 16-column chunks of a block in a loop of chunk pairs instead
 // of fully unrolled (half the pair-loop code); kTcRcp -- the target row's 1/Qt and

@@ -145,11 +145,42 @@ __device__ __forceinline__ void tc_mma_tf32(uint32_t d_tmem, uint64_t a_desc, ui
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same with A in tensor memory: row m of A in lane m, its K elements in consecutive
+// 32-bit columns (kind::tf32 ignores the low 13 bits of an element).  Run by a whole warp,
+// issued by the lane with `leader`: the operands then stay in uniform registers, where an
+// issue from a one-lane branch moves each of them there first.
+__device__ __forceinline__ void tc_mma_tf32_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                               uint32_t idesc, uint32_t accumulate,
+                                               uint32_t leader) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t setp.ne.b32 p, %4, 0;\n\t setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+// 8 consecutive 32-bit TMEM columns of this thread's lane, written; tmem_wait_st completes them.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
+      "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 // Arrive on `bar` once the tensor-core work issued so far by this thread completes.
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
   asm volatile(
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
           smem_addr(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit(uint64_t *bar, uint32_t leader) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          smem_addr(bar)),
+      "r"(leader)
       : "memory");
 }
 // 16 consecutive 32-bit TMEM columns of this thread's lane (32x32b shape).

@@ -14,6 +14,23 @@ __host__ __device__ __forceinline__ int tc_off(int r, int k) {
   return (r >> 3) * 64 + (k >> 2) * 32 + (r & 7) * 4 + (k & 3);
 }
 
+// Row r of an operand pair (hi, lo): the 8 features split into TF32 high parts and
+// TF32 remainders, written as four 16-byte stores (features 0-3 and 4-7 of a row
+// are contiguous; eight consecutive rows fill 128 bytes, so a warp's stores are
+// free of bank conflicts).
+__device__ __forceinline__ void store_row_split(float *hi, float *lo, int r, const float *x) {
+  float h[kTcK], l[kTcK];
+#pragma unroll
+  for (int k = 0; k < kTcK; ++k) {
+    h[k] = ptx::to_tf32_int(x[k]);
+    l[k] = ptx::to_tf32_int(__fsub_rn(x[k], h[k]));
+  }
+  *reinterpret_cast<float4 *>(hi + tc_off(r, 0)) = make_float4(h[0], h[1], h[2], h[3]);
+  *reinterpret_cast<float4 *>(hi + tc_off(r, 4)) = make_float4(h[4], h[5], h[6], h[7]);
+  *reinterpret_cast<float4 *>(lo + tc_off(r, 0)) = make_float4(l[0], l[1], l[2], l[3]);
+  *reinterpret_cast<float4 *>(lo + tc_off(r, 4)) = make_float4(l[4], l[5], l[6], l[7]);
+}
+
 // Bounded wait that gives up at once when the CTA has aborted; sleep_ns > 0: poll with
 // that much sleep in between.
 __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
