@@ -23,11 +23,12 @@ LIB = os.path.join(HERE, "libholo.so")
 CLI = os.path.join(HERE, "holo")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-LIB_UNITS = ["abi.cu", "batch.cu", "epilogue.cu", "expand_plan.cu", "kernel_expand.cu", "kernel_fp64.cu",
+LIB_UNITS = ["abi.cu", "batch.cu", "epilogue.cu", "expand_plan.cu", "fp64_tables.cpp",
+             "kernel_expand.cu", "kernel_fp64.cu",
              "kernel_split.cu", "kernel_tc.cu", "noalloc.cu", "probe.cu", "tiler.cu"]
 CLI_UNITS = ["cli.cpp", "io.cpp", "gen.cu"]
 HEADERS = ["internal.cuh", "ptx.cuh", "split_frame.cuh", "tc_operand.cuh",
-           "expand_plan.h", "io.h", "gen.h"]
+           "expand_plan.h", "fp64_fixed.cuh", "fp64_tables.h", "io.h", "gen.h"]
 
 
 def nvcc() -> str:

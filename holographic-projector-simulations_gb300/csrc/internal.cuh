@@ -17,6 +17,7 @@
 #include <string>
 #include <vector>
 
+#include "fp64_fixed.cuh"
 #include "holo.h"
 
 namespace holo {
@@ -140,6 +141,8 @@ struct Fp64Problem {
   int n_stiles, n_ttiles, splits;
   int sign;
   double k;
+  const fixed::TrigEntry *trig;   // tables of the fixed-point kernel
+  const fixed::TurnWords *turns;
 };
 
 // batched work item: problem index, target tile, [s_begin, s_end) source tiles, split slot
@@ -355,6 +358,8 @@ struct holo_handle_s {
   int sm_count = 0;
   cudaMemPool_t pool = nullptr;
   int *dev_err = nullptr;  // device error word
+  holo::fixed::TrigEntry *trig = nullptr;   // tables of the FP64 kernel
+  holo::fixed::TurnWords *turns = nullptr;
   std::mutex mu;
   // CUDA-event pairs around each pair-evaluation kernel while profiling is on
   bool profiling = false;

@@ -13,6 +13,8 @@
 // shared memory by TMA bulk copies (double-buffered, mbarrier-tracked); each
 // thread owns R targets in registers; splits of the source range are reduced
 // afterwards in a fixed order (deterministic, no atomics).
+#include <type_traits>
+
 #include "internal.cuh"
 #include "ptx.cuh"
 
@@ -127,6 +129,234 @@ __global__ void __launch_bounds__(THREADS, MINB)
   }
 }
 
+// ---- the same terms on the integer and FP32 pipes (fp64_fixed.cuh) ------------------------
+// The FP64 pipe keeps 6.5 to 10 operations a pair instead of 56: the
+// differences, their squares and sums (shared between a thread's four consecutive targets
+// where they agree in a coordinate, as the rows of a lattice do: `share`), the product
+// distance x k and the sum phase + that.  Bit for bit the other kernel's phases; amplitude /
+// distance, sine and cosine are exact to 2^-55 or better and their products are summed as
+// 64-bit integers, a tile of sources at a time, to 2^-54 of the term of the tile's largest
+// amplitude, whose distance sets the scale.  A pair out of the fixed-point ranges (a zero,
+// infinite or NaN value, a distance four times under the one that set the scale, a phase beyond
+// 2^43) takes the FP64 operations instead.
+// Measured (GB300, 1000 sources -> 512^2 lattice targets): 4.4 ms against 30.0 ms (variant 0); the
+// same with targets jittered, so that no coordinate is shared, 5.2 ms; with registers for 4 or
+// 3 CTAs per SM instead of 5 4.6 ms, 2 targets a thread 4.9 ms, 8 4.6 ms.  Bound by the issue
+// slots (4.99 clocks a pair and SM for some 330 instructions) with the FP64 pipe close behind.
+// One target a thread (variant 7) is for problems that would not fill the GPU: a whole call
+// of 64 -> 64^2 0.10 ms against 0.24, of 256 -> 128^2 0.19 against 0.24, but of 1000 ->
+// 128^2 0.44 against 0.37.
+constexpr int kFixThreads = 128;
+template <int CS>
+struct FixSmem {
+  static constexpr size_t trig = 0;                                        // TrigEntry [1024]
+  static constexpr size_t turns = trig + fixed::kTrigEntries * sizeof(fixed::TrigEntry);
+  static constexpr size_t pos = turns + fixed::kTurnEntries * sizeof(fixed::TurnWords);
+  static constexpr size_t ap = pos + 2 * CS * 3 * sizeof(double);      // double2 [2][CS]
+  static constexpr size_t amp = ap + 2 * CS * sizeof(double2);         // int64 [CS]
+  static constexpr size_t bar = amp + CS * 8;                          // uint64 [3]
+  static constexpr size_t bytes = bar + 3 * 8;
+};
+static_assert(sizeof(fixed::TrigEntry) == 32 && sizeof(fixed::TurnWords) == 16, "table layout");
+
+template <int R, int CS, int MINB>
+__global__ void __launch_bounds__(kFixThreads, MINB)
+    k_fp64_fixed(const Fp64Problem P, int n_items, int *err) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  using L = FixSmem<CS>;
+  constexpr int TT = kFixThreads * R;
+  fixed::TrigEntry *trig = reinterpret_cast<fixed::TrigEntry *>(smem + L::trig);
+  fixed::TurnWords *turns = reinterpret_cast<fixed::TurnWords *>(smem + L::turns);
+  double *raw_pos = reinterpret_cast<double *>(smem + L::pos);
+  double2 *raw_ap = reinterpret_cast<double2 *>(smem + L::ap);
+  long long *samp = reinterpret_cast<long long *>(smem + L::amp);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::bar);
+  static_assert(CS == 16 || CS == 64, "the amplitudes' reduction");
+  __shared__ int s_exp[2], s_count[2];
+  const int tid = threadIdx.x;
+  constexpr uint32_t kTables = fixed::kTrigEntries * sizeof(fixed::TrigEntry),
+                     kTurns = fixed::kTurnEntries * sizeof(fixed::TurnWords);
+  if (tid == 0) {
+    for (int b = 0; b < 3; ++b) ptx::mbar_init(&bar[b], 1);
+    ptx::fence_barrier_init();
+    ptx::mbar_arrive_expect_tx(&bar[2], kTables + kTurns);
+    ptx::bulk_g2s(trig, P.trig, kTables, &bar[2]);
+    ptx::bulk_g2s(turns, P.turns, kTurns, &bar[2]);
+  }
+  __syncthreads();
+  const bool tables = ptx::mbar_wait_bounded(&bar[2], 0u, kWaitCycles);
+  if (!__syncthreads_and(tables)) {
+    if (tid == 0) atomicExch(err, kDevErrTimeout);
+    return;
+  }
+  uint32_t par[2] = {0u, 0u};
+  auto issue = [&](int j, int buf) {
+    ptx::mbar_arrive_expect_tx(&bar[buf], CS * (3 * sizeof(double) + sizeof(double2)));
+    ptx::bulk_g2s(raw_pos + buf * CS * 3, P.pos_s + (size_t)j * CS * 3, CS * 3 * sizeof(double),
+                  &bar[buf]);
+    ptx::bulk_g2s(raw_ap + buf * CS, P.ap_s + (size_t)j * CS, CS * sizeof(double2), &bar[buf]);
+  };
+  const double sk = P.sign > 0 ? P.k : -P.k;  // RN(phi - RN(r k)) = RN(phi + RN(r (-k)))
+
+  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const int tt = item / P.splits, split = item % P.splits;
+    const int sb = (int)(((long long)P.n_stiles * split) / P.splits);
+    const int se = (int)(((long long)P.n_stiles * (split + 1)) / P.splits);
+    const int t0 = tt * TT + tid * R;
+    double vx[R], vy[R], vz[R], re[R], im[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int ti = t0 + r;
+      const bool ok = ti < P.M;
+      vx[r] = ok ? P.pos_t[3 * (size_t)ti] : (r ? vx[0] : 0.0);
+      vy[r] = ok ? P.pos_t[3 * (size_t)ti + 1] : (r ? vy[0] : 0.0);
+      vz[r] = ok ? P.pos_t[3 * (size_t)ti + 2] : (r ? vz[0] : 1.0);
+      re[r] = 0.0;
+      im[r] = 0.0;
+    }
+    // coordinates that every thread's targets share (bit for bit)
+    bool same[3] = {true, true, true};
+#pragma unroll
+    for (int r = 1; r < R; ++r) {
+      same[0] = same[0] && __double_as_longlong(vx[r]) == __double_as_longlong(vx[0]);
+      same[1] = same[1] && __double_as_longlong(vy[r]) == __double_as_longlong(vy[0]);
+      same[2] = same[2] && __double_as_longlong(vz[r]) == __double_as_longlong(vz[0]);
+    }
+    bool share[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) share[d] = __syncthreads_and(same[d]);
+    if (tid == 0 && sb < se) issue(sb, 0);
+
+    for (int j = sb; j < se; ++j) {
+      const int buf = (j - sb) & 1;
+      if (tid == 0 && j + 1 < se) issue(j + 1, buf ^ 1);
+      const bool ok_wait = ptx::mbar_wait_bounded(&bar[buf], par[buf], kWaitCycles);
+      par[buf] ^= 1u;
+      if (!__syncthreads_and(ok_wait)) {
+        if (tid == 0) atomicExch(err, kDevErrTimeout);
+        return;
+      }
+      const double *sp = raw_pos + buf * CS * 3;
+      const double2 *sa = raw_ap + buf * CS;
+      const int count = min(CS, P.N - j * CS);
+      // amplitudes of the tile in units of its largest one's exponent: amp = A 2^(ea - 1084)
+      if (tid < 64) {
+        const long long a = tid < count ? __double_as_longlong(sa[tid].y) : 0;
+        const int e = (int)(a >> 52) & 0x7ff;
+        // 4095 marks what has no place here: a subnormal, an infinity, a NaN
+        const bool bad = e == 0x7ff || (e == 0 && (a & 0x7fffffffffffffffLL) != 0);
+        const int top = __reduce_max_sync(0xffffffffu, (bad ? 4095 : e) << 6 | tid);
+        const uint32_t lit = __ballot_sync(0xffffffffu, e != 0);
+        if ((tid & 31) == 0) {
+          s_exp[tid >> 5] = top;
+          s_count[tid >> 5] = __popc(lit);
+        }
+      }
+      __syncthreads();
+      const int lit = s_count[0] + s_count[1];
+      const int key = max(s_exp[0], s_exp[1]), top = min(key & 63, count - 1);
+      const int ea = lit ? key >> 6 : max(key >> 6, 1023);
+      if (tid < CS) {
+        const long long a = tid < count ? __double_as_longlong(sa[tid].y) : 0;
+        const int e = (int)(a >> 52) & 0x7ff, down = ea - e;
+        const long long m = ((a & 0xfffffffffffffLL) | (1LL << 52)) << 9;
+        const long long f = e == 0 || down > 62 ? 0 : m >> down;
+        samp[tid] = a < 0 ? -f : f;
+      }
+      __syncthreads();
+      // the scale: a quarter of the largest source's distance from the thread's first target
+      int qref;
+      {
+        const double a = vx[0] - sp[3 * top], b = vy[0] - sp[3 * top + 1],
+                     c = vz[0] - sp[3 * top + 2];
+        const int hi = __double2hiint(a * a + b * b + c * c);
+        qref = ((((hi >> 20) & 0x7ff) - 1023) >> 1) - 2;
+      }
+      const int es = ea - 1078 - qref + 1023;  // exponent field of the sums' unit
+      const bool usable = ea > 200 && ea < 2047 && es > 0 && es < 2046;
+      const double unit = usable ? __hiloint2double(es << 20, 0) : 0.0;
+      long long fr[R], fi[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) fr[r] = fi[r] = (lit + 1) >> 1;  // each product rounds down
+      // the sources of this tile; mask: coordinates that the targets of each thread share
+      auto sum_tile = [&](auto mask) {
+        constexpr bool SX = decltype(mask)::value & 1, SY = decltype(mask)::value & 2,
+                       SZ = decltype(mask)::value & 4;
+        for (int s = 0; s < count; ++s) {
+          const double ux = sp[3 * s], uy = sp[3 * s + 1], uz = sp[3 * s + 2];
+          const double phi = sa[s].x;
+          const long long am = samp[s];
+          double xx = 0.0, yy = 0.0, zz = 0.0;
+          if (SX) { const double d = __dsub_rn(vx[0], ux); xx = __dmul_rn(d, d); }
+          if (SY) { const double d = __dsub_rn(vy[0], uy); yy = __dmul_rn(d, d); }
+          if (SZ) { const double d = __dsub_rn(vz[0], uz); zz = __dmul_rn(d, d); }
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            if (!SX) { const double d = __dsub_rn(vx[r], ux); xx = __dmul_rn(d, d); }
+            if (!SY) { const double d = __dsub_rn(vy[r], uy); yy = __dmul_rn(d, d); }
+            if (!SZ) { const double d = __dsub_rn(vz[r], uz); zz = __dmul_rn(d, d); }
+            const double ss = __dadd_rn(__dadd_rn(xx, yy), zz);
+            const uint32_t hi = (uint32_t)__double2hiint(ss);
+            const fixed::Root rt = fixed::root(hi, (uint32_t)__double2loint(ss),
+                                               [](float x) { return ptx::rsqrt_approx(x); });
+            const double dist = __hiloint2double((int)(rt.d >> 32) + ((rt.q + 1022) << 20), (int)rt.d);
+            const double ph = __dadd_rn(phi, __dmul_rn(dist, sk));
+            const uint32_t hp = (uint32_t)__double2hiint(ph);
+            const uint32_t te = ((hp >> 20) & 0x7ffu) - (uint32_t)(1023 + fixed::kTurnLow);
+            const uint32_t down = (uint32_t)(rt.q - qref);
+            const bool fast = usable && hi - (200u << 20) < (1600u << 20) && down <= 40u &&
+                              te < (uint32_t)fixed::kTurnEntries;
+            if (fast) {
+              const uint4 k = *reinterpret_cast<const uint4 *>(&turns[te]);
+              const uint64_t t = fixed::turns(hp, (uint32_t)__double2loint(ph), k.x, k.y, k.z, k.w);
+              const uint32_t index = fixed::trig_index(t);
+              const fixed::TrigEntry &E = trig[index & (fixed::kTrigEntries - 1)];
+              int64_t c, sn;
+              fixed::cos_sin(t, index, E, &c, &sn);
+              const int64_t w = fixed::mulhi64(am, fixed::reciprocal(rt)) >> (down + 2);
+              fr[r] += fixed::mulhi64(w, c);
+              fi[r] += fixed::mulhi64(w, sn);
+            } else {
+              const double d = __dsqrt_rn(ss);
+              const double kr = __dmul_rn(d, P.k);
+              const double p = P.sign > 0 ? __dadd_rn(phi, kr) : __dsub_rn(phi, kr);
+              const double w = __ddiv_rn(sa[s].y, d);
+              double sn, cs;
+              sincos(p, &sn, &cs);
+              re[r] = __dadd_rn(re[r], __dmul_rn(w, cs));
+              im[r] = __dadd_rn(im[r], __dmul_rn(w, sn));
+            }
+          }
+        }
+      };
+      if (R == 1) sum_tile(std::integral_constant<int, 7>{});
+      else if (share[2] && share[0]) sum_tile(std::integral_constant<int, 5>{});
+      else if (share[2] && share[1]) sum_tile(std::integral_constant<int, 6>{});
+      else if (share[2]) sum_tile(std::integral_constant<int, 4>{});
+      else sum_tile(std::integral_constant<int, 0>{});
+      if (usable)
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          re[r] = fma((double)fr[r], unit, re[r]);
+          im[r] = fma((double)fi[r], unit, im[r]);
+        }
+      __syncthreads();  // buffer `buf` is refilled two tiles later, the amplitudes at once
+    }
+
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int ti = t0 + r;
+      if (ti < P.M) {
+        const double2 v = make_double2(re[r], im[r]);
+        if (P.splits == 1)
+          P.y[ti] = v;
+        else
+          P.partial[(size_t)split * P.M + ti] = v;
+      }
+    }
+  }
+}
+
 constexpr Variant kVariants[] = {
     {128, 4, 256},  // 0
     {256, 2, 256},  // 1
@@ -134,6 +364,8 @@ constexpr Variant kVariants[] = {
     {64, 4, 256},   // 3
     {128, 2, 256},  // 4: registers for 8 CTAs per SM
     {128, 1, 256},  // 5: registers for 12 CTAs per SM
+    {kFixThreads, 4, 64},  // 6: the fixed-point kernel
+    {kFixThreads, 1, 16},  // 7: the same, one target per thread, 16 sources a tile
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
@@ -161,6 +393,18 @@ int occupancy_variant(int *out) {
   return kernel_setup<k_fp64<THREADS, R, CS, MINB, false>>(THREADS, (int)L::bytes, out);
 }
 
+template <int R, int CS, int MINB>
+int launch_fixed(const Fp64Problem &p, int grid, bool cst, int *err, cudaStream_t s) {
+  if (cst)  // every term 1: nothing to compute (same tiles, the plain kernel)
+    return launch_variant<kFixThreads, R, CS, 1>(p, grid, true, err, s);
+  const int n_items = p.n_ttiles * p.splits;
+  if (n_items <= 0) return HOLO_OK;
+  HOLO_TRY((kernel_setup<k_fp64_fixed<R, CS, MINB>>(kFixThreads, (int)FixSmem<CS>::bytes, nullptr)));
+  k_fp64_fixed<R, CS, MINB><<<grid, kFixThreads, FixSmem<CS>::bytes, s>>>(p, n_items, err); note_launches(1);
+  HOLO_CUDA(cudaGetLastError());
+  return HOLO_OK;
+}
+
 }  // namespace
 
 int fp64_variant_count() { return kNumVariants; }
@@ -179,12 +423,18 @@ Variant fp64_variant(int i) { return kVariants[i]; }
 
 int launch_fp64(const Fp64Problem &p, int variant, int grid, bool const_phase, int *err,
                 cudaStream_t s) {
+  if (variant == 6) return launch_fixed<4, 64, 5>(p, grid, const_phase, err, s);
+  if (variant == 7) return launch_fixed<1, 16, 5>(p, grid, const_phase, err, s);
 #define CALL(T, R, C, B) launch_variant<T, R, C, B>(p, grid, const_phase, err, s)
   HOLO_FP64_DISPATCH(variant, CALL)
 #undef CALL
 }
 
 int fp64_occupancy(int variant, int *ctas_per_sm) {
+  if (variant == 6)
+    return kernel_setup<k_fp64_fixed<4, 64, 5>>(kFixThreads, (int)FixSmem<64>::bytes, ctas_per_sm);
+  if (variant == 7)
+    return kernel_setup<k_fp64_fixed<1, 16, 5>>(kFixThreads, (int)FixSmem<16>::bytes, ctas_per_sm);
 #define CALL(T, R, C, B) occupancy_variant<T, R, C, B>(ctas_per_sm)
   HOLO_FP64_DISPATCH(variant, CALL)
 #undef CALL
