@@ -27,6 +27,7 @@ BACKWARDS = -1
 FLAG_CONST_PHASE = 0x1
 TILE_HILBERT = 0  # tilings of holo_tile_order / holo_plan_tiling
 TILE_PACKED = 1
+INTENSITY_WORK = 2 + 3 * 512  # values of holo_intensity_loss's workspace
 
 _c = ctypes
 _dp = _c.c_void_p  # device or host pointer
@@ -65,6 +66,8 @@ SIGNATURES = {
     "holo_plan_execute_mc": (_i, [_vp, _i, _d, _dp, _dp, _dp, _c.c_uint64, _i, _i, _vp]),
     "holo_plan_adjoint": (_i, [_vp, _i, _d, _dp, _dp, _dp, _dp, _dp, _vp]),
     "holo_adjoint": (_i, [_vp, _i, _d, _dp, _dp, _dp, _sz, _dp, _sz, _dp, _dp, _dp, _i, _vp]),
+    "holo_intensity_loss": (_i, [_vp, _dp, _dp, _sz, _dp, _dp, _dp, _vp]),
+    "holo_intensity_grad": (_i, [_vp, _dp, _dp, _sz, _dp, _dp, _dp, _vp]),
     "holo_normalize_polar": (_i, [_vp, _dp, _sz, _dp, _dp, _c.POINTER(_d), _vp]),
     "holo_project": (_i, [_vp, _d, _dp, _dp, _dp, _sz, _dp, _sz, _dp, _sz, _dp, _dp, _dp, _dp,
                           _i, _i, _d, _vp]),

@@ -1075,6 +1075,39 @@ int holo_normalize_polar(holo_handle h, const double *y_re_im, size_t M, double 
   return HOLO_OK;
 }
 
+// ---- loss of a phase-only hologram ---------------------------------------------------
+int holo_intensity_loss(holo_handle h, const double *z_re_im, const double *target, size_t M,
+                        double *loss, double *diff, double *work, holo_stream_t stream) {
+  if (!h) return fail(HOLO_ERR_INVALID, "null handle");
+  if (!M || !z_re_im || !target || !loss || !work) return fail(HOLO_ERR_INVALID, "null array");
+  if (((uintptr_t)z_re_im | (uintptr_t)work) & 15)
+    return fail(HOLO_ERR_INVALID, "z and work must be 16-byte aligned");
+  if (M > (1u << 30)) return fail(HOLO_ERR_INVALID, "more than 2^30 targets");
+  DeviceGuard g(h->device);
+  bool dev = false;
+  HOLO_TRY(classify_all({z_re_im, target, loss, diff ? diff : work, work}, &dev));
+  if (!dev) return fail(HOLO_ERR_INVALID, "device pointers only");
+  return launch_intensity_loss((const double2 *)z_re_im, target, (int)M, loss, diff, work,
+                               (cudaStream_t)stream);
+}
+
+int holo_intensity_grad(holo_handle h, const double *z_re_im, const double *diff, size_t M,
+                        const double *work, const double *grad, double *grad_z,
+                        holo_stream_t stream) {
+  if (!h) return fail(HOLO_ERR_INVALID, "null handle");
+  if (!M || !z_re_im || !diff || !work || !grad || !grad_z)
+    return fail(HOLO_ERR_INVALID, "null array");
+  if (((uintptr_t)z_re_im | (uintptr_t)grad_z) & 15)
+    return fail(HOLO_ERR_INVALID, "z and grad_z must be 16-byte aligned");
+  if (M > (1u << 30)) return fail(HOLO_ERR_INVALID, "more than 2^30 targets");
+  DeviceGuard g(h->device);
+  bool dev = false;
+  HOLO_TRY(classify_all({z_re_im, diff, work, grad, grad_z}, &dev));
+  if (!dev) return fail(HOLO_ERR_INVALID, "device pointers only");
+  return launch_intensity_grad((const double2 *)z_re_im, diff, (int)M, work, grad,
+                               (double2 *)grad_z, (cudaStream_t)stream);
+}
+
 // ---- x -> y -> z chain ----------------------------------------------------------------
 static int project_dev(holo_handle h, double lambda, const double *xa, const double *xp,
                        const double *u, size_t N, const double *v, size_t M, const double *w,

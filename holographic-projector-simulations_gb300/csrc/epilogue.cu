@@ -8,7 +8,10 @@
 //                          (cuda/transform.cu:106-139, 376, 402-405)
 //   launch_reference_wave  amplitude-only projector (cuda/transform.cu:379-395)
 //   launch_complex_to_polar / launch_adjoint_epilogue   the adjoint's ends
+//   launch_intensity_loss / launch_intensity_grad       the loss of a phase-only hologram
 #include <float.h>
+
+#include <algorithm>
 
 #include "internal.cuh"
 
@@ -146,6 +149,97 @@ __global__ void __launch_bounds__(256) k_reference_wave(const double2 *__restric
   }
 }
 
+// ---- mean((I / mean I - target)^2), I = |z|^2, and its gradient in z ------------------------
+// Two passes over z (16 bytes a target) with sums per block in a fixed order: every block of the
+// second reads the first's partial sums, so nothing waits for the host.  Latency bound at
+// 256^2 targets, memory at 1024^2.  As separate array operations the loss and its gradient were
+// 31 launches, three of them reductions in one block of 27 us: a gradient step of 256^2 ->
+// 256^2 took 920 us with them and 541 us with these four; of 1024^2 -> 512^2 2320 and 2192 us.
+constexpr int kLossThreads = 256;
+
+__device__ double2 block_sum2(double2 v, double2 *shared) {
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_down_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_down_sync(0xffffffffu, v.y, o);
+  }
+  if ((threadIdx.x & 31) == 0) shared[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double2 t = make_double2(0.0, 0.0);
+  for (int w = 0; w < kLossThreads / 32; ++w) {
+    t.x += shared[w].x;
+    t.y += shared[w].y;
+  }
+  __syncthreads();
+  return t;
+}
+
+__device__ double intensity(double2 z) { return fma(z.x, z.x, z.y * z.y); }
+// I / mean by the mean's reciprocal, where that is a normal number
+__device__ double relative(double inten, double mean, double inv) {
+  return inv > 1e-300 && inv < 1e300 ? inten * inv : inten / mean;
+}
+
+__global__ void __launch_bounds__(kLossThreads) k_loss_mean(const double2 *__restrict__ z, int M,
+                                                            double *__restrict__ partial) {
+  __shared__ double2 shared[kLossThreads / 32];
+  double2 sum = make_double2(0.0, 0.0);
+  for (int i = blockIdx.x * kLossThreads + threadIdx.x; i < M; i += gridDim.x * kLossThreads)
+    sum.x += intensity(z[i]);
+  sum = block_sum2(sum, shared);
+  if (threadIdx.x == 0) partial[blockIdx.x] = sum.x;
+}
+
+__global__ void __launch_bounds__(kLossThreads)
+    k_loss_terms(const double2 *__restrict__ z, const double *__restrict__ target, int M,
+                 const double *__restrict__ partial, double2 *__restrict__ sums,
+                 double *__restrict__ diff, double *__restrict__ stats) {
+  __shared__ double2 shared[kLossThreads / 32];
+  double2 sum = make_double2(0.0, 0.0);
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kLossThreads) sum.x += partial[i];
+  const double mean = block_sum2(sum, shared).x / M, inv = 1.0 / mean;
+  sum = make_double2(0.0, 0.0);
+  for (int i = blockIdx.x * kLossThreads + threadIdx.x; i < M; i += gridDim.x * kLossThreads) {
+    const double n = relative(intensity(z[i]), mean, inv), d = n - target[i];
+    if (diff) diff[i] = d;
+    sum.x = fma(d, d, sum.x);
+    sum.y = fma(d, n, sum.y);
+  }
+  sum = block_sum2(sum, shared);
+  if (threadIdx.x == 0) {
+    sums[blockIdx.x] = sum;
+    if (blockIdx.x == 0) stats[0] = mean;
+  }
+}
+
+__global__ void __launch_bounds__(kLossThreads) k_loss_final(const double2 *__restrict__ sums,
+                                                             int blocks, int M,
+                                                             double *__restrict__ loss,
+                                                             double *__restrict__ stats) {
+  __shared__ double2 shared[kLossThreads / 32];
+  double2 sum = make_double2(0.0, 0.0);
+  for (int i = threadIdx.x; i < blocks; i += kLossThreads) {
+    sum.x += sums[i].x;
+    sum.y += sums[i].y;
+  }
+  sum = block_sum2(sum, shared);
+  if (threadIdx.x == 0) {
+    *loss = sum.x / M;
+    stats[1] = sum.y / M;
+  }
+}
+
+// dL / dI_i = 2 / (M mean) (d_i - mean(d I / mean I)), dI / dz = 2 z
+__global__ void __launch_bounds__(kLossThreads)
+    k_loss_grad(const double2 *__restrict__ z, const double *__restrict__ diff, int M,
+                const double *__restrict__ stats, const double *__restrict__ grad,
+                double2 *__restrict__ out) {
+  const double mean = stats[0], shift = stats[1], scale = 4.0 * *grad / M / mean;
+  for (int i = blockIdx.x * kLossThreads + threadIdx.x; i < M; i += gridDim.x * kLossThreads) {
+    const double g = scale * (diff[i] - shift);
+    out[i] = make_double2(g * z[i].x, g * z[i].y);
+  }
+}
+
 int blocks_for(int n) {
   int g = (n + 255) / 256;
   return g < 1 ? 1 : (g > 8192 ? 8192 : g);
@@ -206,6 +300,28 @@ int launch_adjoint_epilogue(const double2 *h, const double *amp, const double *p
                             double *grad_amp, double *grad_phase, cudaStream_t s) {
   if (N <= 0) return HOLO_OK;
   k_adjoint_epilogue<<<blocks_for(N), 256, 0, s>>>(h, amp, phase, N, grad_amp, grad_phase); note_launches(1);
+  HOLO_CUDA(cudaGetLastError());
+  return HOLO_OK;
+}
+
+int launch_intensity_loss(const double2 *z, const double *target, int M, double *loss, double *diff,
+                          double *work, cudaStream_t s) {
+  static_assert(HOLO_INTENSITY_WORK == 2 + 3 * 512, "two statistics, then the blocks' sums");
+  if (M <= 0) return HOLO_OK;
+  const int nb = std::min((M + 4 * kLossThreads - 1) / (4 * kLossThreads), 512);
+  double2 *sums = reinterpret_cast<double2 *>(work + 2);
+  double *partial = work + 2 + 2 * 512;
+  k_loss_mean<<<nb, kLossThreads, 0, s>>>(z, M, partial); note_launches(1);
+  k_loss_terms<<<nb, kLossThreads, 0, s>>>(z, target, M, partial, sums, diff, work); note_launches(1);
+  k_loss_final<<<1, kLossThreads, 0, s>>>(sums, nb, M, loss, work); note_launches(1);
+  HOLO_CUDA(cudaGetLastError());
+  return HOLO_OK;
+}
+
+int launch_intensity_grad(const double2 *z, const double *diff, int M, const double *work,
+                          const double *grad, double2 *out, cudaStream_t s) {
+  if (M <= 0) return HOLO_OK;
+  k_loss_grad<<<blocks_for(M), kLossThreads, 0, s>>>(z, diff, M, work, grad, out); note_launches(1);
   HOLO_CUDA(cudaGetLastError());
   return HOLO_OK;
 }

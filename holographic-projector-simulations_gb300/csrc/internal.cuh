@@ -344,6 +344,10 @@ int launch_normalize_polar(const double2 *y, int M, const double *max_abs, doubl
                            double *phase, cudaStream_t s);
 int launch_complex_to_polar(const double2 *g, int M, double *amp, double *phase,
                             cudaStream_t s);
+int launch_intensity_loss(const double2 *z, const double *target, int M, double *loss, double *diff,
+                          double *work, cudaStream_t s);
+int launch_intensity_grad(const double2 *z, const double *diff, int M, const double *work,
+                          const double *grad, double2 *out, cudaStream_t s);
 int launch_adjoint_epilogue(const double2 *h, const double *amp, const double *phase, int N,
                             double *grad_amp, double *grad_phase, cudaStream_t s);
 int launch_reference_wave(double2 *y, const double2 *y_ref, int M, const double *max_y,

@@ -12,8 +12,10 @@ from __future__ import annotations
 import math
 
 import torch
+from torch.autograd import forward_ad
 
-from .api import Plan
+from . import _native
+from .api import Plan, _handles, handle
 
 
 class HuygensFunction(torch.autograd.Function):
@@ -55,11 +57,76 @@ def dense_reference(amp: torch.Tensor, phase: torch.Tensor, u: torch.Tensor, v: 
     return torch.stack([(w * torch.cos(th)).sum(1), (w * torch.sin(th)).sum(1)], dim=1)
 
 
-def intensity_loss(z: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
-    """MSE between |z|^2 normalised to unit mean and the target intensity."""
+def _intensity_loss_ops(z: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
     inten = z[:, 0] ** 2 + z[:, 1] ** 2
     inten = inten / inten.mean()
     return torch.mean((inten - target) ** 2)
+
+
+def _plain(*tensors: torch.Tensor) -> bool:
+    """Tensors a kernel may read by their address: no subclass, no transform, mode or tracer
+    at work that has to see each operation, no lazy negation, on 16-byte boundaries."""
+    return (not torch._C._are_functorch_transforms_active()
+            and not torch._C._len_torch_dispatch_stack()
+            and not torch._C._len_torch_function_stack()
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and all(type(t) is torch.Tensor and t.is_cuda and t.dtype is torch.float64
+                    and torch._C._has_storage(t) and t.is_contiguous() and not t.is_neg()
+                    and t.data_ptr() % 16 == 0
+                    and forward_ad.unpack_dual(t).tangent is None for t in tensors))
+
+
+def _native_loss(z, target, with_grad: bool):
+    loss = torch.empty((), dtype=torch.float64, device=z.device)
+    work = torch.empty(_native.INTENSITY_WORK, dtype=torch.float64, device=z.device)
+    diff = torch.empty_like(target) if with_grad else None
+    h = handle(z.device.index)
+    _native.check(h.lib.holo_intensity_loss(
+        h.h, z.data_ptr(), target.data_ptr(), target.numel(), loss.data_ptr(),
+        diff.data_ptr() if with_grad else None, work.data_ptr(),
+        torch.cuda.current_stream(z.device).cuda_stream))
+    return loss, diff, work
+
+
+class _IntensityLoss(torch.autograd.Function):
+    """The loss and its gradient as the library's kernels.  ``I / mean I - target`` is kept
+    instead of the target, which may change before the gradient is taken."""
+
+    @staticmethod
+    def forward(ctx, z, target):
+        loss, diff, work = _native_loss(z, target, True)
+        ctx.save_for_backward(z, diff, work)
+        return loss
+
+    @staticmethod
+    def backward(ctx, grad):
+        z, diff, work = ctx.saved_tensors
+        if torch.is_grad_enabled() or not _plain(z, diff, work, grad):
+            # a gradient that is itself differentiated, or batched: the same in array operations
+            inten = z[:, 0] ** 2 + z[:, 1] ** 2
+            mean = inten.mean()
+            rel = inten / mean
+            d = rel - (rel.detach() - diff)
+            by_inten = (2.0 / diff.numel()) * grad / mean * (d - (d * rel).mean())
+            return (2.0 * by_inten)[:, None] * z, None
+        out = torch.empty_like(z)
+        h = handle(z.device.index)
+        _native.check(h.lib.holo_intensity_grad(
+            h.h, z.data_ptr(), diff.data_ptr(), diff.numel(), work.data_ptr(), grad.data_ptr(),
+            out.data_ptr(), torch.cuda.current_stream(z.device).cuda_stream))
+        return out, None
+
+
+def intensity_loss(z: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
+    """MSE between |z|^2 normalised to unit mean and the target intensity."""
+    if (z.dim() == 2 and z.shape[1] == 2 and target.shape == z.shape[:1] and z.shape[0] > 0
+            and z.shape[0] <= 1 << 30 and z.device == target.device and not target.requires_grad
+            and _plain(z, target)
+            and (z.device.index in _handles or not torch.cuda.is_current_stream_capturing())):
+        if z.requires_grad and torch.is_grad_enabled():
+            return _IntensityLoss.apply(z, target)
+        return _native_loss(z, target, False)[0]
+    return _intensity_loss_ops(z, target)
 
 
 def optimise_phase_hologram(projector_pos: torch.Tensor, target_pos: torch.Tensor,

@@ -170,6 +170,18 @@ int holo_adjoint(holo_handle h, int sign, double lambda,
                  const double *v_xyz, size_t M, const double *grad_y,
                  double *grad_amp, double *grad_phase, int precision, holo_stream_t stream);
 
+/* ---- the loss of a phase-only hologram: mean((I / mean I - target)^2) with
+ * I = |z|^2 of M interleaved (re, im) targets, and its gradient in z (times
+ * the scalar *grad).  Device pointers only, z and grad_z 16-byte aligned; no
+ * synchronisation.  diff (M values, NULL where no gradient follows) and work
+ * (HOLO_INTENSITY_WORK values) carry what the gradient needs. */
+#define HOLO_INTENSITY_WORK (2 + 3 * 512)
+int holo_intensity_loss(holo_handle h, const double *z_re_im, const double *target, size_t M,
+                        double *loss, double *diff, double *work, holo_stream_t stream);
+int holo_intensity_grad(holo_handle h, const double *z_re_im, const double *diff, size_t M,
+                        const double *work, const double *grad, double *grad_z,
+                        holo_stream_t stream);
+
 /* ---- output semantics (normalize_amp + polar, cuda/transform.cu:106-139, 376,
  * 402-405): divide by max |y| unless it is below 1e-6, then write
  * amp = |y|, phase = atan2(im, re).  max_amp_out (host, may be NULL) receives
