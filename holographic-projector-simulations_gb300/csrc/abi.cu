@@ -402,6 +402,15 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
     for (int c : cands)
       if (box_level(split_variant(c).cs) < 0 && !p->odd_tiles)
         HOLO_TRY(alloc_plan(pp, (void **)&p->odd_tiles, (size_t)6 * (N / 256 + 1) * sizeof(double), s));
+    auto bounds_of = [&](const Variant &C, double *mb) -> int {
+      double bound = 0.0, curv = 0.0, lin = 0.0, gemm = 0.0;
+      HOLO_TRY(tile_error_bound(pp, C.cs, C.tt(), &bound, &curv, &lin, &gemm, s));
+      mb[0] = bound;
+      mb[1] = bound + curv;
+      mb[2] = mb[1] + lin;
+      mb[3] = mb[2] + gemm;
+      return HOLO_OK;
+    };
     // the first candidate whose bound holds on the current tiles (else the last);
     // leaves that candidate's tile boxes in tiles_s / tiles_t
     auto choose = [&](size_t *chosen) -> int {
@@ -410,12 +419,7 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
       for (size_t i = 0; i < cands.size(); ++i) {
         const Variant C = split_variant(cands[i]);
         if (C.tt() != shape_tt || C.cs != shape_cs) {
-          double bound = 0.0, curv = 0.0, lin = 0.0, gemm = 0.0;
-          HOLO_TRY(tile_error_bound(pp, C.cs, C.tt(), &bound, &curv, &lin, &gemm, s));
-          mb[0] = bound;
-          mb[1] = bound + curv;
-          mb[2] = mb[1] + lin;
-          mb[3] = mb[2] + gemm;
+          HOLO_TRY(bounds_of(C, mb));
           shape_tt = C.tt();
           shape_cs = C.cs;
         }
@@ -447,6 +451,17 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
         HOLO_TRY(order_both(kTileHilbert, nullptr, nullptr));
         HOLO_TRY(choose(&ci));
       }
+    }
+    // Few tiles of 512 x 1024 leave most SMs idle for a whole tile's time: the same kernel on
+    // source tiles of 256, in four times the CTAs, its sums added afterwards.  A replay of
+    // 1024 -> 64^2 takes 30 us against 44, 8192 -> 64^2 41 against 48, 1024 -> 195^2 39
+    // against 45; at 70000 -> 512 (69 tiles) the two meet (60 and 59 us).
+    const size_t tiles = ((M + 511) / 512) * ((N + 1023) / 1024);
+    if (variant == kTcWide && forced_variant < 0 && h->variant_table[precision][bucket] < 0 &&
+        N > 256 && 2 * tiles <= (size_t)h->sm_count) {
+      variant = kTcNarrow;
+      HOLO_TRY(bounds_of(split_variant(variant), p->model_bounds));
+      p->err_bound = p->model_bounds[split_variant(variant).model];
     }
   }
   const Variant V = precision == HOLO_SPLIT32 ? split_variant(variant) : fp64_variant(variant);

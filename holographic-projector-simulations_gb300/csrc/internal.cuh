@@ -82,6 +82,7 @@ int split_variant_count();
 Variant split_variant(int i);
 // Split variants in the planner's order of preference (fastest first) for N x M.
 std::vector<int> split_preferences(size_t N, size_t M);
+constexpr int kTcWide = 73, kTcNarrow = 76;  // builder-warp kernel, source tiles of 1024 and 256
 
 // Largest tile boxes of a source and a target tiling: per set the bounding box
 // of all tiles (lo, hi), the largest tile half-diagonal h and the largest
