@@ -708,6 +708,13 @@ struct Staged {
 using namespace holo;
 
 // =================================================================================
+template <typename T>
+static int upload(const std::vector<T> &table, T **out) {
+  HOLO_CUDA(cudaMalloc(out, table.size() * sizeof(T)));
+  HOLO_CUDA(cudaMemcpy(*out, table.data(), table.size() * sizeof(T), cudaMemcpyHostToDevice));
+  return HOLO_OK;
+}
+
 extern "C" {
 
 int holo_abi_version(void) { return HOLO_ABI_VERSION; }
@@ -739,12 +746,13 @@ int holo_create(int device, holo_handle *out) {
   HOLO_CUDA(cudaMemset(h->dev_err, 0, sizeof(int)));
   std::vector<fixed::TrigEntry> trig(fixed::kTrigEntries);
   std::vector<fixed::TurnWords> turns(fixed::kTurnEntries);
+  std::vector<fixed::PolarEntry> polar(fixed::kPolarEntries);
   fill_trig(trig.data());
   fill_turns(turns.data());
-  HOLO_CUDA(cudaMalloc(&h->trig, trig.size() * sizeof(trig[0])));
-  HOLO_CUDA(cudaMalloc(&h->turns, turns.size() * sizeof(turns[0])));
-  HOLO_CUDA(cudaMemcpy(h->trig, trig.data(), trig.size() * sizeof(trig[0]), cudaMemcpyHostToDevice));
-  HOLO_CUDA(cudaMemcpy(h->turns, turns.data(), turns.size() * sizeof(turns[0]), cudaMemcpyHostToDevice));
+  fill_polar(polar.data());
+  HOLO_TRY(upload(trig, &h->trig));
+  HOLO_TRY(upload(turns, &h->turns));
+  HOLO_TRY(upload(polar, &h->polar));
   *out = h.release();
   return HOLO_OK;
 }
@@ -757,6 +765,7 @@ int holo_destroy(holo_handle h) {
     if (h->dev_err) cudaFree(h->dev_err);
     if (h->trig) cudaFree(h->trig);
     if (h->turns) cudaFree(h->turns);
+    if (h->polar) cudaFree(h->polar);
     if (h->pool) cudaMemPoolDestroy(h->pool);
   }
   delete h;
@@ -994,10 +1003,10 @@ static int adjoint_impl(holo_plan_s *p, int sign, double lambda, const double *a
   double *g_phase = tmp.get<double>(std::max(p->M, 1));
   double2 *H = tmp.get<double2>(p->N);
   if (!g_amp || !g_phase || !H) return fail(HOLO_ERR_ALLOC, "adjoint scratch");
-  HOLO_TRY(launch_complex_to_polar((const double2 *)grad_y, p->M, g_amp, g_phase, s));
+  HOLO_TRY(launch_complex_to_polar((const double2 *)grad_y, p->M, p->h->polar, g_amp, g_phase, s));
   // H_n = sum_m G_m e^{-i s k r_nm} / r_nm: the transform with roles swapped, sign -s
   HOLO_TRY(plan_execute_impl(p->transposed, -sign, lambda, g_amp, g_phase, H, 0, s));
-  HOLO_TRY(launch_adjoint_epilogue(H, amp, phase, p->N, grad_amp, grad_phase, s));
+  HOLO_TRY(launch_adjoint_epilogue(H, amp, phase, p->N, p->h->trig, p->h->turns, grad_amp, grad_phase, s));
   return HOLO_OK;
 }
 
@@ -1049,7 +1058,7 @@ static int normalize_polar_dev(holo_handle h, const double2 *y, size_t M, double
   double *partials = tmp.get<double>(1024);
   if (!partials) return fail(HOLO_ERR_ALLOC, "normalize scratch");
   HOLO_TRY(launch_max_abs(y, (int)M, partials, 1024, max_dev, s));
-  HOLO_TRY(launch_normalize_polar(y, (int)M, max_dev, amp, phase, s));
+  HOLO_TRY(launch_normalize_polar(y, (int)M, max_dev, h->polar, amp, phase, s));
   return HOLO_OK;
 }
 

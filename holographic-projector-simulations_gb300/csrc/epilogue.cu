@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "ptx.cuh"
 
 namespace holo {
 namespace {
@@ -55,12 +56,42 @@ __global__ void __launch_bounds__(256) k_reduce_batched(const SplitProblem *__re
   }
 }
 
+__device__ __forceinline__ bool fast_polar(double x, double y, const fixed::PolarEntry *table,
+                                           double *modulus, double *angle) {
+  return fixed::polar(x, y, table, [](float v, float u) { return atan2f(v, u); },
+                      [](float v) { return ptx::rcp_approx(v); },
+                      [](float v) { return ptx::rsqrt_approx(v); }, modulus, angle);
+}
+
+// The largest modulus.  Bound by the FP64 pipe: the squares' sum (2 operations instead of
+// hypot's ~35) of every value first, then hypot only of those within 2^-40 of the block's largest
+// sum, which the largest hypot is among; a block whose sums leave the safe range takes hypot
+// for all.  512 values a block, not 2048: 512^2 values take 12 us.  With the kernel below, a
+// normalisation of 1024^2 values took 249 us as a call before both, 142 us now.
+constexpr int kMaxPerBlock = 512;
 __global__ void __launch_bounds__(256) k_max_abs_partial(const double2 *__restrict__ y, int M,
                                                          double *__restrict__ partial) {
   __shared__ double s[256];
+  const int step = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+  double most = 0.0;
+  bool odd = false;
+  for (int i = first; i < M; i += step) {
+    const double q = fma(y[i].x, y[i].x, y[i].y * y[i].y);
+    odd = odd || !(q < 1e300);
+    most = q > most ? q : most;
+  }
+  s[threadIdx.x] = most;
+  odd = __syncthreads_or(odd);
+  for (int w = 128; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) s[threadIdx.x] = fmax(s[threadIdx.x], s[threadIdx.x + w]);
+    __syncthreads();
+  }
+  const double limit = odd || s[0] < 1e-280 ? -1.0 : s[0] * (1.0 - 0x1p-40);
+  __syncthreads();
   double m = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x)
-    m = fmax(m, hypot(y[i].x, y[i].y));
+  if (!(most < limit))  // none of this thread's values otherwise
+    for (int i = first; i < M; i += step)
+      if (!(fma(y[i].x, y[i].x, y[i].y * y[i].y) < limit)) m = fmax(m, hypot(y[i].x, y[i].y));
   s[threadIdx.x] = m;
   __syncthreads();
   for (int w = 128; w > 0; w >>= 1) {
@@ -84,40 +115,81 @@ __global__ void __launch_bounds__(256) k_max_final(const double *__restrict__ pa
   if (threadIdx.x == 0) *out = s[0];
 }
 
+// Bound by the FP64 pipe (27 operations a value, fixed::polar, instead of ~130 of two quotients,
+// hypot and atan2): 512^2 values take 21 us.  modulus / max by the
+// reciprocal and one correction, as exact as the quotient.
 __global__ void __launch_bounds__(256) k_normalize_polar(const double2 *__restrict__ y, int M,
                                                          const double *__restrict__ max_abs,
+                                                         const fixed::PolarEntry *__restrict__ table,
                                                          double *__restrict__ amp,
                                                          double *__restrict__ phase) {
+  __shared__ double inverse;
   const double mx = *max_abs;
   const bool scale = !(mx < 1e-6);  // below 1e-6 the reference leaves y unnormalised
+  const double div = scale ? mx : 1.0;
+  if (threadIdx.x == 0) inverse = 1.0 / div;
+  __syncthreads();
+  const double inv = inverse;
+  const bool fast = div < 1e100;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
-    double re = y[i].x, im = y[i].y;
-    if (scale) {
-      re = __ddiv_rn(re, mx);
-      im = __ddiv_rn(im, mx);
+    double re = y[i].x, im = y[i].y, m, a;
+    if (fast && fast_polar(re, im, table, &m, &a)) {
+      const double q = m * inv;
+      m = fma(fma(-q, div, m), inv, q);
+    } else {
+      if (scale) {
+        re = __ddiv_rn(re, mx);
+        im = __ddiv_rn(im, mx);
+      }
+      m = hypot(re, im);
+      a = atan2(im, re);
     }
-    amp[i] = hypot(re, im);
-    phase[i] = atan2(im, re);
+    amp[i] = m;
+    phase[i] = a;
   }
 }
 
 __global__ void __launch_bounds__(256) k_complex_to_polar(const double2 *__restrict__ g, int M,
+                                                          const fixed::PolarEntry *__restrict__ table,
                                                           double *__restrict__ amp,
                                                           double *__restrict__ phase) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
-    amp[i] = hypot(g[i].x, g[i].y);
-    phase[i] = atan2(g[i].y, g[i].x);
+    double m, a;
+    if (!fast_polar(g[i].x, g[i].y, table, &m, &a)) {
+      m = hypot(g[i].x, g[i].y);
+      a = atan2(g[i].y, g[i].x);
+    }
+    amp[i] = m;
+    phase[i] = a;
   }
 }
 
+// Bound by the FP64 pipe: sine and cosine of the phase as fixed-point numbers (fp64_fixed.cuh), 9
+// operations with the products instead of ~60: 1024^2 sources take 23 us.  With the polar form
+// of the gradient it took a step of 1024^2 -> 512^2 from 2192 to 2141 us.
 __global__ void __launch_bounds__(256) k_adjoint_epilogue(const double2 *__restrict__ h,
                                                           const double *__restrict__ amp,
                                                           const double *__restrict__ phase,
-                                                          int N, double *__restrict__ grad_amp,
+                                                          int N, const fixed::TrigEntry *__restrict__ trig,
+                                                          const fixed::TurnWords *__restrict__ words,
+                                                          double *__restrict__ grad_amp,
                                                           double *__restrict__ grad_phase) {
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
     double sp, cp;
-    sincos(phase[n], &sp, &cp);
+    const double ph = phase[n];
+    const uint32_t hi = (uint32_t)__double2hiint(ph);
+    const uint32_t e = ((hi >> 20) & 0x7ffu) - (uint32_t)(1023 + fixed::kTurnLow);
+    if (e < (uint32_t)fixed::kTurnEntries) {
+      const uint4 k = *reinterpret_cast<const uint4 *>(&words[e]);
+      const uint64_t t = fixed::turns(hi, (uint32_t)__double2loint(ph), k.x, k.y, k.z, k.w);
+      const uint32_t index = fixed::trig_index(t);
+      int64_t c, s;
+      fixed::cos_sin(t, index, trig[index & (fixed::kTrigEntries - 1)], &c, &s);
+      cp = (double)c * 0x1p-62;
+      sp = (double)s * 0x1p-62;
+    } else {
+      sincos(ph, &sp, &cp);
+    }
     // w = e^{i phi} conj(H)
     const double wr = cp * h[n].x + sp * h[n].y;
     const double wi = sp * h[n].x - cp * h[n].y;
@@ -272,7 +344,7 @@ int launch_reduce_batched(const SplitProblem *probs_dev, const int *prob_offsets
 
 int launch_max_abs(const double2 *y, int M, double *partials, int n_partials, double *max_out,
                    cudaStream_t s) {
-  int nb = (M + 2047) / 2048;
+  int nb = (M + kMaxPerBlock - 1) / kMaxPerBlock;
   nb = nb < 1 ? 1 : (nb > n_partials ? n_partials : nb);
   k_max_abs_partial<<<nb, 256, 0, s>>>(y, M, partials); note_launches(1);
   k_max_final<<<1, 256, 0, s>>>(partials, nb, max_out); note_launches(1);
@@ -280,26 +352,28 @@ int launch_max_abs(const double2 *y, int M, double *partials, int n_partials, do
   return HOLO_OK;
 }
 
-int launch_normalize_polar(const double2 *y, int M, const double *max_abs, double *amp,
-                           double *phase, cudaStream_t s) {
+int launch_normalize_polar(const double2 *y, int M, const double *max_abs,
+                           const fixed::PolarEntry *table, double *amp, double *phase,
+                           cudaStream_t s) {
   if (M <= 0) return HOLO_OK;
-  k_normalize_polar<<<blocks_for(M), 256, 0, s>>>(y, M, max_abs, amp, phase); note_launches(1);
+  k_normalize_polar<<<blocks_for(M), 256, 0, s>>>(y, M, max_abs, table, amp, phase); note_launches(1);
   HOLO_CUDA(cudaGetLastError());
   return HOLO_OK;
 }
 
-int launch_complex_to_polar(const double2 *g, int M, double *amp, double *phase,
-                            cudaStream_t s) {
+int launch_complex_to_polar(const double2 *g, int M, const fixed::PolarEntry *table, double *amp,
+                            double *phase, cudaStream_t s) {
   if (M <= 0) return HOLO_OK;
-  k_complex_to_polar<<<blocks_for(M), 256, 0, s>>>(g, M, amp, phase); note_launches(1);
+  k_complex_to_polar<<<blocks_for(M), 256, 0, s>>>(g, M, table, amp, phase); note_launches(1);
   HOLO_CUDA(cudaGetLastError());
   return HOLO_OK;
 }
 
 int launch_adjoint_epilogue(const double2 *h, const double *amp, const double *phase, int N,
+                            const fixed::TrigEntry *trig, const fixed::TurnWords *words,
                             double *grad_amp, double *grad_phase, cudaStream_t s) {
   if (N <= 0) return HOLO_OK;
-  k_adjoint_epilogue<<<blocks_for(N), 256, 0, s>>>(h, amp, phase, N, grad_amp, grad_phase); note_launches(1);
+  k_adjoint_epilogue<<<blocks_for(N), 256, 0, s>>>(h, amp, phase, N, trig, words, grad_amp, grad_phase); note_launches(1);
   HOLO_CUDA(cudaGetLastError());
   return HOLO_OK;
 }

@@ -212,5 +212,72 @@ HOLO_HD int64_t reciprocal(const Root &r) {
   return (y << 10) + round_int(fmul((float)(int)(res >> 32), fmul(r.y0, 0x1p-10f)));
 }
 
+// One of 1025 angles a = 2 pi i / 1024, i = -512 .. 512: cosine, sine and angle as a double and
+// what that leaves.
+struct PolarEntry {
+  double c, s, a;
+  float cl, sl, al, none[3];
+};
+constexpr int kPolarHalf = 512, kPolarEntries = 2 * kPolarHalf + 1;
+
+HOLO_HD uint64_t double_bits(double x) {
+#ifdef __CUDA_ARCH__
+  return (uint64_t)__double_as_longlong(x);
+#else
+  uint64_t b;
+  memcpy(&b, &x, 8);
+  return b;
+#endif
+}
+HOLO_HD double as_double(uint64_t b) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)b);
+#else
+  double x;
+  memcpy(&x, &b, 8);
+  return x;
+#endif
+}
+
+// x of exponent field e below or equal to `top`, divided by 2^(top - 1023), cut to FP32.
+HOLO_HD float cut_float(uint64_t bits, int e, int top) {
+  const uint32_t sign = (uint32_t)(bits >> 32) & 0x80000000u;
+  const uint32_t mant = (uint32_t)(bits >> 29) & 0x7fffffu;
+  return as_float(top - e > 100 ? sign : sign | (uint32_t)(e - top + 127) << 23 | mant);
+}
+
+// Modulus and angle of x + i y: a table angle near the FP32 estimate, the point turned back by
+// it (the cancelling component to 2^-60), the small angle left by its series; the modulus as the
+// rounded root of the rounded sum of squares.  24 FP64 operations instead of the ~90 of a hypot
+// and an atan2.
+// False, and nothing written, for what is not well inside the exponent range (zeros, infinities,
+// NaN, components more than 2^500 apart).  angle_of(y, x): atan2 to 2^-16; inverse_of: 1 / x to 2^-20; y0_of: as in root().
+template <typename A, typename R, typename Q>
+HOLO_HD bool polar(double x, double y, const PolarEntry *table, A angle_of, R inverse_of, Q y0_of,
+                   double *modulus, double *angle) {
+  const uint64_t bx = double_bits(x), by = double_bits(y);
+  const int ex = (int)(bx >> 52) & 0x7ff, ey = (int)(by >> 52) & 0x7ff;
+  const int top = ex > ey ? ex : ey, low = ex > ey ? ey : ex;
+  if (top <= 500 || top >= 1500 || low + 500 < top) return false;
+  const uint64_t shift = (uint64_t)(int64_t)(top - 1023) << 52;
+  const double xn = as_double(bx - shift), yn = as_double(by - shift);
+  const float fx = cut_float(bx, ex, top), fy = cut_float(by, ey, top);
+  const int index = round_int(fmul(angle_of(fy, fx), (float)(kPolarHalf / 3.14159265358979)));
+  const PolarEntry &E = table[index + kPolarHalf];
+  const double p = xn * E.s, pe = fma(xn, E.s, -p);
+  const double across = (fma(yn, E.c, -p) - pe) + (double)fmaf(fy, E.cl, -fmul(fx, E.sl));
+  const double along = fma(xn, E.c, yn * E.s);
+  double inv = (double)inverse_of((float)along);
+  inv = fma(fma(-along, inv, 1.0), inv, inv);
+  const double t0 = across * inv, t = fma(fma(-along, t0, across), inv, t0);  // |t| < 2^-8
+  const double t2 = t * t, series = fma(t * t2, fma(t2, 0.2, -1.0 / 3.0), t);
+  *angle = E.a + (series + (double)E.al);
+  const double big = ex > ey ? xn : yn, small = ex > ey ? yn : xn;
+  const uint64_t sum = double_bits(fma(big, big, small * small));
+  const Root r = root((uint32_t)(sum >> 32), (uint32_t)sum, y0_of);
+  *modulus = as_double(r.d + ((uint64_t)(uint32_t)(r.q + top - 1) << 52));
+  return true;
+}
+
 }  // namespace fixed
 }  // namespace holo

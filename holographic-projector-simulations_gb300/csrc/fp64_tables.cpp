@@ -5,20 +5,28 @@
 
 namespace holo {
 
+static const long double kTwoPi = 6.283185307179586476925286766559005768394L;
+
 // cos and sin of 2 pi i / 1024 from the first octant (long double has 64 or 113 bits).
-void fill_trig(fixed::TrigEntry *out) {
+static void circle(int i, long double *cosine, long double *sine) {
   constexpr int n = fixed::kTrigEntries;
-  const long double two_pi = 6.283185307179586476925286766559005768394L;
-  for (int i = 0; i < n; ++i) {
-    const int quadrant = i / (n / 4), j = i % (n / 4);
-    const bool upper = j > n / 8;  // the angle's complement in the quadrant
-    const long double a = two_pi * (upper ? n / 4 - j : j) / n;
-    long double c = upper ? sinl(a) : cosl(a), s = upper ? cosl(a) : sinl(a);
-    for (int q = 0; q < quadrant; ++q) {
-      const long double t = c;
-      c = -s;
-      s = t;
-    }
+  const int quadrant = i / (n / 4), j = i % (n / 4);
+  const bool upper = j > n / 8;  // the angle's complement in the quadrant
+  const long double a = kTwoPi * (upper ? n / 4 - j : j) / n;
+  long double c = upper ? sinl(a) : cosl(a), s = upper ? cosl(a) : sinl(a);
+  for (int q = 0; q < quadrant; ++q) {
+    const long double t = c;
+    c = -s;
+    s = t;
+  }
+  *cosine = c;
+  *sine = s;
+}
+
+void fill_trig(fixed::TrigEntry *out) {
+  for (int i = 0; i < fixed::kTrigEntries; ++i) {
+    long double c, s;
+    circle(i, &c, &s);
     fixed::TrigEntry &e = out[i];
     e.c = (int64_t)llroundl(c * 0x1p62L);
     e.s = (int64_t)llroundl(s * 0x1p62L);
@@ -26,6 +34,24 @@ void fill_trig(fixed::TrigEntry *out) {
     e.cl = (float)(c - (long double)e.ch);
     e.sh = (float)s;
     e.sl = (float)(s - (long double)e.sh);
+  }
+}
+
+void fill_polar(fixed::PolarEntry *out) {
+  constexpr int n = fixed::kTrigEntries;
+  static_assert(n == 2 * fixed::kPolarHalf, "the same angles");
+  for (int i = -fixed::kPolarHalf; i <= fixed::kPolarHalf; ++i) {
+    long double c, s;
+    circle((i + n) % n, &c, &s);
+    const long double a = kTwoPi * i / n;
+    fixed::PolarEntry &e = out[i + fixed::kPolarHalf];
+    e = {};
+    e.c = (double)c;
+    e.s = (double)s;
+    e.a = (double)a;
+    e.cl = (float)(c - (long double)e.c);
+    e.sl = (float)(s - (long double)e.s);
+    e.al = (float)(a - (long double)e.a);
   }
 }
 

@@ -6,4 +6,5 @@
 namespace holo {
 void fill_trig(fixed::TrigEntry *out);    // [fixed::kTrigEntries]
 void fill_turns(fixed::TurnWords *out);   // [fixed::kTurnEntries]
+void fill_polar(fixed::PolarEntry *out);  // [fixed::kPolarEntries]
 }  // namespace holo

@@ -341,15 +341,18 @@ int launch_reduce_batched(const SplitProblem *probs_dev, const int *prob_offsets
                           int total_targets, cudaStream_t s);
 int launch_max_abs(const double2 *y, int M, double *partials, int n_partials, double *max_out,
                    cudaStream_t s);
-int launch_normalize_polar(const double2 *y, int M, const double *max_abs, double *amp,
+int launch_normalize_polar(const double2 *y, int M, const double *max_abs,
+                           const fixed::PolarEntry *table, double *amp,
                            double *phase, cudaStream_t s);
-int launch_complex_to_polar(const double2 *g, int M, double *amp, double *phase,
+int launch_complex_to_polar(const double2 *g, int M, const fixed::PolarEntry *table, double *amp,
+                            double *phase,
                             cudaStream_t s);
 int launch_intensity_loss(const double2 *z, const double *target, int M, double *loss, double *diff,
                           double *work, cudaStream_t s);
 int launch_intensity_grad(const double2 *z, const double *diff, int M, const double *work,
                           const double *grad, double2 *out, cudaStream_t s);
 int launch_adjoint_epilogue(const double2 *h, const double *amp, const double *phase, int N,
+                            const fixed::TrigEntry *trig, const fixed::TurnWords *words,
                             double *grad_amp, double *grad_phase, cudaStream_t s);
 int launch_reference_wave(double2 *y, const double2 *y_ref, int M, const double *max_y,
                           const double *max_ref, double *amp_out, double *phase_out,
@@ -365,6 +368,7 @@ struct holo_handle_s {
   int *dev_err = nullptr;  // device error word
   holo::fixed::TrigEntry *trig = nullptr;   // tables of the FP64 kernel
   holo::fixed::TurnWords *turns = nullptr;
+  holo::fixed::PolarEntry *polar = nullptr;  // and of the conversions to polar form
   std::mutex mu;
   // CUDA-event pairs around each pair-evaluation kernel while profiling is on
   bool profiling = false;
