@@ -474,8 +474,9 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
     // chosen variant, whose boxes the last bound evaluation left in tiles_s/t)
     HOLO_TRY(alloc_plan(p.get(), (void **)&p->geo_s, (size_t)6 * p->n_pad * sizeof(float), s));
     HOLO_TRY(alloc_plan(p.get(), (void **)&p->geo_t, (size_t)6 * std::max<size_t>(M, 1) * sizeof(float), s));
-    HOLO_TRY(launch_rel_hilo(p->pos_s, (int)N, p->n_pad, p->tiles_s, V.cs, p->geo_s, s));
-    HOLO_TRY(launch_rel_hilo(p->pos_t, (int)M, (int)M, p->tiles_t, V.tt(), p->geo_t, s));
+    const RelSet rel[2] = {{p->pos_s, (int)N, p->n_pad, p->tiles_s, V.cs, p->geo_s},
+                           {p->pos_t, (int)M, (int)M, p->tiles_t, V.tt(), p->geo_t}};
+    HOLO_TRY(launch_rel_hilo(rel, 2, s));
   } else {
     HOLO_TRY(alloc_plan(p.get(), (void **)&p->pos_s, (size_t)3 * p->n_pad * sizeof(double), s));
     HOLO_TRY(alloc_plan(p.get(), (void **)&p->pos_t, (size_t)3 * std::max<size_t>(M, 1) * sizeof(double), s));
@@ -635,7 +636,8 @@ static int plan_execute_mc_impl(holo_plan_s *p, int sign, double lambda, const d
     if (!ts || !tt || !gt) return fail(HOLO_ERR_ALLOC, "execute scratch");
     HOLO_TRY(launch_tile_bbox(p->pos_s, p->N, V.cs, ts, s));
     HOLO_TRY(launch_tile_bbox(p->pos_t, p->M, V.tt(), tt, s));
-    HOLO_TRY(launch_rel_hilo(p->pos_t, p->M, p->M, tt, V.tt(), gt, s));
+    const RelSet rel = {p->pos_t, p->M, p->M, tt, V.tt(), gt};
+    HOLO_TRY(launch_rel_hilo(&rel, 1, s));
     tiles_s = ts;
     tiles_t = tt;
     geo_t = gt;

@@ -209,8 +209,18 @@ int launch_iota(int32_t *order, int n, cudaStream_t s);
 // Load the kernels of the Hilbert tiling, the tile boxes and the gathers (CUDA maps a
 // kernel's code on its first use; callers that must not allocate later call this first).
 int tiler_preload_hilbert();
-int launch_rel_hilo(const double *pos_sorted, int n, int n_out, const double *tiles, int tile,
-                    float *out, cudaStream_t s);
+// Offsets of n points (zeros up to n_out) from their tiles' centres; up to two sets a launch.
+struct RelSet {
+  const double *pos;
+  int n, n_out;
+  const double *tiles;
+  int tile;
+  float *out;
+};
+struct RelSets {
+  RelSet s[2];
+};
+int launch_rel_hilo(const RelSet *set, int count, cudaStream_t s);
 int launch_gather_apf(const double *amp, const double *phase, const int32_t *order, int n,
                       int n_pad, float2 *out, cudaStream_t s);
 // The gather of many problems in one launch; first: their first blocks of 1024 records.

@@ -275,8 +275,9 @@ int transform_noalloc(int device, int sign, double lambda, const double *amp,
   }
   const Variant V = split_variant(variant);
   // the last bound evaluation left this variant's tile boxes in tiles_s / tiles_t
-  HOLO_TRY(launch_rel_hilo(pos_s, (int)N, n_pad, tiles_s, V.cs, geo_s, s));
-  HOLO_TRY(launch_rel_hilo(pos_t, (int)M, (int)M, tiles_t, V.tt(), geo_t, s));
+  const RelSet rel[2] = {{pos_s, (int)N, n_pad, tiles_s, V.cs, geo_s},
+                         {pos_t, (int)M, (int)M, tiles_t, V.tt(), geo_t}};
+  HOLO_TRY(launch_rel_hilo(rel, 2, s));
 
   // ---- splits: as many as the occupancy wants and the array holds ----
   int sm = 0, occ = 0;
