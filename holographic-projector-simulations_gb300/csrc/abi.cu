@@ -345,6 +345,24 @@ static int plan_grid(holo_plan_s *p) {
   return HOLO_OK;
 }
 
+// Pairs per clock and SM of a pair kernel: 10.4 on the tensor-core builds (512^2 -> 1024^2 in 90.8
+// ms; 9.5 on 65536 -> 64^2; 94.6 and 99.0 ms on source tiles of 512 and 256), on the CUDA cores
+// 9 with two MUFU operations a pair and 5.5 with three.
+static double pair_rate(const Variant &V) {
+  if (V.tc) return V.cs >= 768 ? 10.0 : V.cs == 512 ? 9.6 : 9.2;
+  return V.model == 2 ? 9.0 : 5.5;
+}
+
+// Time of the plan's pair kernel: the waves of its work items at that rate.
+static double pair_seconds(const holo_plan_s *p) {
+  const Variant V = split_variant(p->variant);
+  const double items = (double)p->n_ttiles * p->splits, per_item = ceil((double)p->n_stiles / p->splits);
+  const double waves = ceil(items / std::max(1, p->grid));
+  const double clocks = waves * per_item * V.cs * V.tt() / pair_rate(V) *
+                        std::max(1.0, (double)p->grid / p->h->sm_count);
+  return clocks / 1.9e9;
+}
+
 int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, size_t M,
                      int precision, int forced_variant, cudaStream_t s, holo_plan_s **out,
                      const int32_t *known_order_s, const int32_t *known_order_t,
@@ -437,13 +455,20 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
     size_t ci = 0;
     HOLO_TRY(order_both(kTileHilbert, known_order_s, known_order_t));
     HOLO_TRY(choose(&ci));
-    bool expands = false;
+    // A call that uses its plan once keeps the Hilbert tiles where they go by expansions, or
+    // where the faster variant would save less than packing takes (0.65 ms: 30000 -> 3000
+    // takes 0.15 ms in all without it)
+    constexpr double kPackSeconds = 0.65e-3;
+    bool stay = false;
     if (ci > 0 && forced_variant < 0 && k_once > 0.0) {
       p->variant = variant;
       HOLO_TRY(plan_grid(pp));
-      expands = plan_expansion(pp, k_once).use;
+      const double saving = pair_seconds(pp) * (1.0 - pair_rate(split_variant(variant)) /
+                                                          pair_rate(split_variant(cands[0])));
+      stay = plan_expansion(pp, k_once).use ||
+             (p->err_bound <= kSplitBoundMetres && saving < kPackSeconds);
     }
-    if (ci > 0 && forced_variant < 0 && !expands) {
+    if (ci > 0 && forced_variant < 0 && !stay) {
       size_t cp = 0;
       HOLO_TRY(order_both(kTilePacked, nullptr, nullptr));
       HOLO_TRY(choose(&cp));
@@ -501,19 +526,14 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
 }
 
 // Whether, and on which clusters, a transform of this plan at wave number k runs by cluster
-// expansions: where they take less time than the plan's pair kernel (~20 pairs per clock
-// and SM on the tensor-core builds, ~16 on the CUDA cores, over the waves of its work items).
+// expansions: where they take less time than the plan's pair kernel.
 ExpandChoice plan_expansion(holo_plan_s *p, double k, double launches) {
   if (p->precision != HOLO_SPLIT32 || p->pair_kernel_only || p->N == 0 || p->M == 0) return {};
   const Variant V = split_variant(p->variant);
   if (box_level(V.cs) < 0) return {};  // its tiles do not nest in the clusters
   if (p->expand_k != k) {
-    const double items = (double)p->n_ttiles * p->splits, per_item = ceil((double)p->n_stiles / p->splits);
-    const double waves = ceil(items / std::max(1, p->grid));
-    const double clocks = waves * per_item * V.cs * V.tt() / (V.tc ? 20.0 : 16.0) *
-                          std::max(1.0, (double)p->grid / p->h->sm_count);
     p->expand = expand_choose(p->stats_s, p->stats_t, p->N, p->M, box_level(V.cs), box_level(V.tt()),
-                              k, clocks / 1.9e9, launches, p->h->sm_count);
+                              k, pair_seconds(p), launches, p->h->sm_count);
     p->expand_k = k;
   }
   return p->expand;
