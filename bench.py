@@ -9,9 +9,12 @@ pitch, z = 0.35 m, Gaussian-blob amplitudes, uniform phases, seed 0) through a
   value     pair-evals/s with inputs resident in HBM (holo_project on device buffers)
   e2e       the same through the C ABI with page-locked host buffers (copies inside
             the timing)
-  roofline  the pair kernel's lane-op rate on its busier pipe (FP32 FMA or XU/MUFU;
-            ops per pair from the planned variant's pair model and sin/cos split)
-            against that pipe's rate on this GPU measured by holo_probe_peak
+            (a pass of this size runs by cluster expansions: a source-target term counts
+            as one pair evaluation however the sum over them is formed)
+  roofline  warp instructions of the y pass's expansion kernels (ncu counts) per second,
+            against the issue slots of the GPU (4 per clock and SM)
+  pair_kernel  the pair-by-pair kernel alone, forced, on a slice of the y pass, against the
+            same pipes (ops per pair from its pair model and sin/cos split)
   cpu_baseline  the C oracle (FP64, all host threads) on a bounded target sample
 
 ``--impl reference`` times the reference's own CPU algorithm for this path --
@@ -59,8 +62,8 @@ def pipe_ops_per_pair(variant: dict) -> tuple[float, float]:
 
 WORKLOAD = "chain512: 512^2 sources -> 1024^2 projector -> 512^2 projection (x->y->z)"
 # committed ncu summaries whose `key: value` lines the roofline reads
-PROF_TRAFFIC = os.path.join(REPO, "profiles", "k_split_traffic_chain512.md")
 PROF_MIX = os.path.join(REPO, "profiles", "k_split_tc_mix_chain512_slice.md")
+PROF_EXPAND = os.path.join(REPO, "profiles", "k_expand_chain512.md")
 PROF_FP64 = os.path.join(REPO, "profiles", "k_fp64_chain512_slice.md")
 
 
@@ -261,16 +264,16 @@ def run_reference(args):
 
 
 def run_profile_case(args):
-    """Two launches of the pair kernel on a slice of the chain512 y pass (512^2 sources
-    onto the central 256^2 of the projector); the second is the one to capture."""
+    """Two executions of the chain512 y pass (512^2 sources onto the 1024^2 projector, by
+    cluster expansions); of its central 64^2 with --precision fp64, of its central 256^2 with a
+    forced pair kernel (--variants).  The second one is the one to capture."""
     import torch
     import __graft_entry__ as entry
     entry._load_build_module().build()
     holo = entry.load_package()
     amp, phase, u, v, _ = workload()
     side = 1024
-    # central 256^2 patch (split32) or 64^2 patch (fp64, ~0.1 s per launch)
-    lo, hi = (384, 640) if args.precision == "split32" else (480, 544)
+    lo, hi = (480, 544) if args.precision == "fp64" else (384, 640) if args.variants else (0, side)
     vv = v.reshape(side, side, 3)[lo:hi, lo:hi].reshape(-1, 3)
     dev = torch.device("cuda", 0)
     t = lambda a: torch.as_tensor(np.ascontiguousarray(a).reshape(-1), device=dev)
@@ -288,6 +291,60 @@ def run_profile_case(args):
             pl.execute(args_[0], args_[1], -1, LAM)
         torch.cuda.synchronize()
         print(json.dumps({"profile_case": pl.info(), "pairs_per_launch": len(amp) * len(vv)}))
+
+
+def sum_roofline(y_ms, terms_per_s, ms_per_sum, sums, sms, clock_mhz):
+    """The y pass's kernels (`y_ms` each time) against the issue slots and the measured copy
+    bandwidth, by the instructions and DRAM bytes that ncu counted for that pass."""
+    counts = profile_figures(PROF_EXPAND)
+    out = {"bound": "issue", "unit": "Ginst/s", "terms_per_s": terms_per_s,
+           "ms_per_sum": ms_per_sum, "sums": sums, "y_pass_ms": y_ms,
+           "note": "cluster expansions: sin/cos and 1/r between Chebyshev nodes, phasors and short "
+                   "sums on the FP32 and integer pipes, products on the tensor cores; no single pipe "
+                   "is busy, the issue slots are"}
+    if y_ms > 0 and clock_mhz and "warp_instructions_y_pass" in counts:
+        rate = counts["warp_instructions_y_pass"] / (y_ms * 1e-3)
+        peak = sms * 4 * clock_mhz * 1e6
+        out.update({"achieved": rate / 1e9, "peak": peak / 1e9, "frac": rate / peak,
+                    "traffic": counts.get("dram_bytes_y_pass"),
+                    "ops_source": "ncu instruction counts (profiles/k_expand_chain512.md)"})
+        peaks_path = os.path.join(REPO, "MEASURED_PEAKS.json")
+        if os.path.exists(peaks_path) and counts.get("dram_bytes_y_pass"):
+            peaks = json.load(open(peaks_path))
+            gbs = counts["dram_bytes_y_pass"] / (y_ms * 1e-3) / 1e9
+            out["measured_peaks"] = {"source": "MEASURED_PEAKS.json (copy bandwidth)",
+                                     "hbm_gbs": peaks.get("hbm_gbs"), "dram_gbs": gbs,
+                                     "hbm_frac": gbs / peaks["hbm_gbs"]
+                                     if peaks.get("hbm_gbs") else None}
+    return out
+
+
+def pair_kernel_roofline(holo, h, inputs, pairs, variant, mufu_peak, ffma_peak):
+    """The pair-by-pair kernel `variant`, forced, on `inputs` (`pairs` pairs): its rate, and its
+    lane-ops on the FP32 and XU pipes against those pipes' measured rates."""
+    var = next(x for x in holo.variants("split32") if x["variant"] == variant)
+    holo.transform(*inputs, -1, LAM, precision="split32", variant=variant)
+    h.profile_begin()
+    for _ in range(3):
+        holo.transform(*inputs, -1, LAM, precision="split32", variant=variant)
+    ms, n = h.profile_end()
+    rate = pairs * n / (ms * 1e-3)
+    mufu, fp32 = pipe_ops_per_pair(var)
+    source = "pair model of the variant"
+    # lane-ops per pair counted by ncu on the same variant (XU instructions x 32, FMA-pipe
+    # instructions x 32 with packed f32x2 ones counted twice, per pair evaluated)
+    mix = profile_figures(PROF_MIX)
+    if mix.get("variant") == variant and "xu_lane_ops_per_pair" in mix:
+        mufu, fp32 = mix["xu_lane_ops_per_pair"], mix["fma_lane_ops_per_pair"]
+        source = "ncu instruction counts (profiles/k_split_tc_mix_chain512_slice.md)"
+    fp32_frac, xu_frac = rate * fp32 / ffma_peak, rate * mufu / mufu_peak
+    bound = min(mufu_peak / mufu if mufu else float("inf"), ffma_peak / fp32)
+    return {"what": "512^2 sources -> central 256^2 of the projector, forced", "variant": var,
+            "pairs_per_s": rate, "ms_per_launch": ms / n,
+            "bound": "fp32" if fp32_frac > xu_frac else "xu",
+            "frac": max(fp32_frac, xu_frac), "fp32_frac": fp32_frac, "xu_frac": xu_frac,
+            "mufu_per_pair": mufu, "fp32_per_pair": fp32, "ops_per_pair_source": source,
+            "pairs_per_s_frac_of_pipe_bound": rate / bound}
 
 
 def mc_expected_rel_l2(amp, u, v, y, sub, n_sample=256, seed=7):
@@ -681,74 +738,26 @@ def main():
     h2d = 8 * (2 * N + 3 * N + 3 * M + 3 * P)
     d2h = 8 * (2 * M + 2 * P)
 
-    # roofline of the pair kernel: FP32 and MUFU (XU pipe) issue rates against measured peaks
     kern_pairs_s = pairs_step * args.steps / (kern_ms * 1e-3) if kern_ms > 0 else 0.0
     mufu_peak = h.probe_peak(0)
     ffma_peak = h.probe_peak(1)
     with holo.Plan(d_u, d_v, args.precision) as pl:
         info = pl.info()
-    var = next(x for x in holo.variants(args.precision) if x["variant"] == info["variant"]) \
-        if args.precision == "split32" else None
-    MUFU_PER_PAIR, FP32_PER_PAIR = pipe_ops_per_pair(var) if var else (0.0, 0.0)
-    ops_source = "pair model of the planned variant"
-    # lane-ops per pair counted by ncu on the same variant (XU instructions x 32, FMA-pipe
-    # instructions x 32 with packed f32x2 ones counted twice, per pair evaluated)
-    mix = profile_figures(PROF_MIX)
-    if var and mix.get("variant") == var["variant"] and "xu_lane_ops_per_pair" in mix:
-        MUFU_PER_PAIR = mix["xu_lane_ops_per_pair"]
-        FP32_PER_PAIR = mix["fma_lane_ops_per_pair"]
-        ops_source = "ncu instruction counts (profiles/k_split_tc_mix_chain512_slice.md)"
-    achieved = kern_pairs_s * MUFU_PER_PAIR
-    # DRAM bytes per pair-kernel launch (the y pass) from the committed ncu capture
-    traffic = None
+        pl.execute(d_amp, d_phase, -1, LAM)
+        torch.cuda.synchronize()
+        h.profile_begin()
+        for _ in range(5):
+            pl.execute(d_amp, d_phase, -1, LAM)
+        y_ms, y_n = h.profile_end()
+    roofline = sum_roofline(y_ms / max(y_n, 1), kern_pairs_s, kern_ms / max(kern_launches, 1),
+                            kern_launches,
+                            torch.cuda.get_device_properties(dev).multi_processor_count,
+                            clk.get("sm_mhz"))
+    pair_kernel = None
     if args.precision == "split32":
-        traffic = profile_figures(PROF_TRAFFIC).get("bytes_per_launch_y_pass")
-        traffic = int(traffic) if traffic else None
-    # the pair rate this variant could reach if its busiest pipe ran at the measured peak
-    bound_rate = min(mufu_peak / MUFU_PER_PAIR if MUFU_PER_PAIR else float("inf"),
-                     ffma_peak / FP32_PER_PAIR if FP32_PER_PAIR else float("inf")) if var else None
-    # the bound named is the busier of the two pipes (FP32 FMA pipe, XU/MUFU pipe)
-    fp32_ops = kern_pairs_s * FP32_PER_PAIR
-    xu_frac = achieved / mufu_peak if mufu_peak else 0.0
-    fp32_frac = fp32_ops / ffma_peak if ffma_peak else 0.0
-    busy_fp32 = fp32_frac > xu_frac
-    roofline = {"bound": "fp32" if busy_fp32 else "xu",
-                "achieved": (fp32_ops if busy_fp32 else achieved) / 1e9,
-                "peak": (ffma_peak if busy_fp32 else mufu_peak) / 1e9,
-                "unit": "Gop/s", "frac": fp32_frac if busy_fp32 else xu_frac,
-                "traffic": traffic,
-                "note": "compute-bound on the FP32 (FMA) and XU (MUFU) pipes: the busier pipe's "
-                        "lane-ops of the pair kernel per second vs that pipe's rate measured by "
-                        "holo_probe_peak (FFMA / sin.approx throughput kernels); neither HBM nor "
-                        "tensor cores bound this path",
-                "xu_frac": xu_frac, "xu_achieved_gops": achieved / 1e9,
-                "xu_peak_gops": mufu_peak / 1e9,
-                "variant": var, "mufu_per_pair": MUFU_PER_PAIR, "fp32_per_pair": FP32_PER_PAIR,
-                "ops_per_pair_source": ops_source,
-                "fp32_frac": fp32_frac,
-                "fma_peak_gops": ffma_peak / 1e9,
-                "pairs_per_s_frac_of_pipe_bound": kern_pairs_s / bound_rate if bound_rate else None,
-                "kernel_pairs_per_s": kern_pairs_s,
-                "kernel_ms_per_launch": kern_ms / max(kern_launches, 1),
-                "kernel_launches": kern_launches}
-    # the same kernel against the measured copy bandwidth and bf16 GEMM rate: it
-    # moves ~1e-4 bytes per pair and runs 4 TF32 MMAs of K = 8 per pair (64 FLOP; TF32
-    # issues at half the bf16 rate), far from both
-    peaks_path = os.path.join(REPO, "MEASURED_PEAKS.json")
-    if os.path.exists(peaks_path) and kern_launches and var and var.get("pair_loop") == 3:
-        peaks = json.load(open(peaks_path))
-        launch_s = kern_ms * 1e-3 / kern_launches
-        tc_tflops = 64.0 * kern_pairs_s / 1e12
-        roofline["measured_peaks"] = {
-            "source": "MEASURED_PEAKS.json (copy bandwidth; cuBLAS bf16 burst)",
-            "hbm_gbs": peaks.get("hbm_gbs"),
-            "dram_gbs": traffic / launch_s / 1e9 if traffic else None,
-            "hbm_frac": traffic / launch_s / 1e9 / peaks["hbm_gbs"]
-            if traffic and peaks.get("hbm_gbs") else None,
-            "bf16_tflops": peaks.get("bf16_tflops"),
-            "tf32_mma_tflops": tc_tflops,
-            "tensor_frac_of_bf16": tc_tflops / peaks["bf16_tflops"]
-            if peaks.get("bf16_tflops") else None}
+        patch = v.reshape(1024, 1024, 3)[384:640, 384:640].reshape(-1, 3)
+        pair_kernel = pair_kernel_roofline(holo, h, (d_amp, d_phase, d_u, t(patch)),
+                                           N * len(patch), info["variant"], mufu_peak, ffma_peak)
 
     # split-FP32 vs the plain FP64 kernel on a bounded target subset; the split result
     # is the full y pass (the timed tiling and variant) read at those targets
@@ -771,19 +780,26 @@ def main():
     rel = float(np.linalg.norm(a32 - a64) / np.linalg.norm(a64))
     phase_err = float(np.max(np.abs(np.angle(a32 / a64))))
     h.status()
-    # roofline of the FP64 kernel: its FP64-pipe lane-ops per pair (ncu count on a slice of
-    # the same y pass) at the measured pair rate, against the DFMA probe's rate
+    # the FP64 kernel's use of the FP64 pipe: its lane-ops there per pair (ncu count on the
+    # central 64^2 of the projector, whose rows share coordinates) at the pair rate measured
+    # there, against the DFMA probe's rate
     dfma_peak = h.probe_peak(3)
     f64 = profile_figures(PROF_FP64)
-    fp64_roofline = {"bound": "fp64", "pair_evals_per_s": fp64_rate, "peak_gops": dfma_peak / 1e9,
+    d_rows = t(v.reshape(1024, 1024, 3)[480:544, 480:544])
+    holo.transform(d_amp, d_phase, d_u, d_rows, -1, LAM, precision="fp64")
+    torch.cuda.synchronize()
+    h.profile_begin()
+    holo.transform(d_amp, d_phase, d_u, d_rows, -1, LAM, precision="fp64")
+    rows_ms, _ = h.profile_end()
+    rows_rate = N * 64 * 64 / (rows_ms * 1e-3)
+    fp64_roofline = {"bound": "fp64", "pair_evals_per_s": rows_rate, "peak_gops": dfma_peak / 1e9,
                      "unit": "Gop/s", "peak_source": "holo_probe_peak kind 3 (DFMA chains)"}
     if "fp64_pipe_slots_per_pair" in f64:
-        # pipe slots: the DFMA/DADD/DMUL arithmetic plus the pipe's other FP64 instructions
         ops = f64["fp64_pipe_slots_per_pair"]
         fp64_roofline.update({"fp64_pipe_slots_per_pair": ops,
                               "fp64_arith_per_pair": f64.get("fp64_lane_ops_per_pair"),
-                              "achieved_gops": fp64_rate * ops / 1e9,
-                              "frac": fp64_rate * ops / dfma_peak if dfma_peak else None,
+                              "achieved_gops": rows_rate * ops / 1e9,
+                              "frac": rows_rate * ops / dfma_peak if dfma_peak else None,
                               "ops_per_pair_source": "ncu counters on a slice of the same pass "
                                                      "(profiles/k_fp64_chain512_slice.md)"})
 
@@ -816,6 +832,7 @@ def main():
                    "pairs_per_step": pairs_step, "l2": "flushed between timed steps (256 MB write)",
                    "parallelism": f"replicas x{world}" if world > 1 else "1 GPU"},
         "roofline": roofline,
+        "pair_kernel": pair_kernel,
         "cpu_baseline": cpu,
         "e2e": {"value": whole_job_rate(pairs_step, world, e2e_s), "unit": "pair-evals/s",
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

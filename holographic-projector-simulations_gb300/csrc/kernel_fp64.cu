@@ -141,8 +141,9 @@ __global__ void __launch_bounds__(THREADS, MINB)
 // 2^43) takes the FP64 operations instead.
 // Measured (GB300, 1000 sources -> 512^2 lattice targets): 4.4 ms against 30.0 ms (variant 0); the
 // same with targets jittered, so that no coordinate is shared, 5.2 ms; with registers for 4 or
-// 3 CTAs per SM instead of 5 4.6 ms, 2 targets a thread 4.9 ms, 8 4.6 ms.  Bound by the issue
-// slots (4.99 clocks a pair and SM for some 330 instructions) with the FP64 pipe close behind.
+// 3 CTAs per SM instead of 5 4.6 ms, 2 targets a thread 4.9 ms, 8 4.6 ms.  Bound by the FP64
+// pipe: 7.1 of its slots a pair at 0.93 of the rate a pure DFMA stream reaches (ncu: pipe 79 %
+// active, issue slots 55 % for 314 instructions a pair).
 // One target a thread (variant 7) is for problems that would not fill the GPU: a whole call
 // of 64 -> 64^2 0.10 ms against 0.24, of 256 -> 128^2 0.19 against 0.24, but of 1000 ->
 // 128^2 0.44 against 0.37.

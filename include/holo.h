@@ -58,7 +58,8 @@ typedef enum {
 
 typedef enum {
   HOLO_FP64 = 0,    /* the reference's FP64 brute force, term for term */
-  HOLO_SPLIT32 = 1  /* FP64 tile frames + FP32 pair arithmetic (rel-L2 <= 1e-5) */
+  HOLO_SPLIT32 = 1  /* FP64 tile frames + FP32 arithmetic, pair by pair or between clusters of
+                       points by expansions, whichever is faster (rel-L2 <= 1e-5) */
 } holo_precision;
 
 typedef enum { HOLO_FORWARDS = 1, HOLO_BACKWARDS = -1 } holo_direction;
@@ -90,7 +91,8 @@ int holo_transform(holo_handle h, int sign, double lambda,
                    const double *v_xyz, size_t M, double *y_re_im,
                    int precision, holo_stream_t stream);
 
-/* Same as holo_transform with an explicit kernel variant (see holo_variant_*). */
+/* Same as holo_transform with an explicit kernel variant (see holo_variant_*), which always
+ * runs pair by pair. */
 int holo_transform_variant(holo_handle h, int sign, double lambda,
                            const double *amp, const double *phase, const double *u_xyz,
                            size_t N, const double *v_xyz, size_t M, double *y_re_im,
@@ -233,14 +235,16 @@ int holo_transform_batched(holo_handle h, const holo_problem *problems, int n_pr
  * pair: 0 = with the curvature correction c^2/8r^3, 1 = without it, 2 = without
  * it and with 1/r replaced by a first-order series of 1/q (no rsqrt), 3 = model
  * 2 with the phase computed on the tensor cores (tcgen05 TF32 MMAs); it is 0
- * for every HOLO_FP64 variant.  The pair loop is 0 for scalar FP32, 1 for
+ * for every HOLO_FP64 variant (of which 0 to 5 run on the FP64 pipe, 6 and 7 form
+ * the same terms on the integer and FP32 pipes).  The pair loop is 0 for scalar FP32, 1 for
  * packed FP32 pairs (f32x2, two sources per instruction), 2 for packed pairs
  * with warp-specialised sin/cos (a quarter of the warps on the FMA-pipe
  * polynomial for all their targets; fma_sincos_targets is then 0), 3 for the
  * tensor-core kernel (fma_sincos_targets then counts source pairs of every
  * 16 on the polynomial).  The planner takes the first of a speed-ordered list
  * of variants whose error bound holds for the point
- * sets; holo_autotune times every variant on a synthetic problem of the given
+ * sets (where few tiles would leave SMs idle, the one with shorter source tiles);
+ * the sums of a plan may run by expansions instead; holo_autotune times every variant on a synthetic problem of the given
  * size and records the fastest for its bucket.  The Python layer persists the
  * table as JSON. */
 int holo_variant_count(int precision);
@@ -257,8 +261,8 @@ int holo_autotune(holo_handle h, int precision, size_t N, size_t M, int repeats,
  * cuda/transform.cu:355, 397-398, and reported 29 FLOP per pair,
  * cuda/macros.h:71-80) ------------------------------------------------------
  * holo_kernel_launches: kernels this library has launched in the process.
- * holo_profile_begin/end: CUDA-event time of every pair-evaluation kernel
- * launched on the handle in between (end synchronises those events).
+ * holo_profile_begin/end: CUDA-event time of every sum (its pair kernel, or its
+ * expansion kernels together) launched on the handle in between (end synchronises those events).
  * holo_probe_peak: measured issue rate of this GPU's pipes, kind 0 = MUFU
  * (sin.approx.f32, the XU pipe), kind 1 = FP32 FMA, kind 2 = packed FP32 pair
  * FMA (fma.rn.f32x2, two FMAs each), kind 3 = FP64 FMA (the FP64 pipe), in
