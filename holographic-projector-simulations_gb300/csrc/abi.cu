@@ -210,18 +210,25 @@ static bool tiler_scratch(Scratch &tmp, int n, bool packed, TileScratch *t) {
 
 // Tile order of both point sets into the plan's buffers (the order does not depend on the
 // tile size), or the order another plan computed for the same array; their box pyramids,
-// and the statistics on the host (the one host round trip of a tiling).
+// and the statistics on the host (the one host round trip of a tiling).  A set is tiled
+// whatever the other one holds: a chain takes the targets' order from a plan without sources,
+// and a batch gathers the sources of a problem without targets.
 static int tile_both(holo_plan_s *p, const double *u, const double *v, int tiling,
                      const int32_t *known_s, const int32_t *known_t, cudaStream_t s) {
-  if (p->N == 0 || p->M == 0) return HOLO_OK;
   Scratch tmp(p->h, s);
   TileSet set[2] = {};
+  int count = 0;
   BoxStats *stats = tmp.get<BoxStats>(2);
   bool ok = stats != nullptr;
   for (int i = 0; i < 2; ++i) {
-    TileSet &t = set[i];
+    const int n = i ? p->M : p->N;
+    if (n == 0) {
+      HOLO_TRY(launch_gather_pos(nullptr, nullptr, 0, i ? 0 : p->n_pad, i ? p->pos_t : p->pos_s, s));
+      continue;
+    }
+    TileSet &t = set[count++];
     t.pos = i ? v : u;
-    t.n = i ? p->M : p->N;
+    t.n = n;
     t.n_pad = i ? p->M : p->n_pad;
     t.known = i ? known_t : known_s;
     t.order = i ? p->order_t : p->order_s;
@@ -232,12 +239,13 @@ static int tile_both(holo_plan_s *p, const double *u, const double *v, int tilin
     ok = ok && t.parts && (t.known || tiler_scratch(tmp, t.n, tiling == kTilePacked, &t.scratch));
   }
   if (!ok) return fail(HOLO_ERR_ALLOC, "tiler scratch");
-  HOLO_TRY(tile_sets(set, 2, tiling, s));
+  if (count == 0) return HOLO_OK;
+  HOLO_TRY(tile_sets(set, count, tiling, s));
   BoxStats both[2];
   HOLO_CUDA(cudaMemcpyAsync(both, stats, sizeof(both), cudaMemcpyDeviceToHost, s));
   HOLO_CUDA(cudaStreamSynchronize(s));
-  p->stats_s = both[0];
-  p->stats_t = both[1];
+  if (p->N) p->stats_s = both[0];
+  if (p->M) p->stats_t = both[1];
   return HOLO_OK;
 }
 
