@@ -212,7 +212,7 @@ struct MomentsSmem {
   static constexpr size_t cheb = b + 4 * 2 * kGroupT * kChunk * 4;  // float [2][16][68]
   static constexpr size_t rec = cheb + 2 * kMaxP * kChebStride * 4;  // float [9][64]
   static constexpr size_t bars = rec + 9 * kSuper * 4;          // uint64 [3]
-  static constexpr size_t misc = bars + 4 * 8;                  // uint32 taddr, abort
+  static constexpr size_t misc = bars + 4 * 8;                  // uint32 taddr, abort, spoilt
   static constexpr size_t bytes = misc + 16;
 };
 constexpr int kMomThreads = 256;
@@ -230,10 +230,12 @@ __global__ void __launch_bounds__(kMomThreads, 2)
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::bars);  // free[2], full
   uint32_t *taddr_slot = reinterpret_cast<uint32_t *>(smem + L::misc);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + L::misc + 4);
+  volatile int *spoilt = reinterpret_cast<volatile int *>(smem + L::misc + 8);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int b = 0; b < 3; ++b) ptx::mbar_init(&bars[b], 1);
     *abort_flag = 0;
+    *spoilt = 0;
     ptx::fence_barrier_init();
   }
   if (warp == 0) ptx::tmem_alloc(taddr_slot, 256);
@@ -304,6 +306,10 @@ __global__ void __launch_bounds__(kMomThreads, 2)
         cluster_offset(P.geo_s, P.shift_s, idx, P.cs_log2, h, l);
         pa = P.apf_s[idx];
       }
+      // a source that is not finite spoils the cluster's moments; it is looked for here, once
+      // a source, because the splits into TF32 parts below turn a NaN into a zero
+      const float zero = fmaf(0.f, h[0], fmaf(0.f, h[1], fmaf(0.f, h[2], fmaf(0.f, pa.x, 0.f * pa.y))));
+      if (!(zero == 0.f)) *spoilt = 1;
       if (axis == 0) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -414,12 +420,14 @@ __global__ void __launch_bounds__(kMomThreads, 2)
     flush(128);
   }
   const int node = 32 * (warp & 3) + lane;
+  // (every staging is behind a barrier of its chunks)
+  const float nan = *spoilt ? __int_as_float(0x7fffffff) : 0.f;
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
     const int T = tg * kGroupT + 32 * (warp >> 2) + j;
     if (T < P.nTs)
       P.moments[((size_t)ks * P.nTs * P.nS + (size_t)T * P.nS + S) * kNodes + node] =
-          make_float2(acc_re[j], acc_im[j]);
+          make_float2(acc_re[j] + nan, acc_im[j] + nan);
   }
   // every commit has arrived before the block ends
   if (tid == 0)
@@ -429,6 +437,12 @@ __global__ void __launch_bounds__(kMomThreads, 2)
   __syncthreads();
   ptx::tc_fence_after();
   if (warp == 0) ptx::tmem_dealloc(tbase, 256);
+}
+
+// x rounded to TF32; NaN and infinities as they are (to_tf32_int's carry runs a NaN's fraction over
+// into the sign: -0).
+__device__ __forceinline__ float tf32_or_nonfinite(float x) {
+  return __fsub_rn(x, x) == 0.f ? ptx::to_tf32_int(x) : x;
 }
 
 // ---- translate -----------------------------------------------------------------------------
@@ -553,11 +567,11 @@ __global__ void __launch_bounds__(kNodes) k_expand_translate(
   const int nSG = (P.nS + kGroupS - 1) / kGroupS, row = S % kGroupS;
   float *o = P.coeffs + ((size_t)Tl * nSG + S / kGroupS) * 2 * kHalfFloats +
              (size_t)(n >> 3) * (4 * kGroupS * kTcK);
-  const float rh = ptx::to_tf32_int(nu.x), ih = ptx::to_tf32_int(nu.y);
+  const float rh = tf32_or_nonfinite(nu.x), ih = tf32_or_nonfinite(nu.y);
   o[tc_off(row, n & 7)] = rh;
   o[tc_off(kGroupS + row, n & 7)] = ih;
-  o[tc_off(2 * kGroupS + row, n & 7)] = ptx::to_tf32_int(__fsub_rn(nu.x, rh));
-  o[tc_off(3 * kGroupS + row, n & 7)] = ptx::to_tf32_int(__fsub_rn(nu.y, ih));
+  o[tc_off(2 * kGroupS + row, n & 7)] = tf32_or_nonfinite(__fsub_rn(nu.x, rh));
+  o[tc_off(3 * kGroupS + row, n & 7)] = tf32_or_nonfinite(__fsub_rn(nu.y, ih));
 }
 
 // ---- targets -------------------------------------------------------------------------------
