@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kFixThreads, MINB)
   long long *samp = reinterpret_cast<long long *>(smem + L::amp);
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::bar);
   static_assert(CS == 16 || CS == 64, "the amplitudes' reduction");
-  __shared__ int s_exp[2], s_count[2];
+  __shared__ int s_exp[2];
   const int tid = threadIdx.x;
   constexpr uint32_t kTables = fixed::kTrigEntries * sizeof(fixed::TrigEntry),
                      kTurns = fixed::kTurnEntries * sizeof(fixed::TurnWords);
@@ -247,16 +247,11 @@ __global__ void __launch_bounds__(kFixThreads, MINB)
         // 4095 marks what has no place here: a subnormal, an infinity, a NaN
         const bool bad = e == 0x7ff || (e == 0 && (a & 0x7fffffffffffffffLL) != 0);
         const int top = __reduce_max_sync(0xffffffffu, (bad ? 4095 : e) << 6 | tid);
-        const uint32_t lit = __ballot_sync(0xffffffffu, e != 0);
-        if ((tid & 31) == 0) {
-          s_exp[tid >> 5] = top;
-          s_count[tid >> 5] = __popc(lit);
-        }
+        if ((tid & 31) == 0) s_exp[tid >> 5] = top;
       }
       __syncthreads();
-      const int lit = s_count[0] + s_count[1];
       const int key = max(s_exp[0], s_exp[1]), top = min(key & 63, count - 1);
-      const int ea = lit ? key >> 6 : max(key >> 6, 1023);
+      const int ea = key >= 64 ? key >> 6 : 1023;  // all zero: any scale
       if (tid < CS) {
         const long long a = tid < count ? __double_as_longlong(sa[tid].y) : 0;
         const int e = (int)(a >> 52) & 0x7ff, down = ea - e;
@@ -265,20 +260,23 @@ __global__ void __launch_bounds__(kFixThreads, MINB)
         samp[tid] = a < 0 ? -f : f;
       }
       __syncthreads();
-      // the scale: a quarter of the largest source's distance from the thread's first target
-      int qref;
+      // the scale: a quarter of the largest source's distance from the thread's first target,
+      // where that is a normal number well inside the exponent range
+      int qref, es;
+      bool usable;
       {
         const double a = vx[0] - sp[3 * top], b = vy[0] - sp[3 * top + 1],
                      c = vz[0] - sp[3 * top + 2];
-        const int hi = __double2hiint(a * a + b * b + c * c);
-        qref = ((((hi >> 20) & 0x7ff) - 1023) >> 1) - 2;
+        const uint32_t hi = (uint32_t)__double2hiint(a * a + b * b + c * c);
+        qref = (((int)(hi >> 20) - 1023) >> 1) - 2;
+        es = ea - 1078 - qref + 1023;  // exponent field of the sums' unit
+        usable = hi - (200u << 20) < (1600u << 20) && ea > 200 && ea < 2047 && es > 0 && es < 2046;
       }
-      const int es = ea - 1078 - qref + 1023;  // exponent field of the sums' unit
-      const bool usable = ea > 200 && ea < 2047 && es > 0 && es < 2046;
       const double unit = usable ? __hiloint2double(es << 20, 0) : 0.0;
       long long fr[R], fi[R];
+      uint32_t made = 0;  // products formed, a byte for each target: each rounds down
 #pragma unroll
-      for (int r = 0; r < R; ++r) fr[r] = fi[r] = (lit + 1) >> 1;  // each product rounds down
+      for (int r = 0; r < R; ++r) fr[r] = fi[r] = 0;
       // the sources of this tile; mask: coordinates that the targets of each thread share
       auto sum_tile = [&](auto mask) {
         constexpr bool SX = decltype(mask)::value & 1, SY = decltype(mask)::value & 2,
@@ -317,6 +315,7 @@ __global__ void __launch_bounds__(kFixThreads, MINB)
               const int64_t w = fixed::mulhi64(am, fixed::reciprocal(rt)) >> (down + 2);
               fr[r] += fixed::mulhi64(w, c);
               fi[r] += fixed::mulhi64(w, sn);
+              made += w != 0 ? 1u << (8 * r) : 0u;
             } else {
               const double d = __dsqrt_rn(ss);
               const double kr = __dmul_rn(d, P.k);
@@ -338,8 +337,9 @@ __global__ void __launch_bounds__(kFixThreads, MINB)
       if (usable)
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          re[r] = fma((double)fr[r], unit, re[r]);
-          im[r] = fma((double)fi[r], unit, im[r]);
+          const long long up = (long long)((made >> (8 * r) & 255u) + 1u) >> 1;
+          re[r] = fma((double)(fr[r] + up), unit, re[r]);
+          im[r] = fma((double)(fi[r] + up), unit, im[r]);
         }
       __syncthreads();  // buffer `buf` is refilled two tiles later, the amplitudes at once
     }
