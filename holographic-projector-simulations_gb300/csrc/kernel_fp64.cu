@@ -135,8 +135,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
 // where they agree in a coordinate, as the rows of a lattice do: `share`), the product
 // distance x k and the sum phase + that.  Bit for bit the other kernel's phases; amplitude /
 // distance, sine and cosine are exact to 2^-55 or better and their products are summed as
-// 64-bit integers, a tile of sources at a time, to 2^-54 of the term of the tile's largest
-// amplitude, whose distance sets the scale.  A pair out of the fixed-point ranges (a zero,
+// 64-bit integers, a tile of sources at a time, to 2^-54 of the target's own term of the tile's
+// largest amplitude, whose distance sets the target's scale.  A pair out of the fixed-point ranges (a zero,
 // infinite or NaN value, a distance four times under the one that set the scale, a phase beyond
 // 2^43) takes the FP64 operations instead.
 // Measured (GB300, 1000 sources -> 512^2 lattice targets): 4.4 ms against 30.0 ms (variant 0); the
@@ -260,27 +260,38 @@ __global__ void __launch_bounds__(kFixThreads, MINB)
         samp[tid] = a < 0 ? -f : f;
       }
       __syncthreads();
-      // the scale: a quarter of the largest source's distance from the thread's first target,
-      // where that is a normal number well inside the exponent range
-      int qref, es;
-      bool usable;
-      {
-        const double a = vx[0] - sp[3 * top], b = vy[0] - sp[3 * top + 1],
-                     c = vz[0] - sp[3 * top + 2];
-        const uint32_t hi = (uint32_t)__double2hiint(a * a + b * b + c * c);
-        qref = (((int)(hi >> 20) - 1023) >> 1) - 2;
-        es = ea - 1078 - qref + 1023;  // exponent field of the sums' unit
-        usable = hi - (200u << 20) < (1600u << 20) && ea > 200 && ea < 2047 && es > 0 && es < 2046;
-      }
-      const double unit = usable ? __hiloint2double(es << 20, 0) : 0.0;
-      long long fr[R], fi[R];
-      uint32_t made = 0;  // products formed, a byte for each target: each rounds down
-#pragma unroll
-      for (int r = 0; r < R; ++r) fr[r] = fi[r] = 0;
+      // exponent field of the unit of sums scaled by 2^-q
+      auto unit_exp = [&](int q) { return ea - 1078 - q + 1023; };
       // the sources of this tile; mask: coordinates that the targets of each thread share
       auto sum_tile = [&](auto mask) {
         constexpr bool SX = decltype(mask)::value & 1, SY = decltype(mask)::value & 2,
                        SZ = decltype(mask)::value & 4;
+        // the scale of each target: a quarter of its distance from the tile's brightest source,
+        // where that is well inside the exponent range; kNoScale sends every pair of the target
+        // to the FP64 operations
+        constexpr int kNoScale = -100000;
+        int qref[R];
+        long long fr[R], fi[R];
+        uint32_t made = 0;  // products formed, a byte for each target: each rounds down
+        {
+          const double ux = sp[3 * top], uy = sp[3 * top + 1], uz = sp[3 * top + 2];
+          double both = 0.0;  // what the targets share
+          if (SX) { const double d = vx[0] - ux; both = d * d; }
+          if (SY) { const double d = vy[0] - uy; both = fma(d, d, both); }
+          if (SZ) { const double d = vz[0] - uz; both = fma(d, d, both); }
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            double ss = both;
+            if (!SX) { const double d = vx[r] - ux; ss = fma(d, d, ss); }
+            if (!SY) { const double d = vy[r] - uy; ss = fma(d, d, ss); }
+            if (!SZ) { const double d = vz[r] - uz; ss = fma(d, d, ss); }
+            const uint32_t hi = (uint32_t)__double2hiint(ss);
+            const int q = (((int)(hi >> 20) - 1023) >> 1) - 2, es = unit_exp(q);
+            const bool in = hi - (200u << 20) < (1600u << 20) && ea > 200 && ea < 2047;
+            qref[r] = in && es > 0 && es < 2046 ? q : kNoScale;
+            fr[r] = fi[r] = 0;
+          }
+        }
         for (int s = 0; s < count; ++s) {
           const double ux = sp[3 * s], uy = sp[3 * s + 1], uz = sp[3 * s + 2];
           const double phi = sa[s].x;
@@ -302,8 +313,8 @@ __global__ void __launch_bounds__(kFixThreads, MINB)
             const double ph = __dadd_rn(phi, __dmul_rn(dist, sk));
             const uint32_t hp = (uint32_t)__double2hiint(ph);
             const uint32_t te = ((hp >> 20) & 0x7ffu) - (uint32_t)(1023 + fixed::kTurnLow);
-            const uint32_t down = (uint32_t)(rt.q - qref);
-            const bool fast = usable && hi - (200u << 20) < (1600u << 20) && down <= 40u &&
+            const uint32_t down = (uint32_t)(rt.q - qref[r]);
+            const bool fast = hi - (200u << 20) < (1600u << 20) && down <= 40u &&
                               te < (uint32_t)fixed::kTurnEntries;
             if (fast) {
               const uint4 k = *reinterpret_cast<const uint4 *>(&turns[te]);
@@ -328,19 +339,20 @@ __global__ void __launch_bounds__(kFixThreads, MINB)
             }
           }
         }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if (qref[r] == kNoScale) continue;
+          const double unit = __hiloint2double(unit_exp(qref[r]) << 20, 0);
+          const long long up = (long long)((made >> (8 * r) & 255u) + 1u) >> 1;
+          re[r] = fma((double)(fr[r] + up), unit, re[r]);
+          im[r] = fma((double)(fi[r] + up), unit, im[r]);
+        }
       };
       if (R == 1) sum_tile(std::integral_constant<int, 7>{});
       else if (share[2] && share[0]) sum_tile(std::integral_constant<int, 5>{});
       else if (share[2] && share[1]) sum_tile(std::integral_constant<int, 6>{});
       else if (share[2]) sum_tile(std::integral_constant<int, 4>{});
       else sum_tile(std::integral_constant<int, 0>{});
-      if (usable)
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const long long up = (long long)((made >> (8 * r) & 255u) + 1u) >> 1;
-          re[r] = fma((double)(fr[r] + up), unit, re[r]);
-          im[r] = fma((double)(fi[r] + up), unit, im[r]);
-        }
       __syncthreads();  // buffer `buf` is refilled two tiles later, the amplitudes at once
     }
 
