@@ -186,6 +186,7 @@ ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk,
   P.shift_s = tmp.take<float>(8 * (size_t)((P.N + P.cs - 1) / P.cs));
   P.shift_t = tmp.take<float>(8 * (size_t)((P.M + P.tt - 1) / P.tt));
   P.cheb = tmp.take<float>(2 * (16 * 16 + 16));
+  P.tops = tmp.take<uint32_t>((size_t)(P.N + 4095) / 4096 + 1);
   P.moments = tmp.take<float2>((size_t)P.ksplit * pairs * kExpandNodes);
   P.coeffs = tmp.take<float>((size_t)P.slab * groups_s * 16384);
   P.partial = P.ssplit > 1 ? tmp.take<double2>((size_t)P.ssplit * P.M) : nullptr;

@@ -304,6 +304,8 @@ struct ExpandProblem {
   float *half_s, *half_t;            // [cluster][4]: half extents along ax and ay, inverses
   float *shift_s, *shift_t;          // [tile][8]: tile centre - cluster centre, float-float
   float *cheb;                       // Chebyshev tables of both axes
+  uint32_t *tops;                    // bits of the largest |amplitude| of every 4096 sources, then
+                                     // the exponent field of the sum's scale
   float2 *moments;                   // [ksplit][nTs][nS][kExpandNodes]
   float *coeffs;                     // [nTs][nS / 32][2][hi, lo][8][64 x 8]: MMA operand
   int N, M, cs, tt, ns, nt, nS, nT, t0, nTs, slab;  // slab: target clusters per launch

@@ -113,7 +113,29 @@ __device__ __forceinline__ float reduce_two_pi_with(float S, float E, float c) {
   return __fadd_rn(r, E);
 }
 
-// ---- set-up: frames of all cluster pairs, offsets of the variant's tile centres from the
+// Amplitudes that a block of the set-up looks at, and the blocks for n of them.
+constexpr int kTopBlock = 4096;
+__host__ __device__ __forceinline__ int top_blocks(int n) { return (n + kTopBlock - 1) / kTopBlock; }
+
+// Exponent field of the power of two that the amplitudes are divided by, from the bits of the
+// largest: moments, nodal weights and coefficients then stay far from the ends of the FP32
+// range, whatever unit the caller's amplitudes are in (a low TF32 part of 1e-36 would be a
+// subnormal of a few bits).  Powers of two: no other rounding than without.
+__device__ __forceinline__ int scale_field(uint32_t top) {
+  const int e = (int)(top >> 23);
+  return top == 0u || e == 255 ? 127 : min(max(e, 1), 253);
+}
+
+// x times the scale, in its exponent (a product would take the FP64 pipe); a sum of two floats and
+// a float's power of two stay far from the ends of the FP64 range.
+__device__ __forceinline__ double scaled(double x, uint32_t field) {
+  const int hi = __double2hiint(x), e = hi & 0x7ff00000;
+  return e == 0 || e == 0x7ff00000
+             ? x
+             : __hiloint2double(hi + (((int)field - 127) << 20), __double2loint(x));
+}
+
+// ---- set-up: frames of all cluster pairs, largest amplitudes, offsets of the variant's tile centres from the
 // cluster centres, Chebyshev tables ----
 // Bound by the FP64 pipe's latency (a frame is ~150 dependent FP64 operations): one thread
 // per pair, so a few thousand pairs run in the time of one.
@@ -123,7 +145,20 @@ __global__ void __launch_bounds__(128) k_expand_setup(const ExpandProblem P0,
                                                       const int *__restrict__ offs, int n_probs) {
   int item;
   const ExpandProblem &P = find_problem<BATCHED>(P0, probs, offs, n_probs, &item);
-  int i = item * blockDim.x + threadIdx.x;
+  const int tops = top_blocks(P.N);
+  if (item < tops) {  // the largest of kTopBlock amplitudes (their bits order like the values)
+    __shared__ uint32_t most[4];
+    uint32_t m = 0;
+    const int first = item * kTopBlock, last = min(P.N, first + kTopBlock);
+    for (int j = first + threadIdx.x; j < last; j += 128)
+      m = max(m, __float_as_uint(P.apf_s[j].y) & 0x7fffffffu);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) most[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) P.tops[item] = max(max(most[0], most[1]), max(most[2], most[3]));
+    return;
+  }
+  int i = (item - tops) * blockDim.x + threadIdx.x;
   const int pairs = P.nTs * P.nS;
   if (i < pairs) {
     const int T = P.t0 + i / P.nS, S = i % P.nS;
@@ -212,7 +247,7 @@ struct MomentsSmem {
   static constexpr size_t cheb = b + 4 * 2 * kGroupT * kChunk * 4;  // float [2][16][68]
   static constexpr size_t rec = cheb + 2 * kMaxP * kChebStride * 4;  // float [9][64]
   static constexpr size_t bars = rec + 9 * kSuper * 4;          // uint64 [3]
-  static constexpr size_t misc = bars + 4 * 8;                  // uint32 taddr, abort, spoilt
+  static constexpr size_t misc = bars + 4 * 8;                  // uint32 taddr, abort, spoilt, unscale
   static constexpr size_t bytes = misc + 16;
 };
 constexpr int kMomThreads = 256;
@@ -251,6 +286,18 @@ __global__ void __launch_bounds__(kMomThreads, 2)
   const int px = P.px, py = P.py, np = px * py;
   const float4 half = reinterpret_cast<const float4 *>(P.half_s)[S];
   const float kap = P.kap;
+  // the sum's scale, for the staging threads; its exponent field for the target kernel
+  float *unscale = reinterpret_cast<float *>(smem + L::misc + 12);
+  if (warp == 1) {
+    uint32_t m = 0;
+    const int tops = top_blocks(P.N);
+    for (int b = lane; b < tops; b += 32) m = max(m, P.tops[b]);
+    const int e = scale_field(__reduce_max_sync(0xffffffffu, m));
+    if (lane == 0) {
+      *unscale = __uint_as_float((uint32_t)(254 - e) << 23);
+      if (item == 0) P.tops[tops] = (uint32_t)e;
+    }
+  }
 
   // this thread's target cluster and its share of a chunk's sources
   const int tq = tid & (kGroupT - 1), quad = tid >> 6, Tl = tg * kGroupT + tq;
@@ -318,7 +365,7 @@ __global__ void __launch_bounds__(kMomThreads, 2)
         }
         rec[6 * kSuper + i] = fmaf(h[0], h[0], fmaf(h[1], h[1], h[2] * h[2]));
         rec[7 * kSuper + i] = pa.x;
-        rec[8 * kSuper + i] = pa.y;
+        rec[8 * kSuper + i] = pa.y * *unscale;
         cheb_row(pick(h, P.ax) * half.z, px, cheb + i, kChebStride);
       } else {
         cheb_row(pick(h, P.ay) * half.w, py, cheb + kMaxP * kChebStride + i, kChebStride);
@@ -837,6 +884,7 @@ __global__ void __launch_bounds__(kTgtThreads, 1)
     auto write_out = [&](uint32_t i) {
       if (half) return;
       const int order = out_t >= 0 && out_p->ssplit == 1 ? out_p->order_t[out_t] : 0;
+      const uint32_t field = out_t >= 0 ? out_p->tops[top_blocks(out_p->N)] : 127u;
       if (!tc_wait(parts_ready, i & 1u, abort_flag, err)) return;
       float4 s = part[row];
 #pragma unroll
@@ -852,7 +900,8 @@ __global__ void __launch_bounds__(kTgtThreads, 1)
       }
       ptx::mbar_arrive(parts_free);
       if (out_t >= 0) {
-        const double2 v = make_double2((double)s.x + (double)s.y, (double)s.z + (double)s.w);
+        const double2 v = make_double2(scaled((double)s.x + (double)s.y, field),
+                                       scaled((double)s.z + (double)s.w, field));
         if (out_p->ssplit == 1)
           out_p->y[order] = v;
         else
@@ -944,7 +993,7 @@ __global__ void __launch_bounds__(kTgtThreads, 1)
 void expand_blocks(const ExpandProblem &p, int blocks[4]) {
   const long long n = (long long)p.nTs * p.nS + (p.N + p.cs - 1) / p.cs + (p.M + p.tt - 1) / p.tt +
                       p.nS + p.nT + 2 * kMaxP * kMaxP;
-  blocks[0] = (int)((n + 127) / 128);
+  blocks[0] = top_blocks(p.N) + (int)((n + 127) / 128);
   blocks[1] = p.nS * ((p.nTs + kGroupT - 1) / kGroupT) * p.ksplit;
   blocks[2] = p.nS * p.nTs;
   const long long m0 = (long long)p.t0 * p.nt, m1 = (long long)(p.t0 + p.nTs) * p.nt;
