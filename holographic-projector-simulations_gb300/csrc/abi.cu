@@ -374,7 +374,7 @@ static double pair_seconds(const holo_plan_s *p) {
 int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, size_t M,
                      int precision, int forced_variant, cudaStream_t s, holo_plan_s **out,
                      const int32_t *known_order_s, const int32_t *known_order_t,
-                     int known_tiling_s, int known_tiling_t, double k_once) {
+                     int known_tiling_s, int known_tiling_t, double k_once, bool replayed) {
   if (precision != HOLO_FP64 && precision != HOLO_SPLIT32)
     return fail(HOLO_ERR_INVALID, "unknown precision %d", precision);
   HOLO_TRY(check_sizes(N, M));
@@ -465,7 +465,7 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
     HOLO_TRY(choose(&ci));
     // A call that uses its plan once keeps the Hilbert tiles where they go by expansions, or
     // where the faster variant would save less than packing takes (0.65 ms: 30000 -> 3000
-    // takes 0.15 ms in all without it)
+    // takes 0.15 ms in all without it); a batch, which is replayed, in the first case only
     constexpr double kPackSeconds = 0.65e-3;
     bool stay = false;
     if (ci > 0 && forced_variant < 0 && k_once > 0.0) {
@@ -473,8 +473,8 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
       HOLO_TRY(plan_grid(pp));
       const double saving = pair_seconds(pp) * (1.0 - pair_rate(split_variant(variant)) /
                                                           pair_rate(split_variant(cands[0])));
-      stay = plan_expansion(pp, k_once).use ||
-             (p->err_bound <= kSplitBoundMetres && saving < kPackSeconds);
+      stay = plan_expansion(pp, k_once, replayed ? 0.0 : kExpandLaunches).use ||
+             (!replayed && p->err_bound <= kSplitBoundMetres && saving < kPackSeconds);
     }
     if (ci > 0 && forced_variant < 0 && !stay) {
       size_t cp = 0;

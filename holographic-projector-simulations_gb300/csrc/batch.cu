@@ -118,7 +118,7 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
     holo_plan_s *p = nullptr;
     HOLO_TRY(plan_create_impl(h, pr[i].u_xyz, pr[i].N, pr[i].v_xyz, pr[i].M, precision, -1, s, &p,
                               nullptr, nullptr, kTileHilbert, kTileHilbert,
-                              (2.0 * M_PI) / pr[i].lambda));
+                              (2.0 * M_PI) / pr[i].lambda, true));
     b->plans.push_back(p);
     b->total_pairs += (long long)pr[i].N * (long long)pr[i].M;
   }

@@ -441,14 +441,16 @@ void pool_free(void *p, cudaStream_t s);
 int size_bucket(size_t N, size_t M);
 // k_once: the wave number of the one transform this plan is for (0: a plan to keep, with the
 // positions its adjoint would need); where that runs by cluster expansions the Hilbert tiles
-// do, whatever their bound for the pair kernels.
+// do, whatever their bound for the pair kernels.  replayed: that transform is run many times (a
+// batch), so what does not go by expansions is tiled as for a plan to keep.
 // known_order_s / known_order_t: the tile order of the same source / target array
 // from another split plan (copied instead of recomputed), of tiling known_tiling_s/t
 int plan_create_impl(holo_handle h, const double *u_dev, size_t N, const double *v_dev,
                      size_t M, int precision, int forced_variant, cudaStream_t s,
                      holo_plan_s **out, const int32_t *known_order_s = nullptr,
                      const int32_t *known_order_t = nullptr, int known_tiling_s = kTileHilbert,
-                     int known_tiling_t = kTileHilbert, double k_once = 0.0);
+                     int known_tiling_t = kTileHilbert, double k_once = 0.0,
+                     bool replayed = false);
 int plan_execute_impl(holo_plan_s *p, int sign, double lambda, const double *amp_dev,
                       const double *phase_dev, double2 *y_dev, int flags, cudaStream_t s);
 void plan_release(holo_plan_s *p, cudaStream_t s);
