@@ -350,6 +350,7 @@ static int plan_grid(holo_plan_s *p) {
   const int max_splits = (int)std::max<size_t>(1, scratch_cap / (std::max<size_t>(p->M, 1) * 16));
   p->splits = choose_splits(p->n_ttiles, p->n_stiles, G, p->M, max_splits);
   p->grid = std::max(1, std::min(G, p->n_ttiles * p->splits));
+  p->expand_k = 0.0;  // chosen against another kernel's time, if at all
   return HOLO_OK;
 }
 
@@ -475,6 +476,7 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
                                                           pair_rate(split_variant(cands[0])));
       stay = plan_expansion(pp, k_once, replayed ? 0.0 : kExpandLaunches).use ||
              (!replayed && p->err_bound <= kSplitBoundMetres && saving < kPackSeconds);
+      p->expand_only = stay && p->err_bound > kSplitBoundMetres;
     }
     if (ci > 0 && forced_variant < 0 && !stay) {
       size_t cp = 0;
@@ -499,7 +501,6 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
   }
   const Variant V = precision == HOLO_SPLIT32 ? split_variant(variant) : fp64_variant(variant);
   p->variant = variant;
-  p->expand_k = 0.0;  // chosen for another tiling, if at all
   HOLO_TRY(plan_grid(p.get()));
 
   if (precision == HOLO_SPLIT32) {
@@ -539,10 +540,11 @@ ExpandChoice plan_expansion(holo_plan_s *p, double k, double launches) {
   if (p->precision != HOLO_SPLIT32 || p->pair_kernel_only || p->N == 0 || p->M == 0) return {};
   const Variant V = split_variant(p->variant);
   if (box_level(V.cs) < 0) return {};  // its tiles do not nest in the clusters
-  if (p->expand_k != k) {
+  if (p->expand_k != k || p->expand_launches != launches) {
     p->expand = expand_choose(p->stats_s, p->stats_t, p->N, p->M, box_level(V.cs), box_level(V.tt()),
                               k, pair_seconds(p), launches, p->h->sm_count);
     p->expand_k = k;
+    p->expand_launches = launches;
   }
   return p->expand;
 }
@@ -562,6 +564,7 @@ int plan_execute_impl(holo_plan_s *p, int sign, double lambda, const double *amp
   const bool cst = (flags & HOLO_FLAG_CONST_PHASE) != 0;
   const ExpandChoice ch = cst ? ExpandChoice{} : plan_expansion(p, k);
   if (ch.use) return expand_execute(p, ch, sign * k, amp, phase, y, s);
+  if (p->expand_only) return fail(HOLO_ERR_UNSUPPORTED, "tiles too wide for the pair kernels");
   double2 *ap = tmp.get<double2>(p->n_pad);
   double2 *partial = p->splits > 1 ? tmp.get<double2>((size_t)p->splits * p->M) : nullptr;
   if (!ap || (p->splits > 1 && !partial)) return fail(HOLO_ERR_ALLOC, "execute scratch");

@@ -131,6 +131,8 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
   for (int i = 0; i < n; ++i) {
     choice[i] = plan_expansion(b->plans[i], (2.0 * M_PI) / pr[i].lambda, 0.0);
     if (choice[i].use) seconds += choice[i].seconds;
+    else if (b->plans[i]->expand_only)
+      return fail(HOLO_ERR_UNSUPPORTED, "problem %d: tiles too wide for the pair kernels", i);
   }
   for (int i = 0; i < n; ++i) {
     if (!choice[i].use) continue;

@@ -412,7 +412,9 @@ struct holo_plan_s {
   holo::BoxStats stats_s{}, stats_t{};
   double *odd_tiles = nullptr;   // boxes of source tiles that are none of these sizes
   bool pair_kernel_only = false; // a forced variant: always that kernel
-  double expand_k = 0.0;         // wave number of `expand` (0: not chosen yet)
+  // wave number and launch cost that `expand` was chosen for (0: not chosen yet)
+  double expand_k = 0.0, expand_launches = 0.0;
+  bool expand_only = false;      // one-shot: tiles whose bound rules the pair kernels out
   holo::ExpandChoice expand;
   int32_t *order_s = nullptr;    // N (split only)
   int32_t *order_t = nullptr;    // M (split only)
