@@ -7,9 +7,10 @@
 // items go into one device work queue sorted longest-first, drained by one
 // persistent split-precision kernel with an atomic counter (no CTA waits on
 // another).  Problems that run by cluster expansions share one launch of each of
-// their four kernels, whose blocks find their problem by its first block.  Gathers
-// (one launch), the queue reset, the queue and expansion kernels and the cross-split
-// reductions are captured once into a CUDA graph; holo_batch_execute replays it.
+// their four kernels, whose blocks find their problem by its first block (several
+// rounds of launches where their scratch is large).  Gathers (one launch), the queue
+// reset, the queue and expansion kernels and the cross-split reductions are captured
+// once into a CUDA graph; holo_batch_execute replays it.
 #include <algorithm>
 #include <memory>
 
@@ -75,26 +76,83 @@ int describe_problem(holo_batch_s *b, const holo_problem &q, holo_plan_s *p, int
   return HOLO_OK;
 }
 
-// Scratch and descriptor of problem i, which fills `share` of the GPU, by cluster expansions;
-// P is what the reduction of its partial sums needs.
-int describe_expansion(holo_batch_s *b, const holo_problem &q, holo_plan_s *p, const ExpandChoice &ch,
-                       double share, ExpandProblem *E, SplitProblem *P, cudaStream_t s) {
-  const double sk = q.sign * ((2.0 * M_PI) / q.lambda);
-  ExpandScratch size, tmp;
-  expand_describe(p, ch, sk, (double2 *)q.y_re_im, share, size);
-  tmp.base = (unsigned char *)pool_alloc(b->h, size.bytes, s);
-  if (!tmp.base) return fail(HOLO_ERR_ALLOC, "batch expansion scratch of %zu bytes", size.bytes);
-  b->owned.push_back(tmp.base);
-  *E = expand_describe(p, ch, sk, (double2 *)q.y_re_im, share, tmp);
-  E->nTs = std::min(E->slab, E->nT);
-  *P = SplitProblem{};
-  P->apf_s = E->apf_s;
-  P->order_t = p->order_t;
-  P->partial = E->partial;
-  P->y = E->y;
-  P->N = p->N;
-  P->M = p->M;
-  P->splits = E->ssplit;
+// Sums by cluster expansions that share one launch of each of their kernels: [first, last) of
+// the batch's, or one that needs several slabs.
+struct Round {
+  int first, last;
+  bool slabs;
+};
+
+// Descriptors and scratch of the problems with choice[i].use, each of which fills its part of all
+// the `seconds`; probs: what the reduction of their partial sums needs.  The rounds run one after
+// another and share one buffer, of kRoundBytes or the largest problem's; where the device has no
+// room for that, the rounds and then the slabs get smaller.
+constexpr size_t kRoundBytes = (size_t)4 << 30;
+int describe_expansions(holo_batch_s *b, const holo_problem *pr, const std::vector<ExpandChoice> &choice,
+                        double seconds, std::vector<ExpandProblem> *out, std::vector<Round> *rounds,
+                        std::vector<SplitProblem> *probs, cudaStream_t s) {
+  const int n = (int)choice.size();
+  auto describe = [&](int i, size_t slab, ExpandScratch &keep, ExpandScratch &tmp) {
+    ExpandProblem E = expand_describe(b->plans[i], choice[i], pr[i].sign * ((2.0 * M_PI) / pr[i].lambda),
+                                      (double2 *)pr[i].y_re_im, choice[i].seconds / seconds, slab,
+                                      keep, tmp);
+    E.nTs = std::min(E.slab, E.nT);
+    return E;
+  };
+  std::vector<int> which;
+  std::vector<size_t> at(n, 0);
+  size_t round_bytes = kRoundBytes, slab = kSlabBytes, kept = 0;
+  unsigned char *shared = nullptr;
+  for (;;) {
+    size_t used = 0, most = 0;
+    which.clear();
+    rounds->clear();
+    kept = 0;
+    for (int slabs = 0; slabs < 2; ++slabs)  // those of one slab first
+      for (int i = 0; i < n; ++i) {
+        if (!choice[i].use) continue;
+        ExpandScratch keep, tmp;
+        const ExpandProblem E = describe(i, slab, keep, tmp);
+        if ((E.nTs < E.nT) != (slabs == 1)) continue;
+        const int k = (int)which.size();
+        if (rounds->empty() || slabs || used + tmp.bytes > round_bytes) {
+          rounds->push_back({k, k, slabs == 1});
+          used = 0;
+        }
+        which.push_back(i);
+        rounds->back().last = k + 1;
+        at[i] = used;
+        used += tmp.bytes;
+        most = std::max(most, used);
+        kept += keep.bytes;
+      }
+    if (which.empty()) return HOLO_OK;
+    shared = (unsigned char *)pool_alloc(b->h, most, s);
+    if (shared) break;
+    if (round_bytes > slab) round_bytes /= 8;
+    else if (slab > kLeastSlabBytes) slab /= 8;
+    else return fail(HOLO_ERR_ALLOC, "batch expansion scratch of %zu bytes", most);
+  }
+  b->owned.push_back(shared);
+  unsigned char *own = (unsigned char *)pool_alloc(b->h, kept, s);
+  if (!own) return fail(HOLO_ERR_ALLOC, "batch amplitudes and partial sums of %zu bytes", kept);
+  b->owned.push_back(own);
+  for (int i : which) {
+    ExpandScratch keep, tmp;
+    keep.base = own;
+    tmp.base = shared + at[i];
+    const ExpandProblem E = describe(i, slab, keep, tmp);
+    own += keep.bytes;
+    out->push_back(E);
+    SplitProblem &P = (*probs)[i] = SplitProblem{};
+    P.apf_s = E.apf_s;
+    P.order_t = E.order_t;
+    P.partial = E.partial;
+    P.y = E.y;
+    P.N = E.N;
+    P.M = E.M;
+    P.splits = E.ssplit;
+  }
   return HOLO_OK;
 }
 
@@ -125,7 +183,8 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
   if (precision != HOLO_SPLIT32) return HOLO_OK;
 
   std::vector<SplitProblem> probs(n);
-  std::vector<ExpandProblem> expands, slabbed;  // slabbed: more scratch than one launch takes
+  std::vector<ExpandProblem> expands;
+  std::vector<Round> rounds;
   std::vector<ExpandChoice> choice(n);
   double seconds = 1e-12;
   for (int i = 0; i < n; ++i) {
@@ -134,20 +193,20 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
     else if (b->plans[i]->expand_only)
       return fail(HOLO_ERR_UNSUPPORTED, "problem %d: tiles too wide for the pair kernels", i);
   }
-  for (int i = 0; i < n; ++i) {
-    if (!choice[i].use) continue;
-    ExpandProblem E;
-    HOLO_TRY(describe_expansion(b, pr[i], b->plans[i], choice[i], choice[i].seconds / seconds, &E,
-                                &probs[i], s));
-    (E.nTs == E.nT ? expands : slabbed).push_back(E);
-  }
-  const int ne = (int)expands.size();
-  std::vector<int> offs(4 * (size_t)(ne + 1), 0);
-  int totals[4] = {0, 0, 0, 0};
-  for (int i = 0; i < ne; ++i) {
-    int blocks[4];
-    expand_blocks(expands[i], blocks);
-    for (int k = 0; k < 4; ++k) offs[(size_t)k * (ne + 1) + i + 1] = totals[k] += blocks[k];
+  HOLO_TRY(describe_expansions(b, pr, choice, seconds, &expands, &rounds, &probs, s));
+  // per round and kernel: the first block of each problem, and the total
+  std::vector<int> offs;
+  for (const Round &r : rounds) {
+    const size_t at = offs.size(), step = r.last - r.first + 1;
+    offs.resize(at + 4 * step, 0);
+    for (int i = r.first; i < r.last; ++i) {
+      int blocks[4];
+      expand_blocks(expands[i], blocks);
+      for (int k = 0; k < 4; ++k) {
+        int *o = &offs[at + k * step + (i - r.first)];
+        o[1] = o[0] + blocks[k];
+      }
+    }
   }
 
   std::vector<Group> groups;
@@ -229,12 +288,23 @@ int batch_build(holo_batch_s *b, const holo_problem *pr, int n, int precision, c
     if (!groups[g].items.empty())
       rc = launch_split_batched(probs_dev, groups[g].items_dev, (int)groups[g].items.size(),
                                 queues + g, groups[g].variant, groups[g].grid, h->dev_err, cap);
-  if (rc == HOLO_OK) rc = launch_expand_batched(expands_dev, offs_dev, totals, ne, h->sm_count, h->dev_err, cap);
-  for (ExpandProblem &E : slabbed)
-    for (E.t0 = 0; E.t0 < E.nT && rc == HOLO_OK; E.t0 += E.slab) {
-      E.nTs = std::min(E.slab, E.nT - E.t0);
-      rc = launch_expand(E, h->sm_count, h->dev_err, cap);
+  size_t at = 0;
+  for (const Round &r : rounds) {
+    const int count = r.last - r.first, step = count + 1;
+    if (r.slabs) {
+      ExpandProblem E = expands[r.first];
+      for (; E.t0 < E.nT && rc == HOLO_OK; E.t0 += E.slab) {
+        E.nTs = std::min(E.slab, E.nT - E.t0);
+        rc = launch_expand(E, h->sm_count, h->dev_err, cap);
+      }
+    } else if (rc == HOLO_OK) {
+      int totals[4];
+      for (int k = 0; k < 4; ++k) totals[k] = offs[at + (size_t)k * step + count];
+      rc = launch_expand_batched(expands_dev + r.first, offs_dev + at, totals, count, h->sm_count,
+                                 h->dev_err, cap);
     }
+    at += 4 * (size_t)step;
+  }
   if (rc == HOLO_OK) rc = launch_reduce_batched(probs_dev, offsets_dev, n, offsets[n], cap);
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(cap, &graph);

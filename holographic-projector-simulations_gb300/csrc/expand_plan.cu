@@ -141,7 +141,8 @@ ExpandChoice expand_choose(const BoxStats &src, const BoxStats &tgt, int N, int 
 }
 
 ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk, double2 *y,
-                              double share, ExpandScratch &tmp) {
+                              double share, size_t slab_bytes, ExpandScratch &keep,
+                              ExpandScratch &tmp) {
   const Variant V = split_variant(p->variant);
   ExpandProblem P{};
   P.geo_s = p->geo_s;
@@ -169,16 +170,16 @@ ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk,
   P.n_quads = expand_quads(P.px, P.py, P.quads);
   P.sk = sk;
   P.kap = (float)(0.5 * sk);
-  // target clusters per launch: at most 1 GiB of frames, moments and coefficients
+  // target clusters per launch: at most slab_bytes of frames, moments and coefficients
   const int groups_s = (P.nS + 31) / 32;
   const size_t row = (size_t)P.nS * (80 + 4 * 1024) + (size_t)groups_s * 65536;
-  const size_t most = std::max<size_t>(1, ((size_t)1 << 30) / row);
+  const size_t most = std::max<size_t>(1, slab_bytes / row);
   P.slab = most >= (size_t)P.nT ? P.nT : most >= 64 ? (int)(most / 64 * 64) : (int)most;
   const int sms = std::max(1, (int)(share * p->h->sm_count));
   P.ksplit = moment_shares(P.nS, P.slab, P.ns, sms);
   P.ssplit = target_shares(P.nS, std::min(P.slab * P.nt, P.M), sms);
   const size_t pairs = (size_t)P.slab * P.nS;
-  P.apf_s = tmp.take<float2>(p->n_pad);
+  P.apf_s = keep.take<float2>(p->n_pad);
   P.frames = tmp.take<float>(12 * pairs);
   P.basis = tmp.take<float>(8 * pairs);
   P.half_s = tmp.take<float>(4 * (size_t)P.nS);
@@ -189,23 +190,30 @@ ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk,
   P.tops = tmp.take<uint32_t>((size_t)(P.N + 4095) / 4096 + 1);
   P.moments = tmp.take<float2>((size_t)P.ksplit * pairs * kExpandNodes);
   P.coeffs = tmp.take<float>((size_t)P.slab * groups_s * 16384);
-  P.partial = P.ssplit > 1 ? tmp.take<double2>((size_t)P.ssplit * P.M) : nullptr;
+  P.partial = P.ssplit > 1 ? keep.take<double2>((size_t)P.ssplit * P.M) : nullptr;
   return P;
 }
 
 int expand_execute(holo_plan_s *p, const ExpandChoice &ch, double sk, const double *amp,
                    const double *phase, double2 *y, cudaStream_t s) {
-  ExpandScratch size;
-  expand_describe(p, ch, sk, y, 1.0, size);
   struct Buffer {
     void *p;
     cudaStream_t s;
     ~Buffer() { pool_free(p, s); }
-  } buf{pool_alloc(p->h, size.bytes, s), s};
-  if (!buf.p) return fail(HOLO_ERR_ALLOC, "expansion scratch of %zu bytes", size.bytes);
+  } buf{nullptr, s};
+  // smaller slabs where the device has no room for those of kSlabBytes
+  size_t slab = kSlabBytes, bytes = 0;
+  for (; !buf.p && slab >= kLeastSlabBytes; slab /= 8) {
+    ExpandScratch size;
+    expand_describe(p, ch, sk, y, 1.0, slab, size, size);
+    bytes = size.bytes;
+    buf.p = pool_alloc(p->h, bytes, s);
+    if (buf.p) break;
+  }
+  if (!buf.p) return fail(HOLO_ERR_ALLOC, "expansion scratch of %zu bytes", bytes);
   ExpandScratch tmp;
   tmp.base = static_cast<unsigned char *>(buf.p);
-  ExpandProblem P = expand_describe(p, ch, sk, y, 1.0, tmp);
+  ExpandProblem P = expand_describe(p, ch, sk, y, 1.0, slab, tmp, tmp);
   HOLO_TRY(launch_gather_apf(amp, phase, p->order_s, p->N, p->n_pad, const_cast<float2 *>(P.apf_s), s));
   HOLO_TRY(profile_mark(p->h, s, true));
   for (P.t0 = 0; P.t0 < P.nT; P.t0 += P.slab) {

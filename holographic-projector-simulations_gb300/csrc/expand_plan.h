@@ -24,10 +24,16 @@ struct ExpandScratch {
   }
 };
 
-// The descriptor of a sum (all but its slab) with its buffers taken from `tmp`; share: the
+// Scratch that a sum's target clusters may take per launch, and what it goes down to where the
+// device has no room for that.
+constexpr size_t kSlabBytes = (size_t)1 << 30, kLeastSlabBytes = (size_t)1 << 24;
+
+// The descriptor of a sum (all but its slab), its sources' amplitudes and phases and its partial
+// sums taken from `keep` and the rest, which only its own launches use, from `tmp`; share: the
 // part of the GPU that it should fill (1 alone, its part of the work in a batch).
 ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk, double2 *y,
-                              double share, ExpandScratch &tmp);
+                              double share, size_t slab_bytes, ExpandScratch &keep,
+                              ExpandScratch &tmp);
 int expand_execute(holo_plan_s *p, const ExpandChoice &ch, double sk, const double *amp,
                    const double *phase, double2 *y, cudaStream_t s);
 
