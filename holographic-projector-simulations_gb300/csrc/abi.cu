@@ -539,9 +539,9 @@ int plan_create_impl(holo_handle h, const double *u, size_t N, const double *v, 
 ExpandChoice plan_expansion(holo_plan_s *p, double k, double launches) {
   if (p->precision != HOLO_SPLIT32 || p->pair_kernel_only || p->N == 0 || p->M == 0) return {};
   const Variant V = split_variant(p->variant);
-  if (box_level(V.cs) < 0) return {};  // its tiles do not nest in the clusters
+  const int least_s = box_level(V.cs) < 0 ? box_level(512) : box_level(V.cs);  // 768: as 512
   if (p->expand_k != k || p->expand_launches != launches) {
-    p->expand = expand_choose(p->stats_s, p->stats_t, p->N, p->M, box_level(V.cs), box_level(V.tt()),
+    p->expand = expand_choose(p->stats_s, p->stats_t, p->N, p->M, least_s, box_level(V.tt()),
                               k, pair_seconds(p), launches, p->h->sm_count);
     p->expand_k = k;
     p->expand_launches = launches;

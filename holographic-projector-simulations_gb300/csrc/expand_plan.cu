@@ -157,8 +157,6 @@ ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk,
   P.M = p->M;
   P.cs = V.cs;
   P.tt = V.tt();
-  P.cs_log2 = 8 + box_level(P.cs);
-  P.tt_log2 = 8 + box_level(P.tt);
   P.ns = 256 << ch.ls;
   P.nt = 256 << ch.lt;
   P.nS = box_count(P.N, ch.ls);
@@ -184,8 +182,8 @@ ExpandProblem expand_describe(holo_plan_s *p, const ExpandChoice &ch, double sk,
   P.basis = tmp.take<float>(8 * pairs);
   P.half_s = tmp.take<float>(4 * (size_t)P.nS);
   P.half_t = tmp.take<float>(4 * (size_t)P.nT);
-  P.shift_s = tmp.take<float>(8 * (size_t)((P.N + P.cs - 1) / P.cs));
-  P.shift_t = tmp.take<float>(8 * (size_t)((P.M + P.tt - 1) / P.tt));
+  P.shift_s = tmp.take<float>(8 * (size_t)box_count(P.N, 0));
+  P.shift_t = tmp.take<float>(8 * (size_t)box_count(P.M, 0));
   P.cheb = tmp.take<float>(2 * (16 * 16 + 16));
   P.tops = tmp.take<uint32_t>((size_t)(P.N + 4095) / 4096 + 1);
   P.moments = tmp.take<float2>((size_t)P.ksplit * pairs * kExpandNodes);

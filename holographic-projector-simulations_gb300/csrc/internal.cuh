@@ -263,7 +263,7 @@ struct BoxStats {
   double h[kBoxLevels];            // largest half diagonal per level
 };
 constexpr int kBoxStatDoubles = sizeof(BoxStats) / sizeof(double);
-inline int box_count(int n, int level) { return (n + (256 << level) - 1) / (256 << level); }
+__host__ __device__ inline int box_count(int n, int level) { return (n + (256 << level) - 1) / (256 << level); }
 inline size_t box_offset(int n, int level) {  // in boxes; level kBoxLevels: all of them
   size_t o = 0;
   for (int l = 0; l < level; ++l) o += box_count(n, l);
@@ -302,7 +302,7 @@ struct ExpandProblem {
   float *frames;                     // [nTs][nS][12]: (s k e hi, r0) (lo, b0 hi) (e, b0 lo)
   float *basis;                      // [nTs][nS][8]: the perpendicular axes of each pair
   float *half_s, *half_t;            // [cluster][4]: half extents along ax and ay, inverses
-  float *shift_s, *shift_t;          // [tile][8]: tile centre - cluster centre, float-float
+  float *shift_s, *shift_t;          // [256 points][8]: tile centre - cluster centre, float-float
   float *cheb;                       // Chebyshev tables of both axes
   uint32_t *tops;                    // bits of the largest |amplitude| of every 4096 sources, then
                                      // the exponent field of the sum's scale
@@ -316,7 +316,6 @@ struct ExpandProblem {
   int n_quads;
   uint32_t quads[32];
   int ksplit, ssplit;                // shares of a cluster's sources / of the source clusters
-  int cs_log2, tt_log2;
   float kap;                         // s k / 2
   double sk;
 };

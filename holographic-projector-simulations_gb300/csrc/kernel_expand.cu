@@ -168,13 +168,14 @@ __global__ void __launch_bounds__(128) k_expand_setup(const ExpandProblem P0,
     return;
   }
   i -= pairs;
-  const int tiles_s = (P.N + P.cs - 1) / P.cs, tiles_t = (P.M + P.tt - 1) / P.tt;
-  if (i < tiles_s + tiles_t) {
-    const bool src = i < tiles_s;
-    const int j = src ? i : i - tiles_s;
-    const double *c = (src ? P.tiles_s : P.tiles_t) + 6 * (size_t)j;
-    const double *b = src ? P.box_s + 6 * (size_t)((long long)j * P.cs / P.ns)
-                          : P.box_t + 6 * (size_t)((long long)j * P.tt / P.nt);
+  const int leaves_s = box_count(P.N, 0), leaves_t = box_count(P.M, 0);
+  if (i < leaves_s + leaves_t) {
+    const bool src = i < leaves_s;
+    const int j = src ? i : i - leaves_s;
+    const double *c = src ? P.tiles_s + 6 * (size_t)(j * kLeafTile / P.cs)
+                          : P.tiles_t + 6 * (size_t)(j * kLeafTile / P.tt);
+    const double *b = src ? P.box_s + 6 * (size_t)(j * kLeafTile / P.ns)
+                          : P.box_t + 6 * (size_t)(j * kLeafTile / P.nt);
     float *o = (src ? P.shift_s : P.shift_t) + 8 * (size_t)j;
     for (int d = 0; d < 3; ++d) {
       const double x = c[d] - b[d];
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(128) k_expand_setup(const ExpandProblem P0,
     }
     return;
   }
-  i -= tiles_s + tiles_t;
+  i -= leaves_s + leaves_t;
   if (i < P.nS + P.nT) {
     const bool src = i < P.nS;
     const int j = src ? i : i - P.nS;
@@ -206,11 +207,12 @@ __global__ void __launch_bounds__(128) k_expand_setup(const ExpandProblem P0,
   }
 }
 
-// Float offset of record i of tile-ordered point arrays relative to its cluster's centre.
+// Float offset of record i of tile-ordered point arrays relative to its cluster's centre.  The
+// shifts are per 256 points, so that tiles need not nest in the clusters (those of 768 do not).
 __device__ __forceinline__ void cluster_offset(const float *geo, const float *shift, int i,
-                                               int tile_log2, float h[3], float l[3]) {
+                                               float h[3], float l[3]) {
   const float2 *g = reinterpret_cast<const float2 *>(geo + 6 * (size_t)i);
-  const float4 *s = reinterpret_cast<const float4 *>(shift + 8 * (size_t)(i >> tile_log2));
+  const float4 *s = reinterpret_cast<const float4 *>(shift + 8 * (size_t)(i / kLeafTile));
   const float2 g0 = g[0], g1 = g[1], g2 = g[2];
   const float4 sh = s[0], sl = s[1];
   add_ff(g0.x, g1.y, sh.x, sl.x, h[0], l[0]);
@@ -350,7 +352,7 @@ __global__ void __launch_bounds__(kMomThreads, 2)
       float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
       float2 pa = make_float2(0.f, 0.f);
       if (idx < P.N) {
-        cluster_offset(P.geo_s, P.shift_s, idx, P.cs_log2, h, l);
+        cluster_offset(P.geo_s, P.shift_s, idx, h, l);
         pa = P.apf_s[idx];
       }
       // a source that is not finite spoils the cluster's moments; it is looked for here, once
@@ -912,7 +914,7 @@ __global__ void __launch_bounds__(kTgtThreads, 1)
       const ExpandProblem &P = locate(item, w);
       const int px = P.px, py = P.py, np = px * py, t = w.m0 + row;
       float th[3] = {0.f, 0.f, 0.f}, tl[3] = {0.f, 0.f, 0.f};
-      if (t < P.M) cluster_offset(P.geo_t, P.shift_t, t, P.tt_log2, th, tl);
+      if (t < P.M) cluster_offset(P.geo_t, P.shift_t, t, th, tl);
       const float4 hx = reinterpret_cast<const float4 *>(P.half_t)[P.t0 + w.Tl];
       // the builders' reads of the last item's factors are behind the barrier below; its
       // records' buffer was released with the parts of item - 2
@@ -991,7 +993,7 @@ __global__ void __launch_bounds__(kTgtThreads, 1)
 }  // namespace
 
 void expand_blocks(const ExpandProblem &p, int blocks[4]) {
-  const long long n = (long long)p.nTs * p.nS + (p.N + p.cs - 1) / p.cs + (p.M + p.tt - 1) / p.tt +
+  const long long n = (long long)p.nTs * p.nS + box_count(p.N, 0) + box_count(p.M, 0) +
                       p.nS + p.nT + 2 * kMaxP * kMaxP;
   blocks[0] = top_blocks(p.N) + (int)((n + 127) / 128);
   blocks[1] = p.nS * ((p.nTs + kGroupT - 1) / kGroupT) * p.ksplit;
