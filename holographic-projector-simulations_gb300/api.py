@@ -115,8 +115,11 @@ def _empty_complex(ref: _Buf, count: int):
 
 def _stream(ref: _Buf):
     if ref.device:
-        # the stream's address without a Stream object around it (4 us a call less)
-        return torch._C._cuda_getCurrentRawStream(ref.dev_index)
+        try:
+            # the stream's address without a Stream object around it (4 us a call less)
+            return torch._C._cuda_getCurrentRawStream(ref.dev_index)
+        except AttributeError:
+            return torch.cuda.current_stream(ref.dev_index).cuda_stream
     return None
 
 

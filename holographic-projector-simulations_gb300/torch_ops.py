@@ -65,15 +65,19 @@ def _intensity_loss_ops(z: torch.Tensor, target: torch.Tensor) -> torch.Tensor:
 
 def _plain(*tensors: torch.Tensor) -> bool:
     """Tensors a kernel may read by their address: no subclass, no transform, mode or tracer
-    at work that has to see each operation, no lazy negation, on 16-byte boundaries."""
-    return (not torch._C._are_functorch_transforms_active()
-            and not torch._C._len_torch_dispatch_stack()
-            and not torch._C._len_torch_function_stack()
-            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
-            and all(type(t) is torch.Tensor and t.is_cuda and t.dtype is torch.float64
-                    and torch._C._has_storage(t) and t.is_contiguous() and not t.is_neg()
-                    and t.data_ptr() % 16 == 0
-                    and forward_ad.unpack_dual(t).tangent is None for t in tensors))
+    at work that has to see each operation, no lazy negation, on 16-byte boundaries.  A PyTorch
+    without one of the functions asked for that says so has array operations do the work."""
+    try:
+        return (not torch._C._are_functorch_transforms_active()
+                and not torch._C._len_torch_dispatch_stack()
+                and not torch._C._len_torch_function_stack()
+                and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+                and all(type(t) is torch.Tensor and t.is_cuda and t.dtype is torch.float64
+                        and torch._C._has_storage(t) and t.is_contiguous() and not t.is_neg()
+                        and t.data_ptr() % 16 == 0
+                        and forward_ad.unpack_dual(t).tangent is None for t in tensors))
+    except AttributeError:
+        return False
 
 
 def _native_loss(z, target, with_grad: bool):
