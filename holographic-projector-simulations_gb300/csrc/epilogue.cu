@@ -63,6 +63,19 @@ __device__ __forceinline__ bool fast_polar(double x, double y, const fixed::Pola
                       [](float v) { return ptx::rsqrt_approx(v); }, modulus, angle);
 }
 
+// Modulus and angle of what fast_polar leaves; zeros, which whole dark fields hold, without the
+// ~90 FP64 operations of a hypot and an atan2 (a normalisation of 2^20 zeros: 226 us with both
+// alone, 237 us with fast_polar tried before them, 86 us here).
+__device__ __forceinline__ void slow_polar(double x, double y, double *modulus, double *angle) {
+  if (x == 0.0 && y == 0.0) {
+    *modulus = 0.0;
+    *angle = signbit(x) ? copysign(3.14159265358979323846, y) : y;
+  } else {
+    *modulus = hypot(x, y);
+    *angle = atan2(y, x);
+  }
+}
+
 // The largest modulus.  Bound by the FP64 pipe: the squares' sum (2 operations instead of
 // hypot's ~35) of every value first, then hypot only of those within 2^-40 of the block's largest
 // sum, which the largest hypot is among; a block whose sums leave the safe range takes hypot
@@ -91,7 +104,8 @@ __global__ void __launch_bounds__(256) k_max_abs_partial(const double2 *__restri
   double m = 0.0;
   if (!(most < limit))  // none of this thread's values otherwise
     for (int i = first; i < M; i += step)
-      if (!(fma(y[i].x, y[i].x, y[i].y * y[i].y) < limit)) m = fmax(m, hypot(y[i].x, y[i].y));
+      if (!(fma(y[i].x, y[i].x, y[i].y * y[i].y) < limit) && !(y[i].x == 0.0 && y[i].y == 0.0))
+        m = fmax(m, hypot(y[i].x, y[i].y));
   s[threadIdx.x] = m;
   __syncthreads();
   for (int w = 128; w > 0; w >>= 1) {
@@ -141,8 +155,7 @@ __global__ void __launch_bounds__(256) k_normalize_polar(const double2 *__restri
         re = __ddiv_rn(re, mx);
         im = __ddiv_rn(im, mx);
       }
-      m = hypot(re, im);
-      a = atan2(im, re);
+      slow_polar(re, im, &m, &a);
     }
     amp[i] = m;
     phase[i] = a;
@@ -155,10 +168,7 @@ __global__ void __launch_bounds__(256) k_complex_to_polar(const double2 *__restr
                                                           double *__restrict__ phase) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
     double m, a;
-    if (!fast_polar(g[i].x, g[i].y, table, &m, &a)) {
-      m = hypot(g[i].x, g[i].y);
-      a = atan2(g[i].y, g[i].x);
-    }
+    if (!fast_polar(g[i].x, g[i].y, table, &m, &a)) slow_polar(g[i].x, g[i].y, &m, &a);
     amp[i] = m;
     phase[i] = a;
   }
