@@ -21,7 +21,7 @@
 //
 // Truncation: for e^{i z x} on [-1, 1] the p-node interpolant is off by at most
 // 2 (z / 2)^p / p!; expand_choose (expand_plan.cu) takes the cheapest cluster sizes for which
-// that stays below 8e-7 along each axis, which measured 2e-7 of the field's norm or less.
+// that stays below 8e-7 along each axis, which measured 2.5e-7 of the field's norm or less.
 //
 // The TF32 accumulator of an MMA drops bits of the running sum at every step, a bias that
 // grows with the length of the chain: the moments kernel moves its accumulator to FP32
@@ -635,9 +635,9 @@ __global__ void __launch_bounds__(kNodes) k_expand_translate(
 //   MMA warp             one thread issues the products into one of two TMEM buffers
 //   consumers (16 warps) read D, rotate by e^{i s k alpha}, sum: each thread one target and
 //                        8 clusters of every 32
-// Bound by the consumers' FP32 and MUFU work (~3,000 clocks per 32 clusters); a block per
-// item without roles took 12,000 clocks of set-up and tail per item (see the figures at
-// expand_plan.h).  Hand-offs are mbarrier phases; those a waiter may trail by two items come in
+// Bound by issue slots: an item of 64 source clusters takes 13,300 clocks (512^2 -> 1024^2: 54 items
+// a CTA, 0.37 ms, ncu: 65 % of the slots issue), most of them the consumers' FP32 work; a block
+// per item without roles took 12,000 clocks of set-up and tail per item beside that.  Hand-offs are mbarrier phases; those a waiter may trail by two items come in
 // pairs.
 struct TargetsSmem {
   static constexpr int kStages = 4;                                 // halves of coefficients

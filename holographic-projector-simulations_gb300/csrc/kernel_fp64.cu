@@ -136,14 +136,16 @@ __global__ void __launch_bounds__(THREADS, MINB)
 // distance x k and the sum phase + that.  Bit for bit the other kernel's phases; amplitude /
 // distance, sine and cosine are exact to 2^-55 or better and their products are summed as
 // 64-bit integers, a tile of sources at a time, to 2^-54 of the target's own term of the tile's
-// largest amplitude, whose distance sets the target's scale.  A pair out of the fixed-point ranges (a zero,
-// infinite or NaN value, a distance four times under the one that set the scale, a phase beyond
-// 2^43) takes the FP64 operations instead.
-// Measured (GB300, 1000 sources -> 512^2 lattice targets): 4.4 ms against 30.0 ms (variant 0); the
+// largest amplitude, whose distance sets the target's scale.  A pair out of the fixed-point
+// ranges (a zero, infinite or NaN value, a distance four times under the one that set the
+// scale, a phase beyond 2^43) takes the FP64 operations instead.
+// Measured (GB300, 1000 sources -> 512^2 lattice targets): 4.35 ms against 30.0 ms (variant 0); the
 // same with targets jittered, so that no coordinate is shared, 5.2 ms; with registers for 4 or
 // 3 CTAs per SM instead of 5 4.6 ms, 2 targets a thread 4.9 ms, 8 4.6 ms.  Bound by the FP64
-// pipe: 7.1 of its slots a pair at 0.93 of the rate a pure DFMA stream reaches (ncu: pipe 79 %
-// active, issue slots 55 % for 314 instructions a pair).
+// pipe: 7.1 of its slots a pair at 0.92 of the rate a pure DFMA stream reaches (ncu: pipe 78 %
+// active, issue slots 55 % for 319 instructions a pair).  One scale for a thread's four targets
+// and one rounding for all sources took 4.28 ms and lost the bits that targets farther from a
+// tile's brightest source than the first one need.
 // One target a thread (variant 7) is for problems that would not fill the GPU: a whole call
 // of 64 -> 64^2 0.10 ms against 0.24, of 256 -> 128^2 0.19 against 0.24, but of 1000 ->
 // 128^2 0.44 against 0.37.

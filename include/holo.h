@@ -113,13 +113,15 @@ int holo_plan_execute_flags(holo_plan p, int sign, double lambda, const double *
 /* Sorted visiting order of the plan's points (which = 0: sources, 1: targets):
  * out[i] = original index of the i-th point in tile order.  Host pointer. */
 int holo_plan_get_order(holo_plan p, int which, int32_t *out);
-/* Selected kernel variant and split factor (for the autotuner and tests). */
+/* Selected pair kernel variant and split factor (for the autotuner and tests), whether or not
+ * the plan's sums go by expansions instead. */
 int holo_plan_info(holo_plan p, int *variant, int *splits, int *target_tile,
                    int *source_tile);
 /* HOLO_SPLIT32: bound (metres) on the path-length error of any term, from the
  * tile extents and the gap between the point sets; the phase error bound is
  * k times it.  The planner picks tiles small enough to keep it under 3.2e-13 m
- * (5e-6 rad at 400 nm) when it can; 0 for HOLO_FP64.  Infinite when the two
+ * (5e-6 rad at 400 nm) when it can; 0 for HOLO_FP64.  It is the bound of the pair kernel:
+ * sums that go by expansions keep their own, 8e-7 of truncation per axis of a cluster.  Infinite when the two
  * point sets' bounding boxes touch (near field: use HOLO_FP64). */
 int holo_plan_error_bound(holo_plan p, double *metres);
 
